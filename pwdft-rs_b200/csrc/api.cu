@@ -44,7 +44,7 @@ static void release(Handle& h) {
   auto f = [](void* p) { if (p) cudaFree(p); };
   GridMaps& g = h.g;
   for (int a = 0; a < 3; ++a) { f(g.tw64[a]); f(g.tw32[a]); }
-  f(g.col_start); f(g.pt_ig); f(g.pt_col); f(g.pt_z); f(g.g_to_fft);
+  f(g.col_start); f(g.col_lo); f(g.pt_ig); f(g.pt_col); f(g.pt_z); f(g.g_to_fft);
   for (auto& k : h.kp) { f(k.kinetic); f(k.b); f(k.b32); }
   h.kp.clear();
   f(h.ch_atom); f(h.atom_ch_start); f(h.d_off); f(h.d_vals);

@@ -35,6 +35,13 @@ struct GridMaps {
   int* pt_col = nullptr;     // n_pw: column of sorted point
   int* pt_z = nullptr;       // n_pw: wrapped z index
   int* g_to_fft = nullptr;   // n_pw (basis order): flat grid index
+  // basis order lists the columns one after the other, each at consecutive n2: column c holds the
+  // basis points col_start[c] .. col_start[c + 1] - 1 from n2 = col_lo[c]
+  bool contiguous = false;
+  int* col_lo = nullptr;     // ncol
+  // the two-stage pipeline of hpsi_plane.cu: radix pair of each axis (-1: none) and whether it applies
+  int pair[3] = {-1, -1, -1};
+  bool plane_ok = false;
   // tile widths chosen for the FFT kernels (lines per block)
   int wz = 1, wy = 1, wx = 1;
   int wz32 = 1, wy32 = 1, wx32 = 1;  // FP32 tiles: measured at handle creation
@@ -85,7 +92,8 @@ struct Handle {
   float* veff_rz32[2] = {nullptr, nullptr};
   // H|psi> scratch: band-chunked compact grids (L2-resident per chunk)
   int chunk = 1;
-  void* work_a = nullptr;   // chunk * ncol * d2 complex (FP64 size)
+  int chunk_a = 1;          // bands of work_a (>= chunk): the two-stage pipeline uses no work_b
+  void* work_a = nullptr;   // chunk_a * ncol * d2 complex (FP64 size)
   void* work_b = nullptr;   // chunk * Xp * d1 * d2 complex
   double2* nl_p = nullptr;  // n_ch x max_nb
   double2* nl_q = nullptr;
@@ -151,6 +159,13 @@ Status set_veff_from_g(Handle& h, int spin, const double2* veff_g_dev, cudaStrea
 // Refresh the z-major copies (veff_rz, veff_rz32) of veff_r[spin].
 Status veff_zmajor(Handle& h, int spin, cudaStream_t stream);
 Status ensure_nl_capacity(Handle& h, int nb);
+// Two-stage local pipeline (hpsi_plane.cu): decides g.plane_ok after the grid
+// maps are built, and applies the local part of H to nb bands with the
+// compact planes in `scratch` (nb * ncol * d2 entries of R).
+Status plane_setup(Handle& h);
+template <typename R>
+Status local_plane(Handle& h, int spin, int ik, const double2* psi, long ldpsi, int nb, double2* hpsi, long ldh,
+                   cudaStream_t s, void* scratch, StageTimer* tm);
 // P = B^H psi into h.nl_p and Q = D P into h.nl_q (FP64), nb columns.
 Status nonlocal_pq(Handle& h, int ik, const double2* psi, long ldpsi, int nb, cudaStream_t s,
                    StageTimer* tm = nullptr);

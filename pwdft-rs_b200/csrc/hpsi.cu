@@ -9,7 +9,11 @@
 // collects V(G) psi_j for every G == G_i - G_j on the wrapped grid, which
 // is V_eff[miller_to_idx(m_i - m_j)] of the dense matrix.
 //
-// Pipeline per chunk of bands (intermediates sized to stay in L2):
+// Grids whose axes are two-stage lengths with room for the sphere's products
+// (4 max|n| < length, the reference's grid rule) and whose basis lists the
+// sphere column by column -- the reference's own grids and order -- run the
+// three kernels of hpsi_plane.cu.  The others, here, per chunk of bands
+// (intermediates sized to stay in L2):
 //   K1 z-inverse on the Xp*Yp sphere columns, scattering psi(G)   -> A
 //   K234, one kernel per z-plane of A (z-major) and group of bands, the plane
 //        in shared memory: y-inverse of the Xp compact x-planes, x-inverse,
@@ -954,7 +958,18 @@ Status build_grid_maps(Handle& h, const int* miller) {
     cs[col[i] + 1]++;
   }
   for (int c = 0; c < g.ncol; ++c) cs[c + 1] += cs[c];
+  // columns of the basis order itself, each at consecutive n2?
+  std::vector<int> lo(g.ncol, 0);
+  g.contiguous = true;
+  for (int c = 0; c < g.ncol; ++c) {
+    if (cs[c + 1] == cs[c]) continue;
+    lo[c] = miller[3 * pig[cs[c]] + 2];
+    for (int s = cs[c]; s < cs[c + 1]; ++s)
+      if (pig[s] != s || miller[3 * s + 2] != lo[c] + (s - cs[c])) g.contiguous = false;
+  }
   Status st;
+  if ((st = dalloc(&g.col_lo, g.ncol)) != kOk) return st;
+  PW_CUDA_TRY(cudaMemcpy(g.col_lo, lo.data(), g.ncol * sizeof(int), cudaMemcpyHostToDevice));
   if ((st = dalloc(&g.col_start, g.ncol + 1)) != kOk) return st;
   if ((st = dalloc(&g.pt_ig, h.n_pw)) != kOk) return st;
   if ((st = dalloc(&g.pt_col, h.n_pw)) != kOk) return st;
@@ -990,10 +1005,14 @@ Status build_grid_maps(Handle& h, const int* miller) {
   // band chunk: keep A + B of one chunk within ~48 MB (FP64) of L2
   const double per_band = 16.0 * ((double)g.ncol * g.d[2] + (double)g.Xp * g.d[1] * g.d[2]);
   h.chunk = std::max(1, std::min(64, (int)(48.0e6 / per_band)));
-  if ((st = dalloc((double2**)&h.work_a, (size_t)h.chunk * g.ncol * g.d[2])) != kOk) return st;
+  if ((st = plane_setup(h)) != kOk) return st;
+  h.chunk_a = h.chunk;
+  if (g.plane_ok) h.chunk_a = std::max(h.chunk, std::min(256, (int)(48.0e6 / (16.0 * (double)g.ncol * g.d[2]))));
+  if ((st = dalloc((double2**)&h.work_a, (size_t)h.chunk_a * g.ncol * g.d[2])) != kOk) return st;
   if ((st = dalloc((double2**)&h.work_b, (size_t)h.chunk * g.Xp * g.d[1] * g.d[2])) != kOk) return st;
   if ((st = dalloc(&h.tmp_grid, (size_t)g.N)) != kOk) return st;
-  return autotune_tiles(h);
+  // the two-stage pipeline has no tile widths to choose
+  return g.plane_ok ? kOk : autotune_tiles(h);
 }
 
 Status ensure_nl_capacity(Handle& h, int nb) {
@@ -1203,6 +1222,20 @@ Status local_apply_on_scratch(Handle& h, int spin, int ik, const double2* psi, l
     return fail(kInvalid, "grid too large for the fixed scratch: one band needs " + std::to_string(per_band) +
                               " bytes, the scratch holds " + std::to_string(scratch_bytes));
   unsigned char* base = static_cast<unsigned char*>(scratch);
+  if (g.plane_ok) {
+    // the two-stage pipeline needs the compact planes only
+    const int wide = (int)std::min<size_t>(256, scratch_bytes / (a_elems * cb));
+    for (int c0 = 0; c0 < nb; c0 += wide) {
+      const int cnt = std::min(wide, nb - c0);
+      const double2* in = psi + (long)c0 * ldpsi;
+      double2* out = hpsi + (long)c0 * ldh;
+      const Status st = precision == 0
+                            ? local_plane<double>(h, spin, ik, in, ldpsi, cnt, out, ldh, s, base, nullptr)
+                            : local_plane<float>(h, spin, ik, in, ldpsi, cnt, out, ldh, s, base, nullptr);
+      if (st != kOk) return st;
+    }
+    return kOk;
+  }
   const size_t a_bytes = ((a_elems * chunk * cb) + 255) / 256 * 256;
   for (int c0 = 0; c0 < nb; c0 += chunk) {
     const int cnt = std::min(chunk, nb - c0);
@@ -1249,12 +1282,19 @@ Status density_accumulate(Handle& h, const double2* psi, long ldpsi, int nb, con
 
 Status apply_local_device(Handle& h, int spin, int ik, const double2* psi, long ldpsi, int nb, double2* hpsi,
                           long ldh, int precision, cudaStream_t s, StageTimer* tm) {
-  // the work buffers are sized for h.chunk FP64 bands; FP32 fits twice as many
-  const int chunk = precision == 0 ? h.chunk : 2 * h.chunk;
+  // the work buffers are sized for FP64 bands; FP32 fits twice as many
+  const int cap = h.g.plane_ok ? h.chunk_a : h.chunk;
+  const int chunk = precision == 0 ? cap : 2 * cap;
   for (int c0 = 0; c0 < nb; c0 += chunk) {
     const int cnt = std::min(chunk, nb - c0);
     Status st;
-    if (precision == 0)
+    if (h.g.plane_ok && precision == 0)
+      st = local_plane<double>(h, spin, ik, psi + (long)c0 * ldpsi, ldpsi, cnt, hpsi + (long)c0 * ldh, ldh, s,
+                               h.work_a, tm);
+    else if (h.g.plane_ok)
+      st = local_plane<float>(h, spin, ik, psi + (long)c0 * ldpsi, ldpsi, cnt, hpsi + (long)c0 * ldh, ldh, s,
+                              h.work_a, tm);
+    else if (precision == 0)
       st = local_chunk<double>(h, spin, ik, psi + (long)c0 * ldpsi, ldpsi, cnt, hpsi + (long)c0 * ldh, ldh, s, tm);
     else
       st = local_chunk<float>(h, spin, ik, psi + (long)c0 * ldpsi, ldpsi, cnt, hpsi + (long)c0 * ldh, ldh, s, tm);

@@ -425,11 +425,12 @@ static Status create_lane(Handle& h, Lane& L, int nd, int nlanes) {
   v.gam_pcap = 0;
   // lanes share the L2: each keeps a proportionally smaller band chunk
   v.chunk = std::max(4, h.chunk / nlanes);
+  v.chunk_a = std::max(v.chunk, h.chunk_a / nlanes);
   PW_CUDA_TRY(cudaStreamCreateWithFlags(&v.stream, cudaStreamNonBlocking));
   if (cublasCreate(&v.blas) != CUBLAS_STATUS_SUCCESS) return fail(kCuda, "cublasCreate failed (lane)");
   cublasSetStream(v.blas, v.stream);
   const GridMaps& g = h.g;
-  cudaError_t e = cudaMalloc(&v.work_a, (size_t)v.chunk * g.ncol * g.d[2] * sizeof(double2));
+  cudaError_t e = cudaMalloc(&v.work_a, (size_t)v.chunk_a * g.ncol * g.d[2] * sizeof(double2));
   if (e == cudaSuccess) e = cudaMalloc(&v.work_b, (size_t)v.chunk * g.Xp * g.d[1] * g.d[2] * sizeof(double2));
   if (e != cudaSuccess) return fail(kOom, std::string("cudaMalloc (lane): ") + cudaGetErrorString(e));
   return eig_work_alloc(L.ew, h.n_pw, nd);
