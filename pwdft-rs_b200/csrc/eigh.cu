@@ -12,16 +12,15 @@
 //     p = tau A v, w = p - tau/2 (p^H v) v, A -= v w^H + w v^H).  The matrix
 //     stays in shared memory for the whole reduction: column j lives in CTA
 //     (j mod C), so the product A v needs no cross-CTA reduction (each CTA
-//     owns whole columns of a Hermitian matrix = whole rows of A v).  Per
-//     step the owner of column k broadcasts v into every CTA's shared
-//     memory (distributed shared memory stores), one cluster barrier, every
-//     CTA broadcasts its entries of p, a second barrier, every CTA updates
-//     its own columns.  v stays in column k for the back-transform.
+//     owns whole columns of a Hermitian matrix = whole rows of A v).  Every
+//     CTA keeps v and w whole and forms each reflector itself, so a step
+//     exchanges once: the entries of p, the partials of p^H v and the next
+//     column go through L2 under one cluster barrier.  Small matrices are
+//     reduced by one CTA, with two block barriers a step (tridiag_one).
 //  2. Eigenvalues of the tridiagonal T by multisection: one warp per
 //     eigenvalue index, 32 Sturm counts per round (the three-term
-//     recurrence of det(T - x I) with power-of-two rescaling; a zero term
-//     takes the sign that counts it, as the zero pivot of the LDL^T count
-//     does), until the interval is a few ulps wide.
+//     recurrence of det(T - x I) with power-of-two rescaling), until the
+//     interval is a few ulps wide.
 //  3. Eigenvectors of T by inverse iteration, one thread per eigenvalue:
 //     Gaussian elimination of T - lambda I with partial pivoting (a zero
 //     pivot is replaced by eps ||T||), then two solves from a seeded start
@@ -30,8 +29,16 @@
 //     twice), one warp per group; elsewhere inverse iteration leaves them
 //     orthogonal to eps ||T|| / gap.
 //  4. Back-transform x = H(0) ... H(m-2) z, one warp per eigenvector, the
-//     vector in registers and the reflectors read from the owning CTAs'
-//     shared memory.
+//     vector in registers and the reflectors streamed through shared memory.
+//
+// What bounds it: latency.  The steps of 1 are serial, and a step at m = 540
+// is ~7,400 cycles: the pass over the owned columns ~3,000 (shared-memory
+// wavefronts and load latency), the cluster barrier ~1,250, the reads from L2
+// ~1,300, two warp-wide sums with a square root and a division ~1,800.  One
+// solve, lowest third of the pairs (all at 180), B200, against the form with
+// two cluster barriers a step and blocked back-transform: m = 540 2.8 ms
+// (3.8), 360 1.65 (2.06), 180 0.77 (0.96), 66 0.18 (0.25); complex m = 64
+// 0.21, 30 0.10 ms.  The one-CTA Jacobi solver takes 1.8 ms at m = 64.
 //
 // Every loop is bounded and every thread reaches the same sequence of
 // cluster barriers.  Status: 0 ok, 1 a non-finite eigenvalue or vector.
@@ -54,21 +61,6 @@ namespace cg = cooperative_groups;
 // CTA 0 records %globaltimer at each phase boundary into eigh_phase_ns[].
 #ifdef PWGPU_EIGH_PHASES
 __device__ unsigned long long eigh_phase_ns[8];
-__device__ long long eigh_sub_cycles[8];
-#define EIGH_SUB_DECL long long sub_last_ = clock64(), sub_acc_[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#define EIGH_SUB(n)                                                             \
-  do {                                                                          \
-    if (rank == 0 && tid == 0) {                                                \
-      const long long t_ = clock64();                                           \
-      sub_acc_[n] += t_ - sub_last_;                                            \
-      sub_last_ = t_;                                                           \
-    }                                                                           \
-  } while (0)
-#define EIGH_SUB_STORE                                                          \
-  do {                                                                          \
-    if (rank == 0 && tid == 0)                                                  \
-      for (int n_ = 0; n_ < 8; ++n_) eigh_sub_cycles[n_] = sub_acc_[n_];        \
-  } while (0)
 #define EIGH_MARK(n)                                                            \
   do {                                                                          \
     if (rank == 0 && tid == 0) {                                                \
@@ -81,13 +73,6 @@ __device__ long long eigh_sub_cycles[8];
 #define EIGH_MARK(n) \
   do {               \
   } while (0)
-#define EIGH_SUB_DECL
-#define EIGH_SUB(n) \
-  do {              \
-  } while (0)
-#define EIGH_SUB_STORE \
-  do {                 \
-  } while (0)
 #endif
 
 namespace pwgpu {
@@ -98,6 +83,8 @@ constexpr int kThreads = 512;
 constexpr int kWarps = kThreads / 32;
 constexpr int kRegRows = 17;               // rows per lane in the back-transform
 constexpr int kMaxM = 32 * kRegRows;       // 544
+constexpr int kRowGroups = (kRegRows + 3) / 4;  // groups of four row slots of the back-transform
+constexpr int kRowsPerThread = (kMaxM + kThreads - 1) / kThreads;
 constexpr int kMaxCluster = 16;
 constexpr int kBisectRounds = 48;
 constexpr double kEps = 1.1102230246251565e-16;  // 2^-53
@@ -112,56 +99,56 @@ __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.w
 
 // Shared-memory layout of one CTA (identical on host and device).
 struct Layout {
-  size_t a, v, p, s, sc, d, e2, tau, eig, grp, red, hh, total;
+  size_t a, v, p, c, d, e2, tau, eig, grp, red, total;
 };
 __host__ __device__ inline size_t align16(size_t x) { return (x + 15) / 16 * 16; }
-__host__ __device__ inline Layout layout(int m, int C, int tsz) {
+__host__ __device__ inline Layout layout(int m, int Ct, int tsz) {
   Layout L;
-  const int ncl = (m + C - 1) / C;
+  const int ncl = (m + Ct - 1) / Ct;
   size_t o = 0;
-  const size_t stage = (size_t)8 * ((m + 31) & ~31);  // 8 staged reflectors of the back-transform
+  const size_t stage = (size_t)4 * ((m + 127) & ~127);  // staged reflectors of the back-transform, two by two
   L.a = o;   o = align16(o + ((size_t)ncl * m > stage ? (size_t)ncl * m : stage) * tsz);  // owned columns
-  L.v = o;   o = align16(o + 2 * (size_t)m * tsz);    // Householder vector, double-buffered
-  L.p = o;   o = align16(o + (size_t)m * tsz);        // p = tau A v, all entries
-  L.s = o;   o = align16(o + 2 * kMaxCluster * (size_t)tsz);  // per-CTA partials of p^H v
-  L.sc = o;  o = align16(o + 2 * 4 * sizeof(double)); // tau (re, im), d_k, e_k per parity
+  L.v = o;   o = align16(o + 2 * (size_t)m * tsz);    // Householder vectors of this and the last step
+  L.p = o;   o = align16(o + (size_t)m * tsz);        // p = tau A v (one CTA)
+  L.c = o;   o = align16(o + (size_t)m * tsz);        // the column to be reflected next
   L.d = o;   o = align16(o + (size_t)m * sizeof(double));
   L.e2 = o;  o = align16(o + (size_t)m * sizeof(double));
-  L.tau = o; o = align16(o + 2 * (size_t)m * tsz);  // tau of every step, then w of the current step
+  L.tau = o; o = align16(o + 2 * (size_t)m * tsz);  // tau of every step, then w of the last step
   L.eig = o; o = align16(o + (size_t)m * sizeof(double));
   L.grp = o; o = align16(o + (size_t)(m + 1) * sizeof(int));
-  L.red = o; o = align16(o + 2 * kWarps * (size_t)tsz);
-  L.hh = o;  o = align16(o + 8 * sizeof(double));
+  L.red = o; o = align16(o + kWarps * (size_t)tsz);
   L.total = o;
   return L;
 }
 
-// Number of eigenvalues of the tridiagonal (d, e2 = e^2 >= 1e-40, scaled to
+// Number of eigenvalues of the tridiagonal (d, ne2 = -e^2 <= -1e-40, scaled to
 // ||T|| <= 1) below x: sign changes of the three-term sequence of
-// det(T - x I).  A zero term counts as a sign change (the zero pivot of the
-// LDL^T count is taken as negative) and cannot repeat, since e2 > 0; with
-// ||T|| <= 1 a term grows by at most 3x a step, so the power-of-two
-// rescaling is checked once every eight steps.  The value chain is one
-// fused multiply-add per step; d and e2 are read eight at a time.
-__device__ __forceinline__ int sturm_count(const double* __restrict__ d, const double* __restrict__ e2, int m,
+// det(T - x I), read off the sign bits.  A zero term cannot repeat, since
+// e2 > 0, and the term after it has the opposite sign of the one before it,
+// so the pair counts one change whichever sign the zero carries.  With
+// ||T|| <= 1 a term grows by at most 3x a step, so the power-of-two rescaling
+// is checked once every eight steps.  The value chain is one fused
+// multiply-add per step; the loop is bound by the FP64 pipe (subtract,
+// multiply, FMA per step), so the sign logic stays on the integer pipe.
+__device__ __forceinline__ int sturm_count(const double* __restrict__ d, const double* __restrict__ ne2, int m,
                                            double x) {
   double pp = 1.0, p = d[0] - x;
-  bool sp = p <= 0.0;  // sign of the previous term as counted (a zero counts as negative after a positive)
-  int cnt = sp;
+  int hp = __double2hiint(p);
+  unsigned cnt = (unsigned)hp >> 31;
   int i = 1;
   for (; i + 8 <= m; i += 8) {
     double dd[8], ee[8];
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       dd[u] = d[i + u] - x;
-      ee[u] = e2[i + u - 1];
+      ee[u] = ne2[i + u - 1];
     }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
-      const double pn = fma(dd[u], p, -ee[u] * pp);
-      const bool sn = pn == 0.0 ? !sp : pn < 0.0;
-      cnt += sn != sp;
-      sp = sn;
+      const double pn = fma(dd[u], p, ee[u] * pp);
+      const int hn = __double2hiint(pn);
+      cnt += (unsigned)(hn ^ hp) >> 31;
+      hp = hn;
       pp = p;
       p = pn;
     }
@@ -175,23 +162,28 @@ __device__ __forceinline__ int sturm_count(const double* __restrict__ d, const d
     }
   }
   for (; i < m; ++i) {
-    const double pn = fma(d[i] - x, p, -e2[i - 1] * pp);
-    const bool sn = pn == 0.0 ? !sp : pn < 0.0;
-    cnt += sn != sp;
-    sp = sn;
+    const double pn = fma(d[i] - x, p, ne2[i - 1] * pp);
+    const int hn = __double2hiint(pn);
+    cnt += (unsigned)(hn ^ hp) >> 31;
+    hp = hn;
     pp = p;
     p = pn;
   }
-  return cnt;
+  return (int)cnt;
 }
 
-// Offset (in doubles) of the Gram blocks in the work buffer: after the 7 m nev
-// doubles of phase 3, rounded up to 32 bytes so that complex entries are aligned.
-__host__ __device__ inline size_t gram_offset(int m, int nev) { return ((size_t)7 * m * nev + 3) / 4 * 4; }
-// Offset of the reflectors copied out of shared memory (m x m, complex size): after the Gram blocks.
-__host__ __device__ inline size_t vglob_offset(int m, int nev) {
-  return gram_offset(m, nev) + (size_t)128 * ((m + 3) / 4 + 1);
+// Offset (in doubles) of the reflectors in the work buffer (m x m, complex size): after the 7 m nev doubles of
+// phase 3, rounded up to 32 bytes so that complex entries are aligned.
+__host__ __device__ inline size_t vglob_offset(int m, int nev) { return ((size_t)7 * m * nev + 3) / 4 * 4; }
+// Offset of the exchange buffers of the tridiagonalisation (4 m + 2 x 16 CTAs x 16 warps entries), and of the
+// eigenvectors' norms (m) after them.
+__host__ __device__ inline size_t xchg_offset(int m, int nev) { return vglob_offset(m, nev) + (size_t)2 * m * m; }
+__host__ __device__ inline size_t norm_offset(int m, int nev) {
+  return xchg_offset(m, nev) + 2 * ((size_t)4 * m + 2 * kMaxCluster * kWarps);
 }
+
+__device__ __forceinline__ double ldcg(const double* p) { return __ldcg(p); }
+__device__ __forceinline__ double2 ldcg(const double2* p) { return __ldcg(p); }
 
 // Seeded start vector entry in [-1, 1).
 __device__ __forceinline__ double start_entry(int i, int j) {
@@ -212,249 +204,428 @@ template <> __device__ __forceinline__ double2 shfl_xor<double2>(double2 v, int 
   return make_double2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
 }
 
+// x - a b, as fused multiply-adds
+__device__ __forceinline__ double nmadd(double x, double a, double b) { return fma(-a, b, x); }
+__device__ __forceinline__ double2 nmadd(double2 x, double2 a, double2 b) {
+  return make_double2(fma(a.y, b.y, fma(-a.x, b.x, x.x)), fma(-a.y, b.x, fma(-a.x, b.y, x.y)));
+}
+
+// Sum over the warp in every lane, on the FP64 tensor core: the 8 x 8 x 4 product with a matrix of ones adds
+// the four lanes of a column of B, the two entries a lane gets back are added, and a second product adds the four
+// distinct values left (two products and one addition against five shuffle-and-add stages).
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+__device__ __forceinline__ double warp_all(double v) {
+  double c[2] = {0.0, 0.0}, d[2] = {0.0, 0.0};
+  dmma(c, 1.0, v);
+  dmma(d, 1.0, c[0] + c[1]);
+  return d[0];
+}
+__device__ __forceinline__ double2 warp_all(double2 v) { return make_double2(warp_all(v.x), warp_all(v.y)); }
+
+__device__ __forceinline__ double pick(bool c, double a, double b) { return c ? a : b; }
+__device__ __forceinline__ double2 pick(bool c, double2 a, double2 b) {
+  return make_double2(c ? a.x : b.x, c ? a.y : b.y);
+}
+
+// v[0 .. 3] summed over the warp: lanes 8 q .. 8 q + 7 hold the sum of v[q].
+template <typename T> __device__ __forceinline__ T warp_sum4(T (&v)[4], int lane) {
+  const bool hi = lane & 16, h8 = lane & 8;
+  const T v0 = v[0], v1 = v[1], v2 = v[2], v3 = v[3];
+  const T a = add(pick(hi, v2, v0), shfl_xor(pick(hi, v0, v2), 16));
+  const T b = add(pick(hi, v3, v1), shfl_xor(pick(hi, v1, v3), 16));
+  T c = add(pick(h8, b, a), shfl_xor(pick(h8, a, b), 8));
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) c = add(c, shfl_xor(c, o));
+  return c;
+}
+
+// tau, 1 / (alpha - beta) and beta of the reflector of a column whose entry
+// below the diagonal is alpha and whose further entries have the squared norm s2.
+template <typename T> __device__ __forceinline__ void reflector(T alpha, double s2, T& tau, T& scale, double& beta) {
+  const double ar = re(alpha), ai = im(alpha);
+  double tr = 0.0, ti = 0.0, sr = 0.0, si = 0.0;
+  beta = ar;
+  if (s2 > 0.0 || ai != 0.0) {
+    const double x = ar * ar + ai * ai + s2;
+    double ib;
+    if (x > 1e-290 && x < 1e290) {
+      const double r = rsqrt(x);
+      beta = ar >= 0.0 ? -x * r : x * r;
+      ib = ar >= 0.0 ? -r : r;
+    } else {
+      beta = ar >= 0.0 ? -sqrt(x) : sqrt(x);
+      ib = 1.0 / beta;
+    }
+    tr = (beta - ar) * ib;
+    ti = -ai * ib;
+    const double dr = ar - beta, iden = 1.0 / (dr * dr + ai * ai);
+    sr = dr * iden;
+    si = -ai * iden;
+  }
+  tau = mk<T>(tr, ti);
+  scale = mk<T>(sr, si);
+}
+
+// Tridiagonalisation of the m x m matrix a (shared memory) by one CTA, m <= 32 RPL: every warp keeps the vectors
+// of a step (rows lane + 32 u) in its registers and forms w, the next column and its norm for itself, so a step has
+// two block barriers and three warp-wide sums on its path.  Columns are spread over the warps four at a time; vs
+// (2 m) and ws (m) carry v and w for the broadcast of their entries at the column index, pb (m) the entries of p.
+template <typename T, int RPL>
+__device__ void tridiag_one(T* a, int m, T* vs, T* ws, T* pb, double* dv, double* ev_off, T* tauv, T* vglob) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const T z0 = mk<T>(0.0, 0.0);
+  T c[RPL], v[RPL], vp[RPL], w[RPL];
+#pragma unroll
+  for (int u = 0; u < RPL; ++u) {
+    const int i = lane + 32 * u;
+    c[u] = i < m ? a[i] : z0;
+    vp[u] = w[u] = z0;
+    if (warp == 0 && i < m) ws[i] = vs[m + i] = z0;
+  }
+  for (int k = 0; k < m - 1; ++k) {
+    const int par = k & 1;
+    // reflector of column k
+    double s2 = 0.0;
+    T ca = z0, cd = z0;
+#pragma unroll
+    for (int u = 0; u < RPL; ++u) {
+      const int i = lane + 32 * u;
+      if (i >= k + 2) s2 += abs2(c[u]);
+      ca = pick(u == (k + 1) >> 5, c[u], ca);
+      cd = pick(u == k >> 5, c[u], cd);
+    }
+    s2 = warp_all(s2);
+    ca = shfl(ca, (k + 1) & 31);
+    T tau, scale;
+    double beta;
+    reflector(ca, s2, tau, scale, beta);
+#pragma unroll
+    for (int u = 0; u < RPL; ++u) {
+      const int i = lane + 32 * u;
+      v[u] = i > k + 1 ? mul(c[u], scale) : mk<T>(i == k + 1 ? 1.0 : 0.0, 0.0);
+      if (warp == 0 && i < m) vs[par * m + i] = v[u];
+      if (warp == 1 && i < m) vglob[(size_t)k * m + i] = v[u];
+    }
+    if (warp == 0 && lane == (k & 31)) {
+      dv[k] = re(cd);
+      ev_off[k] = beta;
+      tauv[k] = tau;
+    }
+    __syncthreads();
+    // rank-2 update of the last step and p = tau A v on the updated columns
+    const T* vq = vs + (par ^ 1) * m;
+    const int u0 = (k + 1) >> 5;
+    for (int j0 = k + 1 + warp * 4; j0 < m; j0 += kWarps * 4) {
+      T acc[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        acc[q] = z0;
+        const int j = j0 + q;
+        if (j < m) {
+          T* col = a + (size_t)j * m;
+          const T cw = cj(ws[j]), cv = cj(vq[j]);
+#pragma unroll
+          for (int u = 0; u < RPL; ++u) {
+            const int i = lane + 32 * u;
+            if (u < u0 || i >= m) continue;
+            const T x = sub(col[i], add(mul(vp[u], cw), mul(w[u], cv)));
+            col[i] = x;
+            acc[q] = add(acc[q], mul(cj(x), v[u]));
+          }
+        }
+      }
+      const T s = warp_sum4(acc, lane);
+      const int j = j0 + (lane >> 3);
+      if ((lane & 7) == 0 && j < m) pb[j] = mul(tau, s);
+    }
+    __syncthreads();
+    // w = p + alpha v and column k + 1
+    T p[RPL];
+    T ssum = z0;
+#pragma unroll
+    for (int u = 0; u < RPL; ++u) {
+      const int i = lane + 32 * u;
+      const bool in = i > k && i < m;
+      p[u] = in ? pb[i] : z0;
+      c[u] = in ? a[(size_t)(k + 1) * m + i] : z0;
+      ssum = add(ssum, mul(cj(p[u]), v[u]));
+    }
+    const T al = mul(mul(tau, warp_all(ssum)), -0.5);
+    const T cwk = cj(add(pb[k + 1], al));
+#pragma unroll
+    for (int u = 0; u < RPL; ++u) {
+      const int i = lane + 32 * u;
+      w[u] = add(p[u], mul(al, v[u]));
+      c[u] = sub(c[u], add(mul(v[u], cwk), w[u]));
+      vp[u] = v[u];
+      if (warp == 0 && i < m) ws[i] = w[u];
+    }
+  }
+  if (warp == 0) {
+#pragma unroll
+    for (int u = 0; u < RPL; ++u)
+      if (lane + 32 * u == m - 1) dv[m - 1] = re(c[u]);
+  }
+}
+constexpr int kOneMaxReal = 128, kOneMaxCplx = 64;  // sizes of tridiag_one
+
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_eigh_cluster(const T* __restrict__ A, long lda, int m, int nev, double* __restrict__ w_out, T* __restrict__ Z,
-                   long ldz, double* __restrict__ work, int* __restrict__ status) {
+    k_eigh_cluster(const T* __restrict__ A, long lda, int m, int nev, int Ct, double gtol, double* __restrict__ w_out,
+                   T* __restrict__ Z, long ldz, double* __restrict__ work, int* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem[];
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks();
   const int rank = (int)cluster.block_rank();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const Layout L = layout(m, C, (int)sizeof(T));
+  const Layout L = layout(m, Ct, (int)sizeof(T));
   T* a_loc = reinterpret_cast<T*>(smem + L.a);
   T* vbuf = reinterpret_cast<T*>(smem + L.v);
   T* pbuf = reinterpret_cast<T*>(smem + L.p);
-  T* sbuf = reinterpret_cast<T*>(smem + L.s);
-  double* scal = reinterpret_cast<double*>(smem + L.sc);
+  T* cbuf = reinterpret_cast<T*>(smem + L.c);
   double* dv = reinterpret_cast<double*>(smem + L.d);
   double* e2v = reinterpret_cast<double*>(smem + L.e2);
   T* tauv = reinterpret_cast<T*>(smem + L.tau);
   double* eig = reinterpret_cast<double*>(smem + L.eig);
   int* grp = reinterpret_cast<int*>(smem + L.grp);
   T* red = reinterpret_cast<T*>(smem + L.red);
-  double* hh = reinterpret_cast<double*>(smem + L.hh);
   __shared__ double ev_off[kMaxM];  // off-diagonal e_k (the signed beta of each step)
+  __shared__ double s2_part[kWarps];  // per-warp partial sums of the squared norm of the next column
   __shared__ double tnorm_s;
   __shared__ int bad;
   __shared__ int ngrp;
-  const int nown = (m - rank + C - 1) / C;  // columns rank, rank + C, ... below m
-  const int lgC = __ffs(C) - 1;              // C is a power of two
-  T* wbuf = tauv + m;                        // w = p + alpha v of the current step
+  const int nown = rank < Ct ? (m - rank + Ct - 1) / Ct : 0;  // columns rank, rank + Ct, ... below m
+  const int lgCt = __ffs(Ct) - 1;                             // Ct is a power of two
 
   EIGH_MARK(0);
   if (tid == 0) bad = 0;
-  for (int s = 0; s < nown; ++s) {
-    const T* src = A + (long)(rank + s * C) * lda;
-    for (int i = tid; i < m; i += kThreads) a_loc[(size_t)s * m + i] = src[i];
+  for (int e = tid; e < nown * m; e += kThreads) {
+    const int sl = e / m, i = e - sl * m;
+    a_loc[e] = A[(long)(rank + sl * Ct) * lda + i];
   }
-  cluster.sync();  // every CTA has started and loaded its columns
+  __syncthreads();
+  if (Ct > 1) cluster.sync();  // every CTA has started
   EIGH_MARK(1);
 
-  // ---- 1. Householder tridiagonalisation ----
-  // Exchanges are pulled, never pushed.  The reflector of a step goes
-  // through L2: its owner writes it to the reflector store in global memory
-  // (which the back-transform reads anyway) and the other CTAs read it from
-  // there, because fifteen CTAs pulling one CTA's shared memory measured
-  // ~5 us a step at m = 540 against well under 1 us from L2.  The entries of
-  // p (spread over all CTAs) and the step's scalars are remote shared-memory
-  // loads; remote stores are several times slower than either.
-  // Reflector of column kk, by all threads of its owner: v into the column
-  // (leading 1) and into the store, (tau, d_kk, e_kk) into the owner's scal
-  // of parity kk & 1.
-  T* vglob_w = reinterpret_cast<T*>(work + vglob_offset(m, nev));
-  __shared__ double s2_part[kWarps];  // per-warp partial sums of |col[i]|^2, rows >= kk + 2
-  // have_parts: s2_part already holds the partials (summed while the column was updated)
-  auto house = [&](int kk, bool have_parts) {
-    T* col = a_loc + (size_t)(kk >> lgC) * m;
-    if (warp == 0) {
+  // ---- 1. Householder tridiagonalisation on the first Ct CTAs ----
+  // One cluster barrier per column.  Every CTA keeps the whole of v and w and
+  // forms each reflector itself (the same operations in the same order, so the
+  // copies agree bit for bit).  Step k:
+  //   b  reflector v_k of column k (cbuf, updated through step k - 1)
+  //   c  one pass over the owned columns j > k: the rank-2 update of step
+  //      k - 1 and, on the updated entries, p_j = tau (A v)_j; a warp takes
+  //      kColBlk columns at once, so v, v_prev and w are read once for them
+  //   -  exchange through L2: entries of p, partials of p^H v, column k + 1
+  //   a  w = p + alpha v, column k + 1 updated by this step, its norm
+  // The exchange buffers alternate with the parity of k: a CTA writes a
+  // parity again only after a barrier that every reader of it has passed.
+  {
+    T* xp = reinterpret_cast<T*>(work + xchg_offset(m, nev));  // [parity][m] entries of p
+    T* xc = xp + 2 * m;                                        // [parity][m] column k + 1
+    T* xs = xc + 2 * m;                                        // [parity][CTA][warp] partials of p^H v
+    T* vglob_w = reinterpret_cast<T*>(work + vglob_offset(m, nev));
+    T* wbuf = tauv + m;
+    constexpr int kColBlk = sizeof(T) == sizeof(double) ? 3 : 2;
+    const bool one = Ct == 1 && m <= (sizeof(T) == sizeof(double) ? kOneMaxReal : kOneMaxCplx);
+    if (one && rank == 0) {
+      if (m <= 32) tridiag_one<T, 1>(a_loc, m, vbuf, wbuf, pbuf, dv, ev_off, tauv, vglob_w);
+      else if (m <= 64) tridiag_one<T, 2>(a_loc, m, vbuf, wbuf, pbuf, dv, ev_off, tauv, vglob_w);
+      else if (sizeof(T) == sizeof(double)) tridiag_one<T, 4>(a_loc, m, vbuf, wbuf, pbuf, dv, ev_off, tauv, vglob_w);
+    }
+    if (!one && rank < Ct) {
       double s2 = 0.0;
-      if (have_parts) {
-        s2 = lane < kWarps ? s2_part[lane] : 0.0;
-      } else {
-        for (int i = kk + 2 + lane; i < m; i += 32) s2 += abs2(col[i]);
+      for (int i = tid; i < m; i += kThreads) {
+        const T x = A[i];
+        cbuf[i] = x;
+        wbuf[i] = mk<T>(0.0, 0.0);
+        vbuf[m + i] = mk<T>(0.0, 0.0);
+        if (i >= 2) s2 += abs2(x);
       }
       s2 = warp_sum(s2);
-      if (lane == 0) {
-        const T alpha = col[kk + 1];
-        const double ar = re(alpha), ai = im(alpha);
-        double tr = 0.0, ti = 0.0, beta = ar, sr = 0.0, si = 0.0;
-        if (s2 > 0.0 || ai != 0.0) {
-          const double nrm = sqrt(ar * ar + ai * ai + s2);
-          beta = ar >= 0.0 ? -nrm : nrm;
-          const double ib = 1.0 / beta;
-          tr = (beta - ar) * ib;
-          ti = -ai * ib;
-          const double dr = ar - beta, di = ai, iden = 1.0 / (dr * dr + di * di);  // scale = 1 / (alpha - beta)
-          sr = dr * iden;
-          si = -di * iden;
-        }
-        double* sc2 = scal + 4 * (kk & 1);
-        sc2[0] = tr;
-        sc2[1] = ti;
-        sc2[2] = re(col[kk]);
-        sc2[3] = beta;
-        hh[0] = sr;
-        hh[1] = si;
-      }
-    }
-    __syncthreads();
-    const double* sc2 = scal + 4 * (kk & 1);
-    const bool rf = sc2[0] != 0.0 || sc2[1] != 0.0;
-    const T scale = mk<T>(hh[0], hh[1]);
-    T* vg = vglob_w + (size_t)kk * m;
-    for (int i = kk + 1 + tid; i < m; i += kThreads) {
-      const T x = i == kk + 1 ? mk<T>(1.0, 0.0) : (rf ? mul(col[i], scale) : mk<T>(0.0, 0.0));
-      col[i] = x;
-      vg[i] = x;
-    }
-  };
-
-  // B1 of a step is split: the owner of the next column arrives as soon as
-  // its reflector is out and updates its other columns afterwards, so that
-  // update is off the path the other CTAs wait on; the rest arrive after
-  // their update.  B2 is a full cluster barrier.
-  if (m > 1 && rank == 0) house(0, false);
-  cluster_arrive();
-  EIGH_SUB_DECL
-  for (int k = 0; k < m - 1; ++k) {
-    const int par = k & 1;
-    const int owner = k & (C - 1);
-    EIGH_SUB(0);
-    cluster_wait();  // B1: the reflector of column k is in the store and its owner's scal
-    EIGH_SUB(1);
-    // pull v (rows k+1 .. m-1) and the step's scalars from the owner
-    const T* vb;
-    if (owner == rank) {
-      vb = a_loc + (size_t)(k >> lgC) * m;
-    } else {
-      const T* src = vglob_w + (size_t)k * m;  // written before B1 by the owner; read past L1
-      for (int i = k + 1 + tid; i < m; i += kThreads) vbuf[i] = __ldcg(src + i);
-      if (tid < 4) scal[4 * par + tid] = cluster.map_shared_rank(scal, owner)[4 * par + tid];
-      vb = vbuf;
+      if (lane == 0) s2_part[warp] = s2;
       __syncthreads();
     }
-    const double* sc = scal + 4 * par;
-    const T tau = mk<T>(sc[0], sc[1]);
-    const bool refl = sc[0] != 0.0 || sc[1] != 0.0;
-    if (tid == 0) {
-      dv[k] = sc[2];
-      ev_off[k] = sc[3];
-      tauv[k] = tau;
-    }
-    const int s0 = k + 1 > rank ? (k + 1 - rank + C - 1) >> lgC : 0;  // first owned slot with column > k
-    const int na = nown - s0;
-    const bool look = k + 1 < m - 1 && rank == ((k + 1) & (C - 1));  // this CTA reflects column k + 1 next
-    // R lanes per owned column (a power of two dividing 32)
-    int R = 32;
-    while (R > 1 && na * R > kThreads) R >>= 1;
-    const int r = lane & (R - 1);
-    const int gpw = 32 / R;  // column groups per warp
-    if (refl) {
-      // p_j = tau sum_i conj(A[i, j]) v_i for owned j > k, R lanes per column; partials of p^H v
-      T part = mk<T>(0.0, 0.0);
-      for (int gb = warp * gpw; gb < na; gb += kWarps * gpw) {
-        const int g = gb + lane / R;
-        const bool act = g < na;
-        const int sl = s0 + (act ? g : 0);
-        const T* col = a_loc + (size_t)sl * m;
-        T acc0 = mk<T>(0.0, 0.0), acc1 = mk<T>(0.0, 0.0), acc2 = mk<T>(0.0, 0.0), acc3 = mk<T>(0.0, 0.0);
-        if (act) {
-          int i = k + 1 + r;
-          for (; i + 3 * R < m; i += 4 * R) {
-            acc0 = add(acc0, mul(cj(col[i]), vb[i]));
-            acc1 = add(acc1, mul(cj(col[i + R]), vb[i + R]));
-            acc2 = add(acc2, mul(cj(col[i + 2 * R]), vb[i + 2 * R]));
-            acc3 = add(acc3, mul(cj(col[i + 3 * R]), vb[i + 3 * R]));
+    const int kend = !one && rank < Ct ? m - 1 : 0;
+    for (int k = 0; k < kend; ++k) {
+      const int par = k & 1;
+      {
+        // b: beta, tau and the scale 1 / (alpha - beta), by every thread
+        T* v = vbuf + par * m;
+        const T* vp = vbuf + (par ^ 1) * m;
+        T tau, scale;
+        {
+          const double s2 = warp_all(lane < kWarps ? s2_part[lane] : 0.0);
+          const T alpha = cbuf[k + 1];
+          double beta;
+          reflector(alpha, s2, tau, scale, beta);
+          if (tid == 0) {
+            dv[k] = re(cbuf[k]);
+            ev_off[k] = beta;
+            tauv[k] = tau;
           }
-          for (; i < m; i += R) acc0 = add(acc0, mul(cj(col[i]), vb[i]));
         }
-        T acc = add(add(acc0, acc1), add(acc2, acc3));
-        for (int o = R / 2; o > 0; o >>= 1) acc = add(acc, shfl_xor(acc, o));
-        if (act && r == 0) {
-          const int j = rank + (sl << lgC);
-          const T pj = mul(tau, acc);
-          pbuf[j] = pj;
-          part = add(part, mul(cj(pj), vb[j]));
+        const bool store = rank == (k & (Ct - 1));
+        for (int i = tid; i < m; i += kThreads) {
+          T x = mk<T>(0.0, 0.0);
+          if (i == k + 1) x = mk<T>(1.0, 0.0);
+          if (i > k + 1) x = mul(cbuf[i], scale);
+          if (i > k) v[i] = x;
+          if (store) vglob_w[(size_t)k * m + i] = x;  // zero above the support, for the back-transform
         }
-      }
-      EIGH_SUB(2);
-      part = warp_sum(part);
-      if (lane == 0) red[warp] = part;
-      __syncthreads();
-      if (warp == 0) {
-        const T tot = warp_sum(lane < kWarps ? red[lane] : mk<T>(0.0, 0.0));
-        if (lane == 0) sbuf[kMaxCluster * par + rank] = tot;
-      }
-      EIGH_SUB(3);
-      cluster.sync();  // B2: every CTA's entries of p and partial of p^H v are in place
-      EIGH_SUB(4);
-      // pull the other partials, then w = p + alpha v over rows k+1 .. m-1 into pbuf (entries of p
-      // owned elsewhere pulled on the way)
-      if (tid < C && tid != rank)
-        sbuf[kMaxCluster * par + tid] = cluster.map_shared_rank(sbuf, tid)[kMaxCluster * par + tid];
-      __syncthreads();
-      T ssum = mk<T>(0.0, 0.0);
-      for (int q = 0; q < C; ++q) ssum = add(ssum, sbuf[kMaxCluster * par + q]);
-      const T alpha = mul(mul(tau, ssum), -0.5);
-      for (int i = k + 1 + tid; i < m; i += kThreads) {
-        const int q = i & (C - 1);
-        const T pi = q == rank ? pbuf[i] : cluster.map_shared_rank(pbuf, q)[i];
-        wbuf[i] = add(pi, mul(alpha, vb[i]));
-      }
-      __syncthreads();
-      EIGH_SUB(5);
-      if (look) {
-        // column k + 1 first, so that its reflector is ready early
-        // (with the norm its reflector needs summed on the way)
-        T* col = a_loc + (size_t)((k + 1) >> lgC) * m;
-        const T cwj = cj(wbuf[k + 1]), cvj = cj(vb[k + 1]);
+        __syncthreads();
+        // c
+        const int s0 = k + 1 > rank ? (k + 1 - rank + Ct - 1) >> lgCt : 0;  // first owned slot with column > k
+        const int na = nown - s0;
+        T part = mk<T>(0.0, 0.0);
+        T* pout = Ct > 1 ? xp + par * m : pbuf;
+        const int i0 = ((k + 1) & ~31) + lane;
+        // columns a warp: as many as spread the owned ones over all warps, kColBlk at most
+        const int cb = na <= kWarps ? 1 : (na <= 2 * kWarps ? 2 : kColBlk);
+        for (int g = warp * cb; g < na; g += kWarps * cb) {
+          T* col[kColBlk];
+          T cw[kColBlk], cv[kColBlk], acc[kColBlk];
+          const int nc = min(cb, na - g);
+#pragma unroll
+          for (int q = 0; q < kColBlk; ++q) {
+            const int sl = s0 + g + (q < nc ? q : 0), j = rank + sl * Ct;
+            col[q] = a_loc + (size_t)sl * m;
+            cw[q] = cj(wbuf[j]);
+            cv[q] = cj(vp[j]);
+            acc[q] = mk<T>(0.0, 0.0);
+          }
+          T* xo = g == 0 && rank + s0 * Ct == k + 1 && Ct > 1 ? xc + par * m : nullptr;  // column k + 1 goes to the others
+          // rows kUn chunks of 32 at a time, their loads ahead of the arithmetic
+          constexpr int kUn = sizeof(T) == sizeof(double) ? 4 : 2;
+          int i = i0;
+          for (; i + 32 * (kUn - 1) < m; i += 32 * kUn) {
+            T vi[kUn], pi[kUn], wi[kUn], x[kUn];
+#pragma unroll
+            for (int u = 0; u < kUn; ++u) {
+              const bool in = i + 32 * u > k;  // rows above the step's range stay as they are
+              vi[u] = in ? v[i + 32 * u] : mk<T>(0.0, 0.0);
+              pi[u] = in ? vp[i + 32 * u] : mk<T>(0.0, 0.0);
+              wi[u] = in ? wbuf[i + 32 * u] : mk<T>(0.0, 0.0);
+            }
+#pragma unroll
+            for (int q = 0; q < kColBlk; ++q) {
+              if (q >= nc) break;
+#pragma unroll
+              for (int u = 0; u < kUn; ++u) x[u] = col[q][i + 32 * u];
+#pragma unroll
+              for (int u = 0; u < kUn; ++u) {
+                x[u] = sub(x[u], add(mul(pi[u], cw[q]), mul(wi[u], cv[q])));
+                col[q][i + 32 * u] = x[u];
+                acc[q] = add(acc[q], mul(cj(x[u]), vi[u]));
+                if (q == 0 && xo) xo[i + 32 * u] = x[u];
+              }
+            }
+          }
+          for (; i < m; i += 32) {
+            if (i <= k) continue;
+            const T vi = v[i], pi = vp[i], wi = wbuf[i];
+#pragma unroll
+            for (int q = 0; q < kColBlk; ++q) {
+              if (q >= nc) break;
+              const T x = sub(col[q][i], add(mul(pi, cw[q]), mul(wi, cv[q])));
+              col[q][i] = x;
+              acc[q] = add(acc[q], mul(cj(x), vi));
+              if (q == 0 && xo) xo[i] = x;
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < kColBlk; ++q) {
+            if (q >= nc) break;
+            const int j = rank + (s0 + g + q) * Ct;
+            const T pj = mul(tau, warp_all(acc[q]));
+            if (lane == 0) pout[j] = pj;
+            part = add(part, mul(cj(pj), v[j]));
+          }
+        }
+        if (lane == 0) {
+          if (Ct > 1) xs[(par * kMaxCluster + rank) * kWarps + warp] = part;
+          else red[warp] = part;
+        }
+        if (Ct > 1) {
+          cluster_arrive();
+          cluster_wait();
+        } else {
+          __syncthreads();
+        }
+        // a
+        T ssum = mk<T>(0.0, 0.0);
+        const T* pin = Ct > 1 ? xp + par * m : pbuf;
+        T pk1;
+        if (Ct > 1) {
+          const T* sx = xs + par * kMaxCluster * kWarps;
+          T pt[kMaxCluster * kWarps / 32];
+#pragma unroll
+          for (int u = 0; u < kMaxCluster * kWarps / 32; ++u)
+            pt[u] = lane + 32 * u < Ct * kWarps ? ldcg(sx + lane + 32 * u) : mk<T>(0.0, 0.0);
+          pk1 = ldcg(pin + k + 1);
+#pragma unroll
+          for (int u = 0; u < kMaxCluster * kWarps / 32; ++u) ssum = add(ssum, pt[u]);
+        } else {
+          if (lane < kWarps) ssum = red[lane];
+          pk1 = pin[k + 1];
+        }
+        T ci[kRowsPerThread], pi[kRowsPerThread];
+#pragma unroll
+        for (int u = 0; u < kRowsPerThread; ++u) {
+          const int i = k + 1 + tid + u * kThreads;
+          ci[u] = pi[u] = mk<T>(0.0, 0.0);
+          if (i < m) {
+            ci[u] = Ct > 1 ? ldcg(xc + par * m + i) : a_loc[(size_t)(k + 1) * m + i];
+            pi[u] = Ct > 1 ? ldcg(pin + i) : pin[i];
+          }
+        }
+        const T al = mul(mul(tau, warp_all(ssum)), -0.5);
+        const T cwk = cj(add(pk1, al));  // conj(w_{k+1}); v_{k+1} = 1
         double s2 = 0.0;
-        for (int i = k + 1 + tid; i < m; i += kThreads) {
-          const T x = sub(col[i], add(mul(vb[i], cwj), mul(wbuf[i], cvj)));
-          col[i] = x;
+#pragma unroll
+        for (int u = 0; u < kRowsPerThread; ++u) {
+          const int i = k + 1 + tid + u * kThreads;
+          if (i >= m) break;
+          const T vi = v[i], wi = add(pi[u], mul(al, vi));
+          const T x = sub(ci[u], add(mul(vi, cwk), wi));
+          wbuf[i] = wi;
+          cbuf[i] = x;
           if (i >= k + 3) s2 += abs2(x);
         }
-        s2 = warp_sum(s2);
+        s2 = warp_all(s2);
         if (lane == 0) s2_part[warp] = s2;
         __syncthreads();
-        house(k + 1, true);
-        cluster_arrive();
       }
-      EIGH_SUB(6);
-      for (int gb = warp * gpw; gb < na; gb += kWarps * gpw) {
-        const int g = gb + lane / R;
-        if (g >= na) continue;
-        const int sl = s0 + g;
-        const int j = rank + (sl << lgC);
-        if (look && j == k + 1) continue;
-        T* col = a_loc + (size_t)sl * m;
-        const T cwj = cj(wbuf[j]), cvj = cj(vb[j]);
-#pragma unroll 4
-        for (int i = k + 1 + r; i < m; i += R) col[i] = sub(col[i], add(mul(vb[i], cwj), mul(wbuf[i], cvj)));
-      }
-    } else if (look) {
-      house(k + 1, false);
-      cluster_arrive();
     }
-    __syncthreads();
-    if (!look) cluster_arrive();
-    EIGH_SUB(7);
+    if (tid == 0) ev_off[m - 1] = 0.0;
+    if (tid == 0 && !one && rank < Ct) dv[m - 1] = re(cbuf[m - 1]);
+    if (Ct < C) {
+      // the CTAs that took no part read T and tau through L2
+      double* xt = reinterpret_cast<double*>(xp);  // free now: d, e, then tau
+      T* xtau = xp + m;
+      __syncthreads();
+      if (rank == 0)
+        for (int i = tid; i < m; i += kThreads) {
+          xt[i] = dv[i];
+          if (sizeof(T) == sizeof(double)) xc[i] = mk<T>(ev_off[i], 0.0);
+          else xt[m + i] = ev_off[i];
+          xtau[i] = i < m - 1 ? tauv[i] : mk<T>(0.0, 0.0);
+        }
+      cluster.sync();
+      if (rank >= Ct)
+        for (int i = tid; i < m; i += kThreads) {
+          dv[i] = __ldcg(xt + i);
+          ev_off[i] = sizeof(T) == sizeof(double) ? __ldcg(reinterpret_cast<double*>(xc) + i) : __ldcg(xt + m + i);
+          tauv[i] = ldcg(xtau + i);
+        }
+      __syncthreads();
+    } else {
+      cluster.sync();
+    }
   }
-  cluster_wait();  // completes the last arrival
-  EIGH_SUB_STORE;
-  // the reflector store complete (column k holds v_k on rows k+1 .. m-1, zero above), for the back-transform
-  for (int sl = 0; sl < nown; ++sl) {
-    const int k = rank + sl * C;
-    const T* col = a_loc + (size_t)sl * m;
-    for (int i = tid; i < m; i += kThreads) vglob_w[(size_t)k * m + i] = i > k ? col[i] : mk<T>(0.0, 0.0);
-  }
-  // last diagonal entry
-  if (rank == (m - 1) % C && tid == 0) dv[m - 1] = re(a_loc[(size_t)((m - 1) / C) * m + (m - 1)]);
-  if (tid == 0) ev_off[m - 1] = 0.0;
-  cluster.sync();
-  if (rank != (m - 1) % C && tid == 0) dv[m - 1] = re(cluster.map_shared_rank(a_loc, (m - 1) % C)[(size_t)((m - 1) / C) * m + (m - 1)]);
-  cluster.sync();
   EIGH_MARK(2);
 
   // ---- 2. eigenvalues by multisection on T / ||T|| ----
@@ -482,7 +653,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     ev_off[i] *= itn;
     // an off-diagonal below 1e-20 ||T|| counts as 1e-20 in the Sturm sequence, so a zero term never
     // propagates (a perturbation far below rounding)
-    e2v[i] = fmax(ev_off[i] * ev_off[i], 1e-40);
+    e2v[i] = -fmax(ev_off[i] * ev_off[i], 1e-40);
   }
   __syncthreads();
   {
@@ -535,6 +706,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     double2* F2 = reinterpret_cast<double2*>(work + (size_t)4 * m * nev);
     double* zt = work + (size_t)6 * m * nev;
     const double piv_min = kEps;
+    double* znorm = work + norm_offset(m, nev);
     const int nj = (nev + C - 1) / C;
     for (int jj = tid; jj < nj; jj += kThreads) {
       const int j = rank * nj + jj;
@@ -610,7 +782,8 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           reinterpret_cast<double*>(&U4[(size_t)(m - 1) * nev + j])[3] = c0;
         }
-        // back-substitution, eight rows per batch of loads
+        // back-substitution, eight rows per batch of loads; the last one writes the vector itself
+        double* zj = zt + (size_t)j * m;
         double y1 = 0.0, y2 = 0.0, nrm2 = 0.0;
         int i = m - 1;
         for (; i >= 7; i -= 8) {
@@ -620,7 +793,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
             const double yi = (u[q].w - u[q].y * y1 - u[q].z * y2) * u[q].x;
-            reinterpret_cast<double*>(&U4[(size_t)(i - q) * nev + j])[3] = yi;
+            if (it == 0) reinterpret_cast<double*>(&U4[(size_t)(i - q) * nev + j])[3] = yi;
+            else zj[i - q] = yi;
             nrm2 += yi * yi;
             y2 = y1;
             y1 = yi;
@@ -629,7 +803,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (; i >= 0; --i) {
           const double4 u = U4[(size_t)i * nev + j];
           const double yi = (u.w - u.y * y1 - u.z * y2) * u.x;
-          reinterpret_cast<double*>(&U4[(size_t)i * nev + j])[3] = yi;
+          if (it == 0) reinterpret_cast<double*>(&U4[(size_t)i * nev + j])[3] = yi;
+          else zj[i] = yi;
           nrm2 += yi * yi;
           y2 = y1;
           y1 = yi;
@@ -638,8 +813,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         scale = okn ? 1.0 / sqrt(nrm2) : 0.0;
         if (!okn) bad = 1;
       }
-      double* zj = zt + (size_t)j * m;
-      for (int i = 0; i < m; ++i) zj[i] = U4[(size_t)i * nev + j].w * scale;
+      znorm[j] = scale;  // applied where the vector is read
     }
   }
   __threadfence();
@@ -651,7 +825,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   {
     double* zt = work + (size_t)6 * m * nev;
     if (tid == 0) {
-      const double gtol = 1e-5;  // in units of ||T||
       int n = 0;
       int start = 0;
       for (int j = 1; j <= nev; ++j) {
@@ -687,116 +860,97 @@ __global__ void __launch_bounds__(kThreads, 1)
         const double scn = n2 > 0.0 ? 1.0 / sqrt(n2) : 0.0;
         if (!(n2 > 0.0) && lane == 0) bad = 1;
         for (int rr = lane; rr < m; rr += 32) zj[rr] *= scn;
+        if (lane == 0) work[norm_offset(m, nev) + j] = 1.0;
         __syncwarp();
       }
     }
-  }
-  // ---- 4a. Gram blocks of the reflectors: G[b][q][p] = v_kq^H v_kp, kq = m-2-BR*b-q, p < q ----
-  constexpr int BR = sizeof(T) == sizeof(double) ? 8 : 4;  // reflectors per round of the back-transform
-  constexpr int NPAIR = BR * (BR - 1) / 2;
-  const int nblk = (m - 1 + BR - 1) / BR;
-  T* gram = reinterpret_cast<T*>(work + gram_offset(m, nev));
-  const T* vglob = reinterpret_cast<const T*>(work + vglob_offset(m, nev));
-  for (int t = gw; t < nblk * NPAIR; t += nw) {
-    const int b = t / NPAIR;
-    int pq = t % NPAIR, q = 1;
-    while (pq >= q) {
-      pq -= q;
-      ++q;
-    }
-    const int p = pq;  // 0 <= p < q < BR
-    const int k0 = m - 2 - BR * b;
-    const int kq = k0 - q, kp = k0 - p;
-    T acc = mk<T>(0.0, 0.0);
-    if (kq >= 0) {
-      const T* vq = vglob + (size_t)kq * m;
-      const T* vp = vglob + (size_t)kp * m;
-      for (int i = kp + 1 + lane; i < m; i += 32) acc = add(acc, mul(cj(vq[i]), vp[i]));
-    }
-    acc = warp_sum(acc);
-    if (lane == 0) gram[(size_t)b * 64 + q * 8 + p] = acc;
   }
   __threadfence();
   cluster.sync();
   EIGH_MARK(5);
 
-  // ---- 4. back-transform x = H(0) ... H(m-2) z, one warp per vector, BR reflectors per round ----
-  // Each round the CTA stages the round's reflectors (from global memory, where they are L2-resident)
-  // and their Gram block into shared memory; every warp then applies them to its vector in registers.
-  // The staged rows have stride mp (m rounded up to 32) and start zeroed, so rows outside a
-  // reflector's support contribute exact zeros and the inner loops carry no predicates; row slots
-  // wholly below the round's first row, or past m, are skipped (warp-uniform tests).
+  // ---- 4. back-transform x = H(0) ... H(m-2) z, one warp per vector, the vector in registers ----
+  // The reflectors pass through shared memory in chunks, the next chunk copied while one is applied, so a CTA waits
+  // twice a chunk and a warp's path through a reflector is one dot product over the warp and one update.  Rows of
+  // a reflector above its support are zero in the store and the staged rows past m are zeroed once, so the loops
+  // carry no predicates; groups of four row slots wholly above the support or past m are skipped (a test per slot
+  // costs more than the slot's arithmetic).
   {
     const double* zt = work + (size_t)6 * m * nev;
-    const int mp = (m + 31) & ~31;
-    const int nt = mp >> 5;
-    T* sv = a_loc;  // BR x mp staged reflectors (the matrix columns are no longer needed)
-    __shared__ T sgram[64];
-    __shared__ T stau[8];
+    const double* znorm = work + norm_offset(m, nev);
+    const T* vglob = reinterpret_cast<const T*>(work + vglob_offset(m, nev));
+    const int mp = (m + 127) & ~127;
+    const int ng = mp >> 7;
+    const size_t cap = max((size_t)((m + Ct - 1) / Ct) * m, (size_t)4 * mp);  // entries of the column buffer
+    const int R = (int)min((size_t)16, cap / (2 * (size_t)mp));             // reflectors per chunk
+    T* sv = a_loc;
     const int waves = (nev + nw - 1) / nw;
+    const int nchunk = (m - 1 + R - 1) / R;
+    auto stage = [&](int c) {
+      const int k0 = m - 2 - R * c;  // reflectors k0, k0 - 1, ..., k0 - R + 1
+      const int lo = max(0, k0 - R + 2) & ~127;
+      T* dst = sv + (size_t)(c & 1) * R * mp;
+      const int rows = m - lo;
+      for (int e = tid; e < R * rows; e += kThreads) {
+        const int q = e / rows, i = lo + e - q * rows, kq = k0 - q;
+        if (kq >= 0) cp_async_zfill<sizeof(T)>(dst + q * mp + i, vglob + (size_t)kq * m + i, true);
+      }
+      cp_async_commit();
+    };
+    __syncthreads();
+    for (int e = tid; e < 2 * R * mp; e += kThreads)
+      if (e % mp >= m) sv[e] = mk<T>(0.0, 0.0);
     for (int wv = 0; wv < waves; ++wv) {
       const int j = gw + wv * nw;
       const bool live = j < nev;  // a warp without a vector still helps to stage
-      // each wave starts from zeroed staging rows (the previous wave's last rounds filled low rows)
-      __syncthreads();
-      for (int e = tid; e < BR * mp; e += kThreads) sv[e] = mk<T>(0.0, 0.0);
-      T z[kRegRows];
+      const double zs = live ? __ldcg(znorm + j) : 0.0;
+      T z[4 * kRowGroups];
 #pragma unroll
-      for (int t = 0; t < kRegRows; ++t) {
+      for (int t = 0; t < 4 * kRowGroups; ++t) {
         const int i = lane + 32 * t;
-        z[t] = mk<T>(live && i < m ? zt[(size_t)j * m + i] : 0.0, 0.0);
+        z[t] = mk<T>(live && i < m ? __ldcg(zt + (size_t)j * m + i) * zs : 0.0, 0.0);
       }
-      for (int b = 0; b < nblk; ++b) {
-        const int k0 = m - 2 - BR * b;
-        const int lo = k0 - BR + 2 > 0 ? k0 - BR + 2 : 0;  // first row any reflector of the round touches
-        __syncthreads();  // the previous round's readers are done
-        for (int q = 0; q < BR; ++q) {
-          const int kq = k0 - q;
-          if (kq < 0) break;
-          const T* src = vglob + (size_t)kq * m;
-          for (int i = lo + tid; i < m; i += kThreads) sv[q * mp + i] = src[i];
+      if (nchunk > 0) stage(0);
+      for (int c = 0; c < nchunk; ++c) {
+        if (c + 1 < nchunk) {
+          stage(c + 1);
+          cp_async_wait<1>();
+        } else {
+          cp_async_wait<0>();
         }
-        if (tid < 64) sgram[tid] = gram[(size_t)b * 64 + tid];
-        if (tid < BR) stau[tid] = k0 - tid >= 0 ? tauv[k0 - tid] : mk<T>(0.0, 0.0);
         __syncthreads();
-        if (!live) continue;
-        const int t0 = lo >> 5;
-        T sq[BR];
+        if (live) {
+          const T* vc = sv + (size_t)(c & 1) * R * mp + lane;
+          const int k0 = m - 2 - R * c, qn = min(R, k0 + 1);
+          for (int q = 0; q < qn; ++q) {
+            const T tau = tauv[k0 - q];
+            const int g0 = (k0 - q + 1) >> 7;
+            const T* vq = vc + q * mp;
+            T s0 = mk<T>(0.0, 0.0), s1 = s0;
 #pragma unroll
-        for (int q = 0; q < BR; ++q) sq[q] = mk<T>(0.0, 0.0);
+            for (int g = 0; g < kRowGroups; ++g) {
+              if (g < g0 || g >= ng) continue;
 #pragma unroll
-        for (int t = 0; t < kRegRows; ++t) {
-          if (t < t0 || t >= nt) continue;
-          const int i = lane + 32 * t;
+              for (int t = 4 * g; t < 4 * g + 4; t += 2) {
+                s0 = nmadd(s0, cj(vq[32 * t]), z[t]);
+                s1 = nmadd(s1, cj(vq[32 * t + 32]), z[t + 1]);
+              }
+            }
+            const T f = mul(tau, mul(warp_all(add(s0, s1)), -1.0));
 #pragma unroll
-          for (int q = 0; q < BR; ++q) sq[q] = add(sq[q], mul(cj(sv[q * mp + i]), z[t]));
+            for (int g = 0; g < kRowGroups; ++g) {
+              if (g < g0 || g >= ng) continue;
+#pragma unroll
+              for (int t = 4 * g; t < 4 * g + 4; ++t) z[t] = nmadd(z[t], vq[32 * t], f);
+            }
+          }
         }
-        for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-          for (int q = 0; q < BR; ++q) sq[q] = add(sq[q], shfl_xor(sq[q], o));
-        }
-        T f[BR];
-#pragma unroll
-        for (int q = 0; q < BR; ++q) {
-          T sv_q = sq[q];
-#pragma unroll
-          for (int p = 0; p < q; ++p) sv_q = sub(sv_q, mul(f[p], sgram[q * 8 + p]));
-          f[q] = mul(stau[q], sv_q);
-        }
-#pragma unroll
-        for (int t = 0; t < kRegRows; ++t) {
-          if (t < t0 || t >= nt) continue;
-          const int i = lane + 32 * t;
-          T zz = z[t];
-#pragma unroll
-          for (int q = 0; q < BR; ++q) zz = sub(zz, mul(sv[q * mp + i], f[q]));
-          z[t] = zz;
-        }
+        __syncthreads();  // the buffer may be filled again
       }
       if (live) {
         bool ok = true;
 #pragma unroll
-        for (int t = 0; t < kRegRows; ++t) {
+        for (int t = 0; t < 4 * kRowGroups; ++t) {
           const int i = lane + 32 * t;
           if (i < m) {
             Z[(size_t)j * ldz + i] = z[t];
@@ -813,23 +967,32 @@ __global__ void __launch_bounds__(kThreads, 1)
   cluster.sync();  // no CTA leaves while another may still read its shared memory
 }
 
+bool layout_fits(int m, int Ct, int tsz) {
+  return layout(m, Ct, tsz).total + 2 * kMaxM * sizeof(double) <= kSmemLimit;
+}
+
 // The smallest cluster whose CTAs hold the matrix in shared memory (0: none).
 int min_cluster(int m, int tsz) {
   for (int C = 1; C <= kMaxCluster; C *= 2)
-    if (layout(m, C, tsz).total + 2 * kMaxM * sizeof(double) <= kSmemLimit) return C;
+    if (layout_fits(m, C, tsz)) return C;
   return 0;
 }
 
-// The cluster size to use: measured on B200, a 16-CTA cluster is fastest
-// for every m > 64 (at m = 135 / 180 / 270 the solve takes 0.43 / 0.53 /
-// 0.74 of its time on the smallest cluster that fits, mostly through the
-// back-transform, bisection and inverse iteration that spread over the
-// CTAs) and within a few percent at m = 360; 8 CTAs below, and never more
-// CTAs than columns.
+// CTAs that hold the matrix during the tridiagonalisation of a cluster of C:
+// one as long as tridiag_one takes the size (real m = 128: 221 us against 335
+// on eight CTAs; complex m = 64 108 against 204 at m = 65), else all.
+int tridiag_ctas(int m, int C, int tsz) {
+  return m <= (tsz == (int)sizeof(double) ? kOneMaxReal : kOneMaxCplx) && layout_fits(m, 1, tsz) ? 1 : C;
+}
+
+// The cluster size to use, never more CTAs than columns: sixteen from m = 161
+// (real) or 181 (complex) on, where the phases after the reduction gain more
+// from the wider cluster than its barrier costs (real m = 150, lowest third:
+// 669 us on eight against 754 on sixteen; m = 180, all pairs: 985 and 773).
 int pick_cluster(int m, int tsz) {
   const int c0 = min_cluster(m, tsz);
   if (c0 == 0) return 0;
-  int want = m > 64 ? 16 : 8;
+  int want = m > (tsz == (int)sizeof(double) ? 160 : 180) ? 16 : 8;
   while (want > m) want /= 2;
   return std::max(c0, want);
 }
@@ -852,11 +1015,12 @@ template <typename T> Status set_attributes() {
   return kOk;
 }
 
-template <typename T> cudaLaunchConfig_t launch_config(int m, int C, cudaLaunchAttribute* attr, cudaStream_t s) {
+template <typename T>
+cudaLaunchConfig_t launch_config(int m, int C, int Ct, cudaLaunchAttribute* attr, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(C, 1, 1);
   cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = layout(m, C, (int)sizeof(T)).total;
+  cfg.dynamicSmemBytes = layout(m, Ct, (int)sizeof(T)).total;
   cfg.stream = s;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = C;
@@ -880,9 +1044,9 @@ template <typename T> bool cluster_fits(int m, int C) {
     if (set_attributes<T>() != kOk) return false;
     int mm = 1;  // the largest m a cluster of C CTAs can hold: the most shared memory
     for (int t = 1; t <= kMaxM; ++t)
-      if (layout(t, C, (int)sizeof(T)).total + 2 * kMaxM * sizeof(double) <= kSmemLimit) mm = t;
+      if (layout_fits(t, C, (int)sizeof(T))) mm = t;
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = launch_config<T>(mm, C, attr, nullptr);
+    cudaLaunchConfig_t cfg = launch_config<T>(mm, C, C, attr, nullptr);
     int n = 0;
     cudaError_t e = cudaOccupancyMaxActiveClusters(&n, k_eigh_cluster<T>, &cfg);
     c = (e == cudaSuccess && n > 0) ? 1 : 2;
@@ -912,8 +1076,13 @@ Status launch_eigh(const T* A, long lda, int m, int nev, double* w, T* Z, long l
   auto kern = k_eigh_cluster<T>;
   PW_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), s));
   cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = launch_config<T>(m, C, attr, s);
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, A, lda, m, nev, w, Z, ldz, work, status);
+  const int Ct = tridiag_ctas(m, C, (int)sizeof(T));
+  cudaLaunchConfig_t cfg = launch_config<T>(m, C, Ct, attr, s);
+  // Eigenvalues closer than gtol ||T|| are orthonormalised as one group: inverse iteration leaves the others
+  // orthogonal to eps / gtol.  Up to m = 64 the groups are few and short, and the wide tolerance keeps the vectors
+  // within 1e-12 of orthonormal; above it the serial Gram-Schmidt of a wide group would dominate.
+  const double gtol = m <= 64 ? 1e-3 : 1e-5;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, A, lda, m, nev, Ct, gtol, w, Z, ldz, work, status);
   count_launch();
   if (e != cudaSuccess) return fail(kCuda, std::string("eigh_cluster launch: ") + cudaGetErrorString(e));
   return kOk;
@@ -923,8 +1092,8 @@ Status launch_eigh(const T* A, long lda, int m, int nev, double* w, T* Z, long l
 }  // namespace
 
 size_t eigh_cluster_work_doubles(int m, int nev) {
-  // U rows, row operations and vectors (7 m nev), then the reflectors' Gram blocks (64 complex per block of 8)
-  return vglob_offset(m, std::max(nev, 1)) + (size_t)2 * m * m;
+  // U rows, row operations and vectors (7 m nev), the reflectors, the exchange buffers, the vectors' norms
+  return norm_offset(m, std::max(nev, 1)) + m;
 }
 
 bool eigh_cluster_supported(int m, bool complex_matrix) {

@@ -47,7 +47,6 @@ namespace {
 
 constexpr double kRyToEv = 13.605693122994;
 constexpr int kColBlocks = 64;      // partial sums per column reduction
-constexpr int kSmallSolveMax = 64;  // subspace size up to which the one-CTA solver runs
 // P columns whose component outside span(X, W) is below this fraction of
 // their norm are dropped (FP64 / reduced-precision search directions)
 constexpr double kPDropFp64 = 1e-5;
@@ -221,16 +220,6 @@ template <typename S> __global__ void k_gram_defect(const S* __restrict__ G, int
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   if ((threadIdx.x & 31) == 0 && v > 0.0)
     atomicMax(reinterpret_cast<unsigned long long*>(out), (unsigned long long)__double_as_longlong(v));
-}
-
-// real m x m <-> complex (zero imaginary part), for the one-CTA complex solver
-__global__ void k_real_to_complex(const double* __restrict__ a, double2* __restrict__ z, long n) {
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) z[t] = make_double2(a[t], 0.0);
-}
-__global__ void k_complex_to_real(const double2* __restrict__ z, double* __restrict__ a, long n) {
-  const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < n) a[t] = z[t].x;
 }
 
 template <typename T> Status walloc(T** p, size_t n) {
@@ -462,34 +451,9 @@ template <typename T> Status orthonormalize(Ctx& c, T* Y, int q) {
 
 // Lowest nev eigenpairs of the Hermitian subspace matrix Hs (m x m): values
 // into w.lam, vectors into *C (ld m).
-template <typename T> Status subspace_eig(Ctx& c, int m, int nev, T** C, bool allow_small = true) {
+template <typename T> Status subspace_eig(Ctx& c, int m, int nev, T** C) {
   Status r;
   T* Hs = as<T>(c.w.Hs);
-  if (allow_small && m <= kSmallSolveMax) {
-    // one-CTA Cholesky + Jacobi solver (complex; a real symmetric input stays real)
-    const double2* Hz = c.w.Hs;
-    if (std::is_same<T, double>::value) {
-      k_real_to_complex<<<blocks_for((long)m * m), 256, 0, c.s>>>(reinterpret_cast<const double*>(c.w.Hs), c.w.G,
-                                                                  (long)m * m); count_launch();
-      Hz = c.w.G;
-    }
-    k_set_identity<double2><<<blocks_for((long)m * m), 256, 0, c.s>>>(c.w.Id, m); count_launch();
-    if ((r = small_geneig_batched(Hz, c.w.Id, m, 0, m, nev, 1, c.w.lam, c.w.Cs, m, 0, c.w.status, c.s)) != kOk)
-      return r;
-    int st = 0;
-    PW_CUDA_TRY(cudaMemcpyAsync(&st, c.w.status, sizeof(int), cudaMemcpyDeviceToHost, c.s));
-    PW_CUDA_TRY(cudaStreamSynchronize(c.s));
-    if (st == 1) return fail(kNotConverged, "eigensolver: subspace solve failed");
-    if (std::is_same<T, double>::value) {
-      // real parts into Hs (the complex vectors of a real symmetric matrix are real)
-      k_complex_to_real<<<blocks_for((long)m * nev), 256, 0, c.s>>>(c.w.Cs, reinterpret_cast<double*>(c.w.Hs),
-                                                                    (long)m * nev); count_launch();
-      *C = Hs;
-    } else {
-      *C = as<T>(c.w.Cs);
-    }
-    return kOk;
-  }
   if (eigh_cluster_supported(m, !std::is_same<T, double>::value)) {
     // this project's cluster eigensolver: lowest nev pairs, vectors into Cs
     const size_t need = eigh_cluster_work_doubles(m, nev);
@@ -502,11 +466,11 @@ template <typename T> Status subspace_eig(Ctx& c, int m, int nev, T** C, bool al
     }
     T* Cv = as<T>(c.w.Cs);
     if ((r = eigh_cluster(Hs, m, m, nev, c.w.lam, Cv, m, c.w.eigh_work, c.w.status, c.s)) != kOk) return r;
+    *C = Cv;
     int st = 0;
     PW_CUDA_TRY(cudaMemcpyAsync(&st, c.w.status, sizeof(int), cudaMemcpyDeviceToHost, c.s));
     PW_CUDA_TRY(cudaStreamSynchronize(c.s));
     if (st != 0) return fail(kNotConverged, "eigensolver: subspace eigensolve produced non-finite values");
-    *C = Cv;
     return kOk;
   }
   // beyond the cluster solver's size (m > 544, or complex m beyond its shared memory)
@@ -742,7 +706,7 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
       count_launch();
       T* C = nullptr;
       pt.mark(5, s);
-      if ((r = subspace_eig<T>(c, ms, na, &C, false)) != kOk) return r;
+      if ((r = subspace_eig<T>(c, ms, na, &C)) != kOk) return r;
       pt.mark(6, s);
       // new active X, HX into the W, HW columns; new P, HP from the (W, P) rows
       if ((r = gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, (int)n, na, ms, Bx, n, C, ms, W, n)) != kOk) return r;
