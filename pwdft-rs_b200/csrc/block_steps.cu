@@ -1,0 +1,739 @@
+// The block steps of the eigensolver for narrow blocks (at most kMaxBlock
+// bands): orthonormalising the search directions W and P, the subspace matrix
+// and the update, one launch each.
+//
+// What bounds these steps at 2 to 16 atoms is neither arithmetic nor memory
+// but the number of dependent launches: a step of 27 bands over 1,045 plane
+// waves is ~50 library GEMMs, split-K sums, norms, gathers and copies of a few
+// microseconds each, plus host round trips for the Cholesky status.  Here
+// the rows of the block are spread over one thread-block cluster (up to 16
+// CTAs) and stay in shared memory from the first projection to the last
+// Cholesky-QR pass; every small matrix (A^H Y over all rows) is summed
+// from the CTAs' partials in rank order through L2, with one cluster barrier,
+// and factored by every CTA alike.  Products run on the FP64 tensor cores
+// (mma.sync m8n8k4), operands straight from L2 or shared memory.
+//
+// Against the library-call steps, with the same subspace eigensolver (B200):
+// restart iteration of 8 Si atoms at Gamma (real, 22 columns, 2,945 rows)
+// 27.7 -> 17.2 ms, of 2 atoms over 6 k-points (complex, 10 columns, 411 rows)
+// 21.0 -> 9.5 ms, whole LSDA run of 8 C atoms (27 columns, 1,045 rows, 40
+// blocks on 8 lanes) 405 -> 264 ms.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <mutex>
+#include <set>
+#include <string>
+
+#include "dense_ops.cuh"
+#include "handle.hpp"
+#include "linalg.hpp"
+#include "lobpcg.hpp"
+
+namespace pwgpu {
+
+namespace {
+
+namespace cg = cooperative_groups;
+using namespace dense;
+
+constexpr int kT = 512;
+constexpr int kW = kT / 32;
+constexpr int kMaxC = 16;
+constexpr size_t kSmemMax = 227 * 1024 - 4096;
+
+__device__ __forceinline__ double ldcg(const double* p) { return __ldcg(p); }
+__device__ __forceinline__ double2 ldcg(const double2* p) { return __ldcg(p); }
+template <typename T> __device__ __forceinline__ T zero() { return mk<T>(0.0, 0.0); }
+
+// c += a b on one 8 x 8 tile: lane holds a(lane / 4, lane % 4), b(lane % 4, lane / 4) and
+// c(lane / 4, 2 (lane % 4) + {0, 1}).
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+template <typename T> struct Tile;
+template <> struct Tile<double> {
+  double c[2];
+  __device__ __forceinline__ void clear() { c[0] = c[1] = 0.0; }
+  __device__ __forceinline__ void mma(double a, double b) { dmma(c, a, b); }
+  __device__ __forceinline__ double get(int h) const { return c[h]; }
+};
+template <> struct Tile<double2> {
+  double re[2], im[2];
+  __device__ __forceinline__ void clear() { re[0] = re[1] = im[0] = im[1] = 0.0; }
+  __device__ __forceinline__ void mma(double2 a, double2 b) {
+    dmma(re, a.x, b.x);
+    dmma(im, a.x, b.y);
+    dmma(re, -a.y, b.y);
+    dmma(im, a.y, b.x);
+  }
+  __device__ __forceinline__ double2 get(int h) const { return make_double2(re[h], im[h]); }
+};
+
+// Row stride of a shared-memory block of `rows` rows: 4 mod 16, so that the
+// operand reads of a tile (4 rows x 8 columns) touch every bank equally.
+__host__ __device__ constexpr int pad_ld(int rows) { return (rows + 15) / 16 * 16 + 4; }
+
+// Z (p x q, ld ldz in shared memory) = sum over the local rows of conj(A(i, a)) B(i, b).  Warps share the row
+// tiles of Z (8 x up to 32 entries each) and, when those are fewer than the warps, slices of the rows, added in
+// slice order.  la / lb return an entry, zero outside.
+template <typename T, typename LA, typename LB>
+__device__ void local_gram(int rows, int p, int q, LA la, LB lb, T* Z, int ldz) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int kr = lane & 3, kc = lane >> 2;
+  const int tp = (p + 7) >> 3, tg = (q + 31) >> 5;
+  const int items = tp * tg;
+  const int S = items >= kW ? 1 : kW / items;  // row slices
+  const int per = ((rows + S - 1) / S + 3) & ~3;
+  for (int base = 0; base < items * S; base += kW) {
+    const int it = base + warp;
+    const bool live = it < items * S;
+    const int sl = live ? it / items : 0, tile = live ? it % items : 0;
+    const int p0 = (tile % tp) * 8, q0 = (tile / tp) * 32;
+    Tile<T> acc[4];
+#pragma unroll
+    for (int t = 0; t < 4; ++t) acc[t].clear();
+    if (live) {
+      const int i1 = min(rows, (sl + 1) * per);
+#pragma unroll 4
+      for (int i = sl * per; i < i1; i += 4) {
+        const bool in = i + kr < i1;
+        const T a = in ? cj(la(i + kr, p0 + kc)) : zero<T>();
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          if (q0 + 8 * t >= q) break;
+          acc[t].mma(a, in ? lb(i + kr, q0 + 8 * t + kc) : zero<T>());
+        }
+      }
+    }
+    for (int s = 0; s < S; ++s) {
+      if (live && sl == s) {
+        const int r = p0 + kc;
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int c = q0 + 8 * t + 2 * kr + h;
+            if (r < p && c < q) Z[r + c * ldz] = s == 0 ? acc[t].get(h) : add(Z[r + c * ldz], acc[t].get(h));
+          }
+      }
+      __syncthreads();
+    }
+  }
+}
+
+// Entry e of the sum over the CTAs' partials (C x n in xch), in rank order.
+template <typename T> __device__ __forceinline__ T rank_sum(const T* xch, int C, size_t n, size_t e) {
+  T v[kMaxC];
+#pragma unroll
+  for (int r = 0; r < kMaxC; ++r) v[r] = r < C ? ldcg(xch + r * n + e) : zero<T>();
+  T s = v[0];
+#pragma unroll
+  for (int r = 1; r < kMaxC; ++r) s = add(s, v[r]);
+  return s;
+}
+
+// Sum of the CTAs' Z (p x q) into every CTA's Z, in rank order.  xch: this
+// call's buffer in global memory ((C + 1) p q entries); consecutive calls
+// alternate between two.  Every CTA adds up all entries (one barrier), or,
+// from kTwoPhase entries on, its share of them, and reads the others' sums
+// after a second barrier (C times fewer reads).
+constexpr int kTwoPhase = 1024;
+template <typename T>
+__device__ void cluster_sum(cg::cluster_group& cl, T* Z, int ldz, int p, int q, T* xch) {
+  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  if (C == 1) return;
+  const int n = p * q;
+  for (int e = threadIdx.x; e < n; e += kT) xch[(size_t)rank * n + e] = Z[e % p + (e / p) * ldz];
+  cl.sync();
+  if (n < kTwoPhase) {
+    for (int e = threadIdx.x; e < n; e += kT) Z[e % p + (e / p) * ldz] = rank_sum<T>(xch, C, n, e);
+  } else {
+    T* tot = xch + (size_t)C * n;
+    for (int e = rank * kT + threadIdx.x; e < n; e += C * kT) tot[e] = rank_sum<T>(xch, C, n, e);
+    cl.sync();
+    for (int e = threadIdx.x; e < n; e += kT) Z[e % p + (e / p) * ldz] = ldcg(tot + e);
+  }
+  __syncthreads();
+}
+
+// out(i, c) = base(i, c) - sum_k A(i, k) Z(k, c), c < q, over 8-row strips of the local rows (NQ tiles of 8
+// columns in registers).  A strip is read whole before it is written, so out may alias A.
+template <int NQ, bool SUB, typename T, typename LA, typename LC, typename ST>
+__device__ void local_update(int rows, int kdim, int q, LA la, const T* Z, int ldz, LC lc, ST st) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int kr = lane & 3, kc = lane >> 2;
+  for (int i0 = warp * 8; i0 < rows; i0 += kW * 8) {
+    Tile<T> acc[NQ];
+#pragma unroll
+    for (int t = 0; t < NQ; ++t) acc[t].clear();
+    const bool rin = i0 + kc < rows;
+#pragma unroll 4
+    for (int k = 0; k < kdim; k += 4) {
+      const bool kin = k + kr < kdim;
+      const T a = rin && kin ? la(i0 + kc, k + kr) : zero<T>();
+#pragma unroll
+      for (int t = 0; t < NQ; ++t) {
+        if (8 * t >= q) break;
+        const int c = 8 * t + kc;
+        acc[t].mma(a, kin && c < q ? Z[(k + kr) + c * ldz] : zero<T>());
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int t = 0; t < NQ; ++t)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = 8 * t + 2 * kr + h;
+        if (rin && c < q) st(i0 + kc, c, SUB ? sub(lc(i0 + kc, c), acc[t].get(h)) : acc[t].get(h));
+      }
+    __syncwarp();
+  }
+}
+
+// Upper Cholesky factor of the q x q Hermitian G (upper triangle used) in place; false when a pivot is not
+// positive.  *rmin: smallest diagonal entry.  All threads; ends at a block barrier.
+template <typename T> __device__ bool block_cholesky(T* G, int ldg, int q, double* rmin) {
+  __syncthreads();
+  double mn = 1e300;
+  for (int c = 0; c < q; ++c) {
+    const double d = re(G[c + c * ldg]);
+    if (!(d > 0.0)) {  // the same value in every thread
+      __syncthreads();
+      return false;
+    }
+    const double r = sqrt(d), ir = 1.0 / r;
+    mn = fmin(mn, r);
+    __syncthreads();
+    for (int j = c + threadIdx.x; j < q; j += kT) G[c + j * ldg] = j == c ? mk<T>(r, 0.0) : mul(G[c + j * ldg], ir);
+    __syncthreads();
+    const int rem = q - c - 1;
+    for (int e = threadIdx.x; e < rem * rem; e += kT) {
+      const int i = c + 1 + e % rem, j = c + 1 + e / rem;
+      if (i <= j) G[i + j * ldg] = sub(G[i + j * ldg], mul(cj(G[c + i * ldg]), G[c + j * ldg]));
+    }
+    __syncthreads();
+  }
+  *rmin = mn;
+  return true;
+}
+
+// Ri = R^-1 (q x q, zero below the diagonal), one warp per column: lane l keeps entries l and l + 32.
+template <typename T> __device__ void block_inverse(const T* R, int ldr, int q, T* Ri, int ldi) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int c = warp; c < q; c += kW) {
+    T z0 = mk<T>(lane == c ? 1.0 : 0.0, 0.0), z1 = mk<T>(lane + 32 == c ? 1.0 : 0.0, 0.0);
+    for (int i = c; i >= 0; --i) {
+      const double id = 1.0 / re(R[i + i * ldr]);
+      const T zi = mul(i < 32 ? shfl(z0, i) : shfl(z1, i - 32), id);
+      if (lane < i) z0 = sub(z0, mul(R[lane + i * ldr], zi));
+      if (lane + 32 < i) z1 = sub(z1, mul(R[lane + 32 + i * ldr], zi));
+      if (lane == i) z0 = zi;
+      if (lane + 32 == i) z1 = zi;
+    }
+    if (lane < q) Ri[lane + c * ldi] = lane <= c ? z0 : zero<T>();
+    if (lane + 32 < q) Ri[lane + 32 + c * ldi] = lane + 32 <= c ? z1 : zero<T>();
+  }
+  __syncthreads();
+}
+
+// max |G - I| of the q x q Gram matrix (the same value in every thread)
+template <typename T> __device__ double block_defect(const T* G, int ldg, int q, double* red) {
+  double v = 0.0;
+  for (int e = threadIdx.x; e < q * q; e += kT) {
+    const int r = e % q, c = e / q;
+    const T g = G[r + c * ldg];
+    v = fmax(v, hypot(r == c ? re(g) - 1.0 : re(g), im(g)));
+  }
+  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = red[0];
+  for (int w = 1; w < kW; ++w) v = fmax(v, red[w]);
+  __syncthreads();
+  return v;
+}
+
+constexpr double kSkipTol = 1e-12;  // a Cholesky-QR pass is skipped when its block is orthonormal to this
+
+// W = orthonormal basis of the part of Tb(:, idx) outside span(X): two projections, columns scaled, two
+// Cholesky-QR passes (a pass that finds the block orthonormal stops; a first pass that breaks down is repeated
+// with a diagonal shift).  idx NULL: the columns in order.  status[0] = 1 when the block is rank deficient.
+template <typename T, int NQ>
+__global__ void __launch_bounds__(kT, 1)
+    k_block_w(const T* __restrict__ X, int nd, const T* Tb, const int* __restrict__ idx, int na, T* W, long n,
+              int rpc, int ldy, int ldz, T* __restrict__ xch, long xch_len, int* __restrict__ status) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ double red[kW];
+  __shared__ double scol[kMaxBlock];
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank();
+  T* Y = reinterpret_cast<T*>(smem);       // rpc x na
+  T* Z = Y + (size_t)ldy * na;             // max(nd, na) x na
+  T* Ri = Z + (size_t)ldz * na;            // na x na
+  const long r0 = (long)rank * rpc;
+  const int rows = (int)max(0L, min((long)rpc, n - r0));
+  for (int e = threadIdx.x; e < rows * na; e += kT) {
+    const int i = e % rows, c = e / rows;
+    Y[i + c * ldy] = Tb[r0 + i + (long)(idx ? idx[c] : c) * n];
+  }
+  __syncthreads();
+  int par = 0;
+  auto ly = [&](int i, int c) { return c < na ? Y[i + c * ldy] : zero<T>(); };
+  for (int pass = 0; pass < 2 && nd > 0; ++pass) {
+    auto lx = [&](int i, int c) { return c < nd ? X[r0 + i + (long)c * n] : zero<T>(); };
+    local_gram<T>(rows, nd, na, lx, ly, Z, ldz);
+    cluster_sum<T>(cl, Z, ldz, nd, na, xch + par * xch_len);
+    par ^= 1;
+    local_update<NQ, true, T>(rows, nd, na, lx, Z, ldz, ly, [&](int i, int c, T v) { Y[i + c * ldy] = v; });
+    __syncthreads();
+  }
+  bool ok = true;
+  for (int pass = 0; pass < 2; ++pass) {
+    local_gram<T>(rows, na, na, ly, ly, Z, ldz);
+    cluster_sum<T>(cl, Z, ldz, na, na, xch + par * xch_len);
+    par ^= 1;
+    if (pass == 0) {
+      // the Gram matrix of the unit columns
+      if (threadIdx.x < na) {
+        const double d = re(Z[threadIdx.x + threadIdx.x * ldz]);
+        scol[threadIdx.x] = d > 0.0 ? 1.0 / sqrt(d) : 0.0;
+      }
+      __syncthreads();
+      for (int e = threadIdx.x; e < na * na; e += kT) {
+        const int r = e % na, c = e / na;
+        Z[r + c * ldz] = mul(Z[r + c * ldz], scol[r] * scol[c]);
+      }
+    } else if (threadIdx.x < na) {
+      scol[threadIdx.x] = 1.0;
+    }
+    __syncthreads();
+    if (block_defect<T>(Z, ldz, na, red) <= kSkipTol) {
+      if (pass == 0) {
+        for (int e = threadIdx.x; e < rows * na; e += kT) {
+          const int i = e % rows, c = e / rows;
+          Y[i + c * ldy] = mul(Y[i + c * ldy], scol[c]);
+        }
+        __syncthreads();
+      }
+      break;
+    }
+    double rmin;
+    // keep a copy in Ri's place for the shifted retry
+    for (int e = threadIdx.x; e < na * na; e += kT) Ri[e % na + (e / na) * ldz] = Z[e % na + (e / na) * ldz];
+    __syncthreads();
+    ok = block_cholesky<T>(Z, ldz, na, &rmin);
+    if (!ok && pass == 0) {
+      for (int e = threadIdx.x; e < na * na; e += kT) {
+        const int r = e % na, c = e / na;
+        T g = Ri[r + c * ldz];
+        if (r == c) g = add(g, mk<T>(1e-10 * na, 0.0));
+        Z[r + c * ldz] = g;
+      }
+      __syncthreads();
+      ok = block_cholesky<T>(Z, ldz, na, &rmin);
+    }
+    if (!ok) break;
+    block_inverse<T>(Z, ldz, na, Ri, ldz);
+    for (int e = threadIdx.x; e < na * na; e += kT) {
+      const int r = e % na, c = e / na;
+      Ri[r + c * ldz] = mul(Ri[r + c * ldz], scol[r]);
+    }
+    __syncthreads();
+    local_update<NQ, false, T>(rows, na, na, ly, Ri, ldz, ly, [&](int i, int c, T v) { Y[i + c * ldy] = v; });
+    __syncthreads();
+  }
+  for (int e = threadIdx.x; e < rows * na; e += kT) {
+    const int i = e % rows, c = e / rows;
+    W[r0 + i + (long)c * n] = Y[i + c * ldy];
+  }
+  if (rank == 0 && threadIdx.x == 0) status[0] = ok ? 0 : 1;
+}
+
+// P, HP = the previous directions Pn(:, idx), HPn(:, idx) outside span(X, W), orthonormal: projections against X and W
+// (H with them), columns that keep less than p_drop of their norm dropped, two Cholesky-QR passes.  status[1] =
+// columns of P (0 when the block is nearly dependent).
+template <typename T, int NQ>
+__global__ void __launch_bounds__(kT, 1)
+    k_block_p(const T* __restrict__ X, const T* __restrict__ HX, int nd, const T* __restrict__ W,
+              const T* __restrict__ HW, int na, const T* __restrict__ Pn, const T* __restrict__ HPn,
+              const int* __restrict__ idx, int np, T* __restrict__ P, T* __restrict__ HP, long n, int rpc, int ldy,
+              int ldz, double p_drop, T* __restrict__ xch, long xch_len, int* __restrict__ status) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ double red[kW];
+  __shared__ double scol[kMaxBlock], nu0[kMaxBlock];
+  __shared__ int keep[kMaxBlock];
+  __shared__ int nkeep_s;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank();
+  T* Y = reinterpret_cast<T*>(smem);
+  T* Z = Y + (size_t)ldy * np;
+  T* Ri = Z + (size_t)ldz * np;
+  const long r0 = (long)rank * rpc;
+  const int rows = (int)max(0L, min((long)rpc, n - r0));
+  for (int e = threadIdx.x; e < rows * np; e += kT) {
+    const int i = e % rows, c = e / rows;
+    Y[i + c * ldy] = Pn[r0 + i + (long)idx[c] * n];
+  }
+  __syncthreads();
+  // squared column norms of this CTA's rows, summed with the first projection (row nd of Z)
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int c = warp; c < np; c += kW) {
+    double s = 0.0;
+    for (int i = lane; i < rows; i += 32) s += abs2(Y[i + c * ldy]);
+    s = warp_sum(s);
+    if (lane == 0) nu0[c] = s;
+  }
+  __syncthreads();
+  int par = 0;
+  auto ly = [&](int i, int c) { return c < np ? Y[i + c * ldy] : zero<T>(); };
+  auto sy = [&](int i, int c, T v) { Y[i + c * ldy] = v; };
+  {
+    auto lx = [&](int i, int c) { return c < nd ? X[r0 + i + (long)c * n] : zero<T>(); };
+    local_gram<T>(rows, nd, np, lx, ly, Z, ldz);
+    if (threadIdx.x < np) Z[nd + threadIdx.x * ldz] = mk<T>(nu0[threadIdx.x], 0.0);
+    __syncthreads();
+    cluster_sum<T>(cl, Z, ldz, nd + 1, np, xch + par * xch_len);
+    par ^= 1;
+    if (threadIdx.x < np) nu0[threadIdx.x] = re(Z[nd + threadIdx.x * ldz]);
+    local_update<NQ, true, T>(rows, nd, np, lx, Z, ldz, ly, sy);
+    local_update<NQ, true, T>(
+        rows, nd, np, [&](int i, int c) { return HX[r0 + i + (long)c * n]; }, Z, ldz,
+        [&](int i, int c) { return HPn[r0 + i + (long)idx[c] * n]; },
+        [&](int i, int c, T v) { HP[r0 + i + (long)c * n] = v; });
+    __syncthreads();
+  }
+  auto lhp = [&](int i, int c) { return HP[r0 + i + (long)c * n]; };
+  auto shp = [&](int i, int c, T v) { HP[r0 + i + (long)c * n] = v; };
+  {
+    auto lw = [&](int i, int c) { return c < na ? W[r0 + i + (long)c * n] : zero<T>(); };
+    local_gram<T>(rows, na, np, lw, ly, Z, ldz);
+    cluster_sum<T>(cl, Z, ldz, na, np, xch + par * xch_len);
+    par ^= 1;
+    local_update<NQ, true, T>(rows, na, np, lw, Z, ldz, ly, sy);
+    local_update<NQ, true, T>(
+        rows, na, np, [&](int i, int c) { return HW[r0 + i + (long)c * n]; }, Z, ldz, lhp, shp);
+    __syncthreads();
+  }
+  int nk = np;
+  bool ok = true;
+  for (int pass = 0; pass < 2; ++pass) {
+    auto lyk = [&](int i, int c) { return c < nk ? Y[i + c * ldy] : zero<T>(); };
+    local_gram<T>(rows, nk, nk, lyk, lyk, Z, ldz);
+    cluster_sum<T>(cl, Z, ldz, nk, nk, xch + par * xch_len);
+    par ^= 1;
+    if (pass == 0) {
+      if (threadIdx.x == 0) {
+        int k = 0;
+        for (int c = 0; c < np; ++c) {
+          const double d = re(Z[c + c * ldz]);
+          if (d > p_drop * p_drop * nu0[c] && d > 0.0) {
+            keep[k] = c;
+            scol[k++] = 1.0 / sqrt(d);
+          }
+        }
+        nkeep_s = k;
+      }
+      __syncthreads();
+      nk = nkeep_s;
+      if (nk == 0) break;
+      // the scaled Gram matrix of the kept columns, through Ri
+      for (int e = threadIdx.x; e < nk * nk; e += kT) {
+        const int r = e % nk, c = e / nk;
+        Ri[r + c * ldz] = mul(Z[keep[r] + keep[c] * ldz], scol[r] * scol[c]);
+      }
+      __syncthreads();
+      for (int e = threadIdx.x; e < nk * nk; e += kT) Z[e % nk + (e / nk) * ldz] = Ri[e % nk + (e / nk) * ldz];
+      __syncthreads();
+    } else {
+      if (threadIdx.x < nk) {
+        keep[threadIdx.x] = threadIdx.x;
+        scol[threadIdx.x] = 1.0;
+      }
+      __syncthreads();
+      if (block_defect<T>(Z, ldz, nk, red) <= kSkipTol) break;
+    }
+    double rmin = 0.0;
+    ok = block_cholesky<T>(Z, ldz, nk, &rmin);
+    if (!ok || (pass == 0 && rmin < p_drop)) {
+      nk = 0;
+      break;
+    }
+    block_inverse<T>(Z, ldz, nk, Ri, ldz);
+    for (int e = threadIdx.x; e < nk * nk; e += kT) {
+      const int r = e % nk, c = e / nk;
+      Ri[r + c * ldz] = mul(Ri[r + c * ldz], scol[r]);
+    }
+    __syncthreads();
+    local_update<NQ, false, T>(
+        rows, nk, nk, [&](int i, int c) { return Y[i + keep[c] * ldy]; }, Ri, ldz, ly, sy);
+    local_update<NQ, false, T>(
+        rows, nk, nk, [&](int i, int c) { return HP[r0 + i + (long)keep[c] * n]; }, Ri, ldz, lhp, shp);
+    __syncthreads();
+  }
+  for (int e = threadIdx.x; e < rows * nk; e += kT) {
+    const int i = e % rows, c = e / rows;
+    P[r0 + i + (long)c * n] = Y[i + c * ldy];
+  }
+  if (rank == 0 && threadIdx.x == 0) status[1] = nk;
+}
+
+// Subspace matrix Hs (m x m, m = nx + q) over [X(:, cols) | B]: diag(lam) (or (XX + XX^H) / 2 when XX is given), Z = B^H
+// HX(:, cols), (G + G^H) / 2 with G = B^H HB.  cols NULL: the columns in order.
+template <typename T>
+__global__ void __launch_bounds__(kT, 1)
+    k_block_rr(const T* __restrict__ B, const T* __restrict__ HB, int q, const T* __restrict__ HX,
+               const int* __restrict__ cols, int nx, const double* __restrict__ lam, const T* __restrict__ XX, long n,
+               int rpc, int ldz, T* __restrict__ xch, T* __restrict__ Hs) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  T* Z = reinterpret_cast<T*>(smem);  // q x (nx + q)
+  cg::cluster_group cl = cg::this_cluster();
+  const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
+  const long r0 = (long)rank * rpc;
+  const int rows = (int)max(0L, min((long)rpc, n - r0));
+  const int m = nx + q, nz = q * m;
+  auto lb = [&](int i, int c) { return c < q ? B[r0 + i + (long)c * n] : zero<T>(); };
+  local_gram<T>(
+      rows, q, m, lb,
+      [&](int i, int c) {
+        if (c >= m) return zero<T>();
+        return c < nx ? HX[r0 + i + (long)(cols ? cols[c] : c) * n] : HB[r0 + i + (long)(c - nx) * n];
+      },
+      Z, ldz);
+  for (int e = threadIdx.x; e < nz; e += kT) xch[(size_t)rank * nz + e] = Z[e % q + (e / q) * ldz];
+  cl.sync();
+  // entry (r, c) of B^H [HX | HB], summed over the CTAs
+  auto entry = [&](int r, int c) { return rank_sum<T>(xch, C, nz, r + (size_t)c * q); };
+  for (int e = rank * kT + threadIdx.x; e < m * m; e += C * kT) {
+    const int r = e % m, c = e / m;
+    T v;
+    if (r < nx && c < nx) {
+      if (XX) {
+        const T a = XX[r + (long)c * nx], b = cj(XX[c + (long)r * nx]);
+        v = mul(add(a, b), mk<T>(0.5, 0.0));
+      } else {
+        v = mk<T>(r == c ? lam[r] : 0.0, 0.0);
+      }
+    } else if (c < nx) {
+      v = entry(r - nx, c);
+    } else if (r < nx) {
+      v = cj(entry(c - nx, r));
+    } else {
+      v = mul(add(entry(r - nx, c), cj(entry(c - nx, r))), mk<T>(0.5, 0.0));
+    }
+    Hs[e] = v;
+  }
+}
+
+// Update of V = X (blockIdx.y 0) and of HV (1) over 8-row strips, one warp each: T = B C_b (C's rows nx .. nx + q - 1),
+// Pn(:, t) = T(:, pcols[t]), X(:, cols) <- X(:, cols) C_x + T in place (a strip is read whole before it is written).
+constexpr int kUpdThreads = 128;
+template <typename T, int NQ>
+__global__ void __launch_bounds__(kUpdThreads)
+    k_block_update(T* __restrict__ X, const T* __restrict__ B, T* __restrict__ Pn, T* __restrict__ HX,
+                   const T* __restrict__ HB, T* __restrict__ HPn, const T* __restrict__ Cm, int m, int nx, int q,
+                   const int* __restrict__ cols, const int* __restrict__ pcols, int np, long n) {
+  T* x = blockIdx.y ? HX : X;
+  const T* b = blockIdx.y ? HB : B;
+  T* pn = blockIdx.y ? HPn : Pn;
+  __shared__ int pos[kMaxBlock];  // column of Pn that takes column j of T, or -1
+  __shared__ int xc[kMaxBlock];   // column of X behind subspace column j
+  for (int j = threadIdx.x; j < nx; j += kUpdThreads) {
+    pos[j] = -1;
+    xc[j] = cols ? cols[j] : j;
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < np; t += kUpdThreads) pos[pcols ? pcols[t] : t] = t;
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int kr = lane & 3, kc = lane >> 2;
+  const long i = ((long)blockIdx.x * (kUpdThreads / 32) + warp) * 8 + kc;
+  const bool in = i < n;
+  Tile<T> acc[NQ];
+#pragma unroll
+  for (int t = 0; t < NQ; ++t) acc[t].clear();
+  auto run = [&](int k0, int kdim, auto la) {
+#pragma unroll 4
+    for (int k = 0; k < kdim; k += 4) {
+      const bool kin = k + kr < kdim;
+      const T a = in && kin ? la(k + kr) : zero<T>();
+#pragma unroll
+      for (int t = 0; t < NQ; ++t) {
+        if (8 * t >= nx) break;
+        const int c = 8 * t + kc;
+        acc[t].mma(a, kin && c < nx ? Cm[k0 + k + kr + (long)c * m] : zero<T>());
+      }
+    }
+  };
+  run(nx, q, [&](int k) { return b[i + (long)k * n]; });
+#pragma unroll
+  for (int t = 0; t < NQ; ++t)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int c = 8 * t + 2 * kr + h;
+      if (in && c < nx && pos[c] >= 0) pn[i + (long)pos[c] * n] = acc[t].get(h);
+    }
+  run(0, nx, [&](int k) { return x[i + (long)xc[k] * n]; });
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < NQ; ++t)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int c = 8 * t + 2 * kr + h;
+      if (in && c < nx) x[i + (long)xc[c] * n] = acc[t].get(h);
+    }
+}
+
+// Rows per CTA and cluster size for n rows: at least 32 rows a CTA, rows in multiples of 8.
+void split_rows(long n, int& C, int& rpc) {
+  C = kMaxC;
+  while (C > 1 && n < 32L * C) C /= 2;
+  rpc = (int)(((n + C - 1) / C + 7) / 8 * 8);
+}
+
+template <typename T> size_t step_smem(int rpc, int cols, int zrows) {
+  return ((size_t)pad_ld(rpc) + 2 * (size_t)pad_ld(zrows)) * cols * sizeof(T);
+}
+
+template <typename K> Status opt_in(K kern, bool cluster) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
+  if (e == cudaSuccess && cluster) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e != cudaSuccess) return fail(kCuda, std::string("block step attributes: ") + cudaGetErrorString(e));
+  return kOk;
+}
+
+// Per-device attributes, and whether 16-CTA clusters of these kernels can be resident.
+template <typename T> Status configure(bool* fits) {
+  static std::mutex mu;
+  static std::set<int> good, bad;
+  int dev = 0;
+  PW_CUDA_TRY(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(mu);
+  if (!good.count(dev) && !bad.count(dev)) {
+    Status r;
+    if ((r = opt_in(k_block_w<T, 4>, true)) != kOk || (r = opt_in(k_block_w<T, 8>, true)) != kOk ||
+        (r = opt_in(k_block_p<T, 4>, true)) != kOk || (r = opt_in(k_block_p<T, 8>, true)) != kOk ||
+        (r = opt_in(k_block_rr<T>, true)) != kOk)
+      return r;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    cfg.gridDim = dim3(kMaxC, 1, 1);
+    cfg.blockDim = dim3(kT, 1, 1);
+    cfg.dynamicSmemBytes = kSmemMax;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kMaxC;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    const bool ok = cudaOccupancyMaxActiveClusters(&n, k_block_p<T, 8>, &cfg) == cudaSuccess && n > 0;
+    if (!ok) cudaGetLastError();
+    (ok ? good : bad).insert(dev);
+  }
+  *fits = good.count(dev) > 0;
+  return kOk;
+}
+
+template <typename... P, typename... A>
+Status launch(void (*kern)(P...), int C, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(C, 1, 1);
+  cfg.blockDim = dim3(kT, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+  count_launch();
+  if (e != cudaSuccess) return fail(kCuda, std::string("block step launch: ") + cudaGetErrorString(e));
+  return kOk;
+}
+
+}  // namespace
+
+template <typename T> bool block_steps_fit(long n, int nd) {
+  if (nd < 1 || nd > kMaxBlock) return false;
+  int C, rpc;
+  split_rows(n, C, rpc);
+  // P's block: nd columns, small matrices of nd + 1 rows; the subspace matrix: 2 nd rows, 3 nd columns
+  if (step_smem<T>(rpc, nd, nd + 1) > kSmemMax) return false;
+  if ((size_t)pad_ld(2 * nd) * 3 * nd * sizeof(T) > kSmemMax) return false;
+  bool fits = false;
+  return configure<T>(&fits) == kOk && fits;
+}
+
+size_t block_steps_xch(int nd) {
+  // two buffers of (nd + 1) x nd, or one of 2 nd x 3 nd, per CTA
+  return (size_t)(kMaxC + 1) * std::max<size_t>(2 * (size_t)(nd + 1) * nd, (size_t)6 * nd * nd);
+}
+
+template <typename T>
+Status block_w(const T* X, int nd, const T* Tb, const int* idx, int na, T* W, long n, T* xch, int* status,
+               cudaStream_t s) {
+  int C, rpc;
+  split_rows(n, C, rpc);
+  const int zr = std::max(nd, na), ldy = pad_ld(rpc), ldz = pad_ld(zr);
+  const size_t sm = step_smem<T>(rpc, na, zr);
+  const long xl = (long)(kMaxC + 1) * std::max(nd, na) * na;
+  if (na <= 32) return launch(k_block_w<T, 4>, C, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, xch, xl, status);
+  return launch(k_block_w<T, 8>, C, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, xch, xl, status);
+}
+
+template <typename T>
+Status block_p(const T* X, const T* HX, int nd, const T* W, const T* HW, int na, const T* Pn, const T* HPn,
+               const int* idx, int np, T* P, T* HP, long n, double p_drop, T* xch, int* status, cudaStream_t s) {
+  int C, rpc;
+  split_rows(n, C, rpc);
+  const int zr = std::max(nd + 1, std::max(na, np)), ldy = pad_ld(rpc), ldz = pad_ld(zr);
+  const size_t sm = step_smem<T>(rpc, np, zr);
+  const long xl = (long)(kMaxC + 1) * (nd + 1) * np;
+  if (np <= 32)
+    return launch(k_block_p<T, 4>, C, sm, s, X, HX, nd, W, HW, na, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, p_drop,
+                  xch, xl, status);
+  return launch(k_block_p<T, 8>, C, sm, s, X, HX, nd, W, HW, na, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, p_drop,
+                xch, xl, status);
+}
+
+template <typename T>
+Status block_rr(const T* B, const T* HB, int q, const T* HX, const int* cols, int nx, const double* lam, const T* XX,
+                long n, T* xch, T* Hs, cudaStream_t s) {
+  int C, rpc;
+  split_rows(n, C, rpc);
+  const int ldz = pad_ld(q);
+  return launch(k_block_rr<T>, C, (size_t)ldz * (nx + q) * sizeof(T), s, B, HB, q, HX, cols, nx, lam, XX, n, rpc, ldz,
+                xch, Hs);
+}
+
+template <typename T>
+Status block_update(T* X, const T* B, T* Pn, T* HX, const T* HB, T* HPn, const T* Cm, int m, int nx, int q,
+                    const int* cols, const int* pcols, int np, long n, cudaStream_t s) {
+  const dim3 grid((unsigned)((n + 8 * (kUpdThreads / 32) - 1) / (8 * (kUpdThreads / 32))), 2);
+  if (nx <= 32)
+    k_block_update<T, 4><<<grid, kUpdThreads, 0, s>>>(X, B, Pn, HX, HB, HPn, Cm, m, nx, q, cols, pcols, np, n);
+  else
+    k_block_update<T, 8><<<grid, kUpdThreads, 0, s>>>(X, B, Pn, HX, HB, HPn, Cm, m, nx, q, cols, pcols, np, n);
+  count_launch();
+  PW_CUDA_TRY(cudaGetLastError());
+  return kOk;
+}
+
+#define PW_BLOCK(T)                                                                                                  \
+  template bool block_steps_fit<T>(long, int);                                                                      \
+  template Status block_w<T>(const T*, int, const T*, const int*, int, T*, long, T*, int*, cudaStream_t);            \
+  template Status block_p<T>(const T*, const T*, int, const T*, const T*, int, const T*, const T*, const int*, int, \
+                             T*, T*, long, double, T*, int*, cudaStream_t);                                          \
+  template Status block_rr<T>(const T*, const T*, int, const T*, const int*, int, const double*, const T*, long,     \
+                              T*, T*, cudaStream_t);                                                                 \
+  template Status block_update<T>(T*, const T*, T*, T*, const T*, T*, const T*, int, int, int, const int*,           \
+                                  const int*, int, long, cudaStream_t);
+PW_BLOCK(double)
+PW_BLOCK(double2)
+#undef PW_BLOCK
+
+}  // namespace pwgpu

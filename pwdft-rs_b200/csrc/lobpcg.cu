@@ -451,7 +451,8 @@ template <typename T> Status orthonormalize(Ctx& c, T* Y, int q) {
 
 // Lowest nev eigenpairs of the Hermitian subspace matrix Hs (m x m): values
 // into w.lam, vectors into *C (ld m).
-template <typename T> Status subspace_eig(Ctx& c, int m, int nev, T** C) {
+// defer: the caller reads w.status itself (only where the cluster solver runs).
+template <typename T> Status subspace_eig(Ctx& c, int m, int nev, T** C, bool defer = false) {
   Status r;
   T* Hs = as<T>(c.w.Hs);
   if (eigh_cluster_supported(m, !std::is_same<T, double>::value)) {
@@ -467,6 +468,7 @@ template <typename T> Status subspace_eig(Ctx& c, int m, int nev, T** C) {
     T* Cv = as<T>(c.w.Cs);
     if ((r = eigh_cluster(Hs, m, m, nev, c.w.lam, Cv, m, c.w.eigh_work, c.w.status, c.s)) != kOk) return r;
     *C = Cv;
+    if (defer) return kOk;
     int st = 0;
     PW_CUDA_TRY(cudaMemcpyAsync(&st, c.w.status, sizeof(int), cudaMemcpyDeviceToHost, c.s));
     PW_CUDA_TRY(cudaStreamSynchronize(c.s));
@@ -570,7 +572,15 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
     PW_CUDA_TRY(cudaStreamSynchronize(s));
     k.init = true;
   }
-  if ((r = orthonormalize(c, X, nd)) != kOk) return r;
+  // narrow blocks take the fused block steps (block_steps.cu): one launch each for W, P, the subspace
+  // matrix and the update
+  const bool steps = block_steps_fit<T>(n, nd);
+  T* xch = as<T>(w.xch);
+  int* bst = w.status + 1;
+  PW_CUDA_TRY(cudaMemsetAsync(w.status, 0, 3 * sizeof(int), s));
+  if (steps) r = block_w<T>(nullptr, 0, X, nullptr, nd, X, n, xch, bst, s);
+  else r = orthonormalize(c, X, nd);
+  if (r != kOk) return r;
   // HX in FP64: the residuals below refer to the full-precision operator
   if ((r = apply_op(h, spin, ik, X, n, nd, HX, 0, s)) != kOk) return r;
   out.happ += nd;
@@ -581,8 +591,11 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
   T* XX = as<T>(w.XX);
   if ((r = gemm(c, CUBLAS_OP_C, CUBLAS_OP_N, nd, nd, (int)n, X, n, HX, n, XX, nd)) != kOk) return r;
   k_diag_real<T><<<blocks_for(nd), 256, 0, s>>>(XX, nd, nd, w.lam); count_launch();
+  int wbad = 0;
   PW_CUDA_TRY(cudaMemcpyAsync(k.evals.data(), w.lam, nd * sizeof(double), cudaMemcpyDeviceToHost, s));
+  PW_CUDA_TRY(cudaMemcpyAsync(&wbad, bst, sizeof(int), cudaMemcpyDeviceToHost, s));
   PW_CUDA_TRY(cudaStreamSynchronize(s));
+  if (wbad) return fail(kNotConverged, "eigensolver: start block is numerically rank deficient");
   bool first = true;
 
   const double p_drop = precision == 0 ? kPDropFp64 : kPDropMixed;
@@ -590,6 +603,8 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
   T* Pn = as<T>(w.Pn);
   T* HPn = as<T>(w.HPn);
   std::vector<double> rn(nd), nu0, nu1;
+  std::vector<double> pack(steps ? 2 + 4 * (size_t)nd : 0);  // w.status, w.lam0 (3 nd), w.colsq
+  bool dev_lam = false;  // the Ritz values of the last step are in w.lam0 only
   std::vector<int> act, pband, keep, pk;
   int np = 0;  // columns of Pn / HPn (bands pband)
   out.iters = 0;
@@ -597,12 +612,24 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
   for (;;) {
     const auto t0 = std::chrono::steady_clock::now();
     pt.mark(0, s);
-    PW_CUDA_TRY(cudaMemcpyAsync(w.lam0, k.evals.data(), nd * sizeof(double), cudaMemcpyHostToDevice, s));
+    if (!dev_lam) PW_CUDA_TRY(cudaMemcpyAsync(w.lam0, k.evals.data(), nd * sizeof(double), cudaMemcpyHostToDevice, s));
     k_resid_precond<T><<<dim3(c.gx, nd), 256, 0, s>>>(X, HX, Tb, n, (int)n, w.lam0, kin, v0, w.partials);
     count_launch();
     k_col_final<<<blocks_for(nd), 256, 0, s>>>(w.partials, (int)c.gx, nd, w.colsq); count_launch();
-    PW_CUDA_TRY(cudaMemcpyAsync(rn.data(), w.colsq, nd * sizeof(double), cudaMemcpyDeviceToHost, s));
-    PW_CUDA_TRY(cudaStreamSynchronize(s));
+    if (steps) {
+      // status, Ritz values and residual norms in one copy (they are adjacent)
+      PW_CUDA_TRY(cudaMemcpyAsync(pack.data(), w.status, pack.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
+      PW_CUDA_TRY(cudaStreamSynchronize(s));
+      const int* st = reinterpret_cast<const int*>(pack.data());
+      if (st[0] != 0) return fail(kNotConverged, "eigensolver: subspace eigensolve produced non-finite values");
+      if (st[1] != 0) return fail(kNotConverged, "eigensolver: search block is numerically rank deficient");
+      if (dev_lam) std::copy(pack.begin() + 2, pack.begin() + 2 + nd, k.evals.begin());
+      dev_lam = false;
+      std::copy(pack.begin() + 2 + 3 * nd, pack.begin() + 2 + 4 * nd, rn.begin());
+    } else {
+      PW_CUDA_TRY(cudaMemcpyAsync(rn.data(), w.colsq, nd * sizeof(double), cudaMemcpyDeviceToHost, s));
+      PW_CUDA_TRY(cudaStreamSynchronize(s));
+    }
     out.max_res = 0.0;
     for (int b = 0; b < nconv; ++b) out.max_res = std::max(out.max_res, std::sqrt(rn[b]));
     if (out.max_res < tol || out.iters >= max_iter) {
@@ -623,10 +650,14 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
     T* HW = HX + n * nd;
     pt.mark(1, s);
     PW_CUDA_TRY(cudaMemcpyAsync(w.idx, act.data(), na * sizeof(int), cudaMemcpyHostToDevice, s));
-    k_gather_cols<T><<<dim3(c.gx, na), 256, 0, s>>>(Tb, n, w.idx, W, n, (int)n); count_launch();
-    if ((r = project_out(c, (const T*)X, (const T*)nullptr, nd, W, (T*)nullptr, na)) != kOk) return r;
-    if ((r = project_out(c, (const T*)X, (const T*)nullptr, nd, W, (T*)nullptr, na)) != kOk) return r;
-    if ((r = orthonormalize(c, W, na)) != kOk) return r;
+    if (steps) {
+      if ((r = block_w<T>(X, nd, Tb, w.idx, na, W, n, xch, bst, s)) != kOk) return r;
+    } else {
+      k_gather_cols<T><<<dim3(c.gx, na), 256, 0, s>>>(Tb, n, w.idx, W, n, (int)n); count_launch();
+      if ((r = project_out(c, (const T*)X, (const T*)nullptr, nd, W, (T*)nullptr, na)) != kOk) return r;
+      if ((r = project_out(c, (const T*)X, (const T*)nullptr, nd, W, (T*)nullptr, na)) != kOk) return r;
+      if ((r = orthonormalize(c, W, na)) != kOk) return r;
+    }
     pt.mark(2, s);
     if ((r = apply_op(h, spin, ik, W, n, na, HW, precision, s)) != kOk) return r;
     out.happ += na;
@@ -641,7 +672,13 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
     if ((long)pk.size() > n - nd - na) pk.resize((size_t)std::max<long>(0, n - nd - na));
     T* P = W + n * na;
     T* HP = HW + n * na;
-    if (!pk.empty()) {
+    if (!pk.empty() && steps) {
+      npc = (int)pk.size();
+      PW_CUDA_TRY(cudaMemcpyAsync(w.idx, pk.data(), npc * sizeof(int), cudaMemcpyHostToDevice, s));
+      if ((r = block_p<T>(X, HX, nd, W, HW, na, Pn, HPn, w.idx, npc, P, HP, n, p_drop, xch, bst, s)) != kOk) return r;
+      PW_CUDA_TRY(cudaMemcpyAsync(&npc, bst + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+      PW_CUDA_TRY(cudaStreamSynchronize(s));
+    } else if (!pk.empty()) {
       npc = (int)pk.size();
       PW_CUDA_TRY(cudaMemcpyAsync(w.idx, pk.data(), npc * sizeof(int), cudaMemcpyHostToDevice, s));
       k_gather_cols<T><<<dim3(c.gx, npc), 256, 0, s>>>(Pn, n, w.idx, P, n, (int)n); count_launch();
@@ -689,33 +726,41 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
       // and P is their residual, below tol) at a third of the subspace size
       pt.mark(4, s);
       const int ms = na + q;
-      T* Bx = Tb;                      // [X_a | W | P], n x ms
-      T* Bh = as<T>(w.HXn);            // [HX_a | HW | HP]
-      PW_CUDA_TRY(cudaMemcpyAsync(w.idx, act.data(), na * sizeof(int), cudaMemcpyHostToDevice, s));
-      k_gather_cols<T><<<dim3(c.gx, na), 256, 0, s>>>(X, n, w.idx, Bx, n, (int)n); count_launch();
-      k_gather_cols<T><<<dim3(c.gx, na), 256, 0, s>>>(HX, n, w.idx, Bh, n, (int)n); count_launch();
-      PW_CUDA_TRY(cudaMemcpyAsync(Bx + n * na, W, n * q * sizeof(T), cudaMemcpyDeviceToDevice, s));
-      PW_CUDA_TRY(cudaMemcpyAsync(Bh + n * na, HW, n * q * sizeof(T), cudaMemcpyDeviceToDevice, s));
       std::vector<double> lam_a(na);
       for (int j = 0; j < na; ++j) lam_a[j] = k.evals[act[j]];
+      PW_CUDA_TRY(cudaMemcpyAsync(w.idx, act.data(), na * sizeof(int), cudaMemcpyHostToDevice, s));
       PW_CUDA_TRY(cudaMemcpyAsync(w.lam0, lam_a.data(), na * sizeof(double), cudaMemcpyHostToDevice, s));
-      if ((r = gemm(c, CUBLAS_OP_C, CUBLAS_OP_N, q, na, (int)n, W, n, Bh, n, as<T>(w.Z), q)) != kOk) return r;
-      if ((r = gemm(c, CUBLAS_OP_C, CUBLAS_OP_N, q, q, (int)n, W, n, HW, n, as<T>(w.G), q)) != kOk) return r;
-      k_assemble_rr<T><<<blocks_for((long)ms * ms), 256, 0, s>>>(as<T>(w.Hs), ms, na, w.lam0, as<T>(w.Z),
-                                                                  as<T>(w.G));
-      count_launch();
       T* C = nullptr;
-      pt.mark(5, s);
-      if ((r = subspace_eig<T>(c, ms, na, &C)) != kOk) return r;
-      pt.mark(6, s);
-      // new active X, HX into the W, HW columns; new P, HP from the (W, P) rows
-      if ((r = gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, (int)n, na, ms, Bx, n, C, ms, W, n)) != kOk) return r;
-      if ((r = gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, (int)n, na, ms, Bh, n, C, ms, HW, n)) != kOk) return r;
-      if ((r = gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, (int)n, na, q, Bx + n * na, n, C + na, ms, Pn, n)) != kOk) return r;
-      if ((r = gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, (int)n, na, q, Bh + n * na, n, C + na, ms, HPn, n)) != kOk)
-        return r;
-      k_scatter_cols<T><<<dim3(c.gx, na), 256, 0, s>>>(W, n, w.idx, X, n, (int)n); count_launch();
-      k_scatter_cols<T><<<dim3(c.gx, na), 256, 0, s>>>(HW, n, w.idx, HX, n, (int)n); count_launch();
+      if (steps) {
+        if ((r = block_rr<T>(W, HW, q, HX, w.idx, na, w.lam0, nullptr, n, xch, as<T>(w.Hs), s)) != kOk) return r;
+        pt.mark(5, s);
+        if ((r = subspace_eig<T>(c, ms, na, &C)) != kOk) return r;
+        pt.mark(6, s);
+        if ((r = block_update<T>(X, W, Pn, HX, HW, HPn, C, ms, na, q, w.idx, nullptr, na, n, s)) != kOk) return r;
+      } else {
+        T* Bx = Tb;                      // [X_a | W | P], n x ms
+        T* Bh = as<T>(w.HXn);            // [HX_a | HW | HP]
+        k_gather_cols<T><<<dim3(c.gx, na), 256, 0, s>>>(X, n, w.idx, Bx, n, (int)n); count_launch();
+        k_gather_cols<T><<<dim3(c.gx, na), 256, 0, s>>>(HX, n, w.idx, Bh, n, (int)n); count_launch();
+        PW_CUDA_TRY(cudaMemcpyAsync(Bx + n * na, W, n * q * sizeof(T), cudaMemcpyDeviceToDevice, s));
+        PW_CUDA_TRY(cudaMemcpyAsync(Bh + n * na, HW, n * q * sizeof(T), cudaMemcpyDeviceToDevice, s));
+        if ((r = gemm(c, CUBLAS_OP_C, CUBLAS_OP_N, q, na, (int)n, W, n, Bh, n, as<T>(w.Z), q)) != kOk) return r;
+        if ((r = gemm(c, CUBLAS_OP_C, CUBLAS_OP_N, q, q, (int)n, W, n, HW, n, as<T>(w.G), q)) != kOk) return r;
+        k_assemble_rr<T><<<blocks_for((long)ms * ms), 256, 0, s>>>(as<T>(w.Hs), ms, na, w.lam0, as<T>(w.Z),
+                                                                    as<T>(w.G));
+        count_launch();
+        pt.mark(5, s);
+        if ((r = subspace_eig<T>(c, ms, na, &C)) != kOk) return r;
+        pt.mark(6, s);
+        // new active X, HX into the W, HW columns; new P, HP from the (W, P) rows
+        if ((r = gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, (int)n, na, ms, Bx, n, C, ms, W, n)) != kOk) return r;
+        if ((r = gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, (int)n, na, ms, Bh, n, C, ms, HW, n)) != kOk) return r;
+        if ((r = gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, (int)n, na, q, Bx + n * na, n, C + na, ms, Pn, n)) != kOk) return r;
+        if ((r = gemm(c, CUBLAS_OP_N, CUBLAS_OP_N, (int)n, na, q, Bh + n * na, n, C + na, ms, HPn, n)) != kOk)
+          return r;
+        k_scatter_cols<T><<<dim3(c.gx, na), 256, 0, s>>>(W, n, w.idx, X, n, (int)n); count_launch();
+        k_scatter_cols<T><<<dim3(c.gx, na), 256, 0, s>>>(HW, n, w.idx, HX, n, (int)n); count_launch();
+      }
       PW_CUDA_TRY(cudaMemcpyAsync(lam_a.data(), w.lam, na * sizeof(double), cudaMemcpyDeviceToHost, s));
       PW_CUDA_TRY(cudaStreamSynchronize(s));
       for (int j = 0; j < na; ++j) k.evals[act[j]] = lam_a[j];
@@ -764,13 +809,38 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
     // Rayleigh-Ritz over [X | W | P]
     pt.mark(4, s);
     const int m = nd + q;
+    T* C = nullptr;
+    if (steps) {
+      if ((r = block_rr<T>(W, HW, q, HX, nullptr, nd, w.lam0, first ? XX : nullptr, n, xch, as<T>(w.Hs), s)) != kOk)
+        return r;
+      first = false;
+      pt.mark(5, s);
+      if ((r = subspace_eig<T>(c, m, nd, &C, true)) != kOk) return r;
+      pt.mark(6, s);
+      PW_CUDA_TRY(cudaMemcpyAsync(w.idx, act.data(), na * sizeof(int), cudaMemcpyHostToDevice, s));
+      if ((r = block_update<T>(X, W, Pn, HX, HW, HPn, C, m, nd, q, nullptr, w.idx, na, n, s)) != kOk) return r;
+      // values and status are read with the next residual norms
+      PW_CUDA_TRY(cudaMemcpyAsync(w.lam0, w.lam, nd * sizeof(double), cudaMemcpyDeviceToDevice, s));
+      pt.mark(7, s);
+      dev_lam = true;
+      np = na;
+      pband = act;
+      ++out.iters;
+      if (h.trace) {
+        PW_CUDA_TRY(cudaStreamSynchronize(s));
+        pt.accumulate();
+        std::fprintf(stderr, "pwgpu lobpcg k=%d it=%d res=%.3e na=%d np=%d steps %.2f ms\n", ik, out.iters, out.max_res,
+                     na, npc,
+                     std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count());
+      }
+      continue;
+    }
     if ((r = gemm(c, CUBLAS_OP_C, CUBLAS_OP_N, q, nd, (int)n, W, n, HX, n, as<T>(w.Z), q)) != kOk) return r;
     if ((r = gemm(c, CUBLAS_OP_C, CUBLAS_OP_N, q, q, (int)n, W, n, HW, n, as<T>(w.G), q)) != kOk) return r;
     k_assemble_rr<T><<<blocks_for((long)m * m), 256, 0, s>>>(as<T>(w.Hs), m, nd, w.lam0, as<T>(w.Z), as<T>(w.G),
                                                             first ? XX : nullptr);
     count_launch();
     first = false;
-    T* C = nullptr;
     pt.mark(5, s);
     if ((r = subspace_eig<T>(c, m, nd, &C)) != kOk) return r;
     pt.mark(6, s);
@@ -827,11 +897,15 @@ Status eig_work_alloc(EigWork& w, long n, int nd) {
   if ((r = walloc(&w.XX, (size_t)nd * nd)) != kOk) return r;
   if ((r = walloc(&w.defect, 2)) != kOk) return r;
   if ((r = walloc(&w.lam, m)) != kOk) return r;
-  if ((r = walloc(&w.lam0, m)) != kOk) return r;
-  if ((r = walloc(&w.colsq, m)) != kOk) return r;
+  // status (two doubles' room), lam0 and colsq are adjacent: one copy brings them to the host
+  double* adj = nullptr;
+  if ((r = walloc(&adj, 2 + 2 * m)) != kOk) return r;
+  w.status = reinterpret_cast<int*>(adj);
+  w.lam0 = adj + 2;
+  w.colsq = adj + 2 + m;
+  if (nd <= kMaxBlock && (r = walloc(&w.xch, block_steps_xch(nd))) != kOk) return r;
   if ((r = walloc(&w.partials, m * kColBlocks)) != kOk) return r;
   if ((r = walloc(&w.idx, m)) != kOk) return r;
-  if ((r = walloc(&w.status, 1)) != kOk) return r;
   if ((r = walloc(&w.info, 1)) != kOk) return r;
   return kOk;
 }
@@ -839,7 +913,7 @@ Status eig_work_alloc(EigWork& w, long n, int nd) {
 void eig_work_release(EigWork& w) {
   auto f = [](void* p) { if (p) cudaFree(p); };
   f(w.T); f(w.HXn); f(w.Pn); f(w.HPn); f(w.Hs); f(w.Cs); f(w.G); f(w.Z); f(w.Id);
-  f(w.lam); f(w.lam0); f(w.colsq); f(w.partials); f(w.idx); f(w.status); f(w.solver_work); f(w.info);
+  f(w.lam); f(w.status); f(w.xch); f(w.partials); f(w.idx); f(w.solver_work); f(w.info);
   f(w.eigh_work); f(w.XX); f(w.defect);
   w = EigWork();
 }

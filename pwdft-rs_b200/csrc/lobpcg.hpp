@@ -36,7 +36,8 @@ struct EigWork {
   double* colsq = nullptr; // 3 nd
   double* partials = nullptr;
   int* idx = nullptr;      // 3 nd
-  int* status = nullptr;
+  int* status = nullptr;   // [0] subspace eigensolve, [1] W rank deficient, [2] columns of P (block steps)
+  double2* xch = nullptr;  // exchange buffer of the block steps (nd <= kMaxBlock)
   double2* solver_work = nullptr;
   size_t solver_lwork = 0;
   int* info = nullptr;
@@ -64,5 +65,29 @@ void eig_vecs_release(EigVecs& v);
 // diagonal shift.
 Status lobpcg(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, double tol, int max_iter, int nconv,
               int precision, EigStats& out);
+
+// Fused block steps for narrow blocks (block_steps.cu), T = double or double2.
+// block_steps_fit: whether a block of nd columns of n rows takes them.
+constexpr int kMaxBlock = 64;
+template <typename T> bool block_steps_fit(long n, int nd);
+size_t block_steps_xch(int nd);  // entries of T in the exchange buffer
+// W (n x na) = orthonormal basis of Tb(:, idx) outside span(X) (idx NULL: columns in order; nd 0: no projection, W
+// may be Tb); status[0] = 1 when rank deficient.
+template <typename T>
+Status block_w(const T* X, int nd, const T* Tb, const int* idx, int na, T* W, long n, T* xch, int* status,
+               cudaStream_t s);
+// P, HP from Pn(:, idx), HPn(:, idx): projected out of X and W, near-dependent columns dropped, orthonormal;
+// status[1] = columns kept.
+template <typename T>
+Status block_p(const T* X, const T* HX, int nd, const T* W, const T* HW, int na, const T* Pn, const T* HPn,
+               const int* idx, int np, T* P, T* HP, long n, double p_drop, T* xch, int* status, cudaStream_t s);
+// Subspace matrix over [X(:, cols) | B], B = [W | P] with q columns (cols NULL: all in order).
+template <typename T>
+Status block_rr(const T* B, const T* HB, int q, const T* HX, const int* cols, int nx, const double* lam, const T* XX,
+                long n, T* xch, T* Hs, cudaStream_t s);
+// X(:, cols) and Pn from the subspace eigenvectors Cm (m x nx), and the same for HX, HPn.
+template <typename T>
+Status block_update(T* X, const T* B, T* Pn, T* HX, const T* HB, T* HPn, const T* Cm, int m, int nx, int q,
+                    const int* cols, const int* pcols, int np, long n, cudaStream_t s);
 
 }  // namespace pwgpu

@@ -1,0 +1,61 @@
+"""The fused block steps of the eigensolver (narrow blocks) against dense diagonalisation.
+
+Block widths at the edges of the kernels: 3 columns, 32 / 33 (four and eight column tiles), 47 / 48 complex and 64 / 65
+real (the widest fused block and the first that takes the library products), and row counts from fewer than a
+cluster's CTAs hold to several thousand with a remainder.  nd = bands + max(2, bands // 8).  Bars as the other
+eigensolver tests: eigenvalues 1e-7 Ha; residuals below the requested 1e-7 eV; |X^H X - I| 1e-11 (Cholesky-QR passes
+leave 1e-12, the Ritz rotations since then a few rounding errors each)."""
+
+import numpy as np
+import pytest
+
+from conftest import rng
+from oracle import pwdft_oracle as O
+from pwgpu.context import build_system
+from pwgpu.crystal import KPoint, diamond_primitive, diamond_supercell, gamma_only
+from pwgpu.lib import PwGpu
+from pwgpu.symmetry import SymmetryInfo
+
+pytestmark = pytest.mark.gpu
+
+HA = 27.211386245988
+
+
+def _veff(s):
+    rho_g = O.density_r_to_g(s.rho_init_r, s.dims)
+    _, vxc = O.lda_xc(O.add_core(s.rho_init_r, s.rho_core_r))
+    return s.v_local_g + O.hartree(rho_g, s.g_squared) + O.density_r_to_g(vxc, s.dims)
+
+
+def _check(s, bands):
+    veff = _veff(s)
+    p = s.projectors[0]
+    h = O.dense_hamiltonian(s.basis.miller, s.kinetic[0], veff, s.dims, p.b, p.d_dense())
+    ref = np.linalg.eigvalsh(h)[:bands]
+    with PwGpu(s) as dev:
+        dev.set_veff_g(veff)
+        ev, psi, _, res = dev.eigensolve(bands, tol=1e-7, max_iter=400)
+    assert np.max(np.abs(ev - ref)) / HA < 1e-7
+    assert res < 1e-7
+    assert np.max(np.abs(psi.conj().T @ psi - np.eye(bands))) < 1e-11
+    assert np.max(np.linalg.norm(h @ psi - psi * ev, axis=0)) < 1e-6
+
+
+@pytest.mark.parametrize("bands", [1, 7, 29, 30, 42, 43])
+def test_complex_blocks(bands, si_pp):
+    s = build_system(diamond_primitive("Si", 5.431), {"Si": si_pp}, 260.0, [KPoint(np.array([0.11, -0.23, 0.31]), 1.0)])
+    _check(s, bands)
+
+
+@pytest.mark.parametrize("bands", [1, 20, 29, 30, 57, 58])
+def test_gamma_real_blocks(bands, si_pp):
+    cr = diamond_supercell("Si", 5.431, (1, 1, 1), 0.02, rng(5))
+    s = build_system(cr, {"Si": si_pp}, 190.0, gamma_only(), SymmetryInfo.identity_only())
+    _check(s, bands)
+
+
+@pytest.mark.parametrize("ecut,bands", [(30.0, 3), (45.0, 9), (80.0, 4)])
+def test_few_plane_waves(ecut, bands, si_pp):
+    """Rows for one or two CTAs only, and blocks close to the whole space."""
+    s = build_system(diamond_primitive("Si", 5.431), {"Si": si_pp}, ecut, [KPoint(np.array([0.05, 0.1, -0.2]), 1.0)])
+    _check(s, bands)
