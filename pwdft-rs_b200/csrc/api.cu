@@ -50,7 +50,7 @@ static void release(Handle& h) {
   f(h.ch_atom); f(h.atom_ch_start); f(h.d_off); f(h.d_vals);
   f(h.v_local_g); f(h.g_squared); f(h.rho_core_r); f(h.rho_sad); f(h.sym_src); f(h.sym_arg);
   for (int s = 0; s < 2; ++s) { f(h.veff_r[s]); f(h.veff_r32[s]); f(h.veff_rz[s]); f(h.veff_rz32[s]); }
-  f(h.work_a); f(h.work_b); f(h.nl_p); f(h.nl_q); f(h.tmp_grid);
+  f(h.work_a); f(h.work_b); f(h.nl_p); f(h.nl_q); f(h.nl_xch); f(h.tmp_grid);
   release_scf(h);
   release_nl_mixed(h);
   f(h.solver_work); f(h.solver_info);

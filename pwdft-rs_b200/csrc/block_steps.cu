@@ -159,9 +159,9 @@ __device__ void cluster_sum(cg::cluster_group& cl, T* Z, int ldz, int p, int q, 
   __syncthreads();
 }
 
-// out(i, c) = base(i, c) - sum_k A(i, k) Z(k, c), c < q, over 8-row strips of the local rows (NQ tiles of 8
-// columns in registers).  A strip is read whole before it is written, so out may alias A.
-template <int NQ, bool SUB, typename T, typename LA, typename LC, typename ST>
+// out(i, c) = sum_k A(i, k) Z(k, c), or base(i, c) minus / plus it (OP -1 / +1), c < q, over 8-row strips of the
+// local rows (NQ tiles of 8 columns in registers).  A strip is read whole before it is written, so out may alias A.
+template <int NQ, int OP, typename T, typename LA, typename LC, typename ST>
 __device__ void local_update(int rows, int kdim, int q, LA la, const T* Z, int ldz, LC lc, ST st) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kr = lane & 3, kc = lane >> 2;
@@ -187,7 +187,10 @@ __device__ void local_update(int rows, int kdim, int q, LA la, const T* Z, int l
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int c = 8 * t + 2 * kr + h;
-        if (rin && c < q) st(i0 + kc, c, SUB ? sub(lc(i0 + kc, c), acc[t].get(h)) : acc[t].get(h));
+        if (rin && c < q) {
+          const T v = acc[t].get(h);
+          st(i0 + kc, c, OP < 0 ? sub(lc(i0 + kc, c), v) : OP > 0 ? add(lc(i0 + kc, c), v) : v);
+        }
       }
     __syncwarp();
   }
@@ -287,7 +290,7 @@ __global__ void __launch_bounds__(kT, 1)
     local_gram<T>(rows, nd, na, lx, ly, Z, ldz);
     cluster_sum<T>(cl, Z, ldz, nd, na, xch + par * xch_len);
     par ^= 1;
-    local_update<NQ, true, T>(rows, nd, na, lx, Z, ldz, ly, [&](int i, int c, T v) { Y[i + c * ldy] = v; });
+    local_update<NQ, -1, T>(rows, nd, na, lx, Z, ldz, ly, [&](int i, int c, T v) { Y[i + c * ldy] = v; });
     __syncthreads();
   }
   bool ok = true;
@@ -342,7 +345,7 @@ __global__ void __launch_bounds__(kT, 1)
       Ri[r + c * ldz] = mul(Ri[r + c * ldz], scol[r]);
     }
     __syncthreads();
-    local_update<NQ, false, T>(rows, na, na, ly, Ri, ldz, ly, [&](int i, int c, T v) { Y[i + c * ldy] = v; });
+    local_update<NQ, 0, T>(rows, na, na, ly, Ri, ldz, ly, [&](int i, int c, T v) { Y[i + c * ldy] = v; });
     __syncthreads();
   }
   for (int e = threadIdx.x; e < rows * na; e += kT) {
@@ -398,8 +401,8 @@ __global__ void __launch_bounds__(kT, 1)
     cluster_sum<T>(cl, Z, ldz, nd + 1, np, xch + par * xch_len);
     par ^= 1;
     if (threadIdx.x < np) nu0[threadIdx.x] = re(Z[nd + threadIdx.x * ldz]);
-    local_update<NQ, true, T>(rows, nd, np, lx, Z, ldz, ly, sy);
-    local_update<NQ, true, T>(
+    local_update<NQ, -1, T>(rows, nd, np, lx, Z, ldz, ly, sy);
+    local_update<NQ, -1, T>(
         rows, nd, np, [&](int i, int c) { return HX[r0 + i + (long)c * n]; }, Z, ldz,
         [&](int i, int c) { return HPn[r0 + i + (long)idx[c] * n]; },
         [&](int i, int c, T v) { HP[r0 + i + (long)c * n] = v; });
@@ -412,8 +415,8 @@ __global__ void __launch_bounds__(kT, 1)
     local_gram<T>(rows, na, np, lw, ly, Z, ldz);
     cluster_sum<T>(cl, Z, ldz, na, np, xch + par * xch_len);
     par ^= 1;
-    local_update<NQ, true, T>(rows, na, np, lw, Z, ldz, ly, sy);
-    local_update<NQ, true, T>(
+    local_update<NQ, -1, T>(rows, na, np, lw, Z, ldz, ly, sy);
+    local_update<NQ, -1, T>(
         rows, na, np, [&](int i, int c) { return HW[r0 + i + (long)c * n]; }, Z, ldz, lhp, shp);
     __syncthreads();
   }
@@ -467,9 +470,9 @@ __global__ void __launch_bounds__(kT, 1)
       Ri[r + c * ldz] = mul(Ri[r + c * ldz], scol[r]);
     }
     __syncthreads();
-    local_update<NQ, false, T>(
+    local_update<NQ, 0, T>(
         rows, nk, nk, [&](int i, int c) { return Y[i + keep[c] * ldy]; }, Ri, ldz, ly, sy);
-    local_update<NQ, false, T>(
+    local_update<NQ, 0, T>(
         rows, nk, nk, [&](int i, int c) { return HP[r0 + i + (long)keep[c] * n]; }, Ri, ldz, lhp, shp);
     __syncthreads();
   }
@@ -586,6 +589,39 @@ __global__ void __launch_bounds__(kUpdThreads)
     }
 }
 
+// hpsi += B D B^H psi for nb bands: P = B^H psi summed over the cluster, Q = D P (D block-diagonal over atoms, blocks
+// row-major) and the update of the rows, in one launch.
+template <typename T, int NQ>
+__global__ void __launch_bounds__(kT, 1)
+    k_block_nl(const T* __restrict__ B, int n_ch, const T* __restrict__ psi, long ldpsi, int nb, T* __restrict__ hpsi,
+               long ldh, long n, int rpc, int ldz, T* __restrict__ xch, const int* __restrict__ ch_atom,
+               const int* __restrict__ atom_ch_start, const int* __restrict__ d_off,
+               const double* __restrict__ d_vals) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  T* Z = reinterpret_cast<T*>(smem);    // n_ch x nb
+  T* Q = Z + (size_t)ldz * nb;          // n_ch x nb
+  cg::cluster_group cl = cg::this_cluster();
+  const long r0 = (long)cl.block_rank() * rpc;
+  const int rows = (int)max(0L, min((long)rpc, n - r0));
+  auto lb = [&](int i, int c) { return c < n_ch ? B[r0 + i + (long)c * n] : zero<T>(); };
+  local_gram<T>(
+      rows, n_ch, nb, lb, [&](int i, int c) { return c < nb ? psi[r0 + i + (long)c * ldpsi] : zero<T>(); }, Z, ldz);
+  cluster_sum<T>(cl, Z, ldz, n_ch, nb, xch);
+  for (int e = threadIdx.x; e < n_ch * nb; e += kT) {
+    const int c = e % n_ch, b = e / n_ch, a = ch_atom[c], s = atom_ch_start[a], nc = atom_ch_start[a + 1] - s;
+    const double* drow = d_vals + d_off[a] + (long)(c - s) * nc;
+    T acc = zero<T>();
+    for (int j = 0; j < nc; ++j) acc = add(acc, mul(Z[s + j + b * ldz], drow[j]));
+    Q[c + b * ldz] = acc;
+  }
+  __syncthreads();
+  for (int b0 = 0; b0 < nb; b0 += 8 * NQ)
+    local_update<NQ, 1, T>(
+        rows, n_ch, min(8 * NQ, nb - b0), lb, Q + (size_t)b0 * ldz, ldz,
+        [&](int i, int c) { return hpsi[r0 + i + (long)(b0 + c) * ldh]; },
+        [&](int i, int c, T v) { hpsi[r0 + i + (long)(b0 + c) * ldh] = v; });
+}
+
 // Rows per CTA and cluster size for n rows: at least 32 rows a CTA, rows in multiples of 8.
 void split_rows(long n, int& C, int& rpc) {
   C = kMaxC;
@@ -615,7 +651,7 @@ template <typename T> Status configure(bool* fits) {
     Status r;
     if ((r = opt_in(k_block_w<T, 4>, true)) != kOk || (r = opt_in(k_block_w<T, 8>, true)) != kOk ||
         (r = opt_in(k_block_p<T, 4>, true)) != kOk || (r = opt_in(k_block_p<T, 8>, true)) != kOk ||
-        (r = opt_in(k_block_rr<T>, true)) != kOk)
+        (r = opt_in(k_block_rr<T>, true)) != kOk || (r = opt_in(k_block_nl<T, 4>, true)) != kOk)
       return r;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
@@ -723,7 +759,39 @@ Status block_update(T* X, const T* B, T* Pn, T* HX, const T* HB, T* HPn, const T
   return kOk;
 }
 
+// One launch is the faster form while the products are small enough for one
+// cluster's FP64 rate (16 of the 148 SMs); beyond that the library products'
+// spread over the whole GPU wins.
+template <typename T> bool nl_fused_ok(const Handle& h, int nb) {
+  const double work = (double)h.n_pw * h.n_ch * nb;
+  if (h.n_ch < 1 || work > (sizeof(T) == sizeof(double) ? 8.0e6 : 2.5e6)) return false;
+  if ((size_t)2 * pad_ld(h.n_ch) * nb * sizeof(T) > kSmemMax) return false;
+  bool fits = false;
+  return configure<T>(&fits) == kOk && fits;
+}
+
+template <typename T>
+Status nl_fused(Handle& h, const T* B, const T* psi, long ldpsi, int nb, T* hpsi, long ldh, cudaStream_t s) {
+  const size_t need = (size_t)(kMaxC + 1) * h.n_ch * nb * sizeof(T);
+  if (need > h.nl_xch_bytes) {
+    if (h.nl_xch) cudaFree(h.nl_xch);
+    h.nl_xch = nullptr;
+    h.nl_xch_bytes = 0;
+    cudaError_t e = cudaMalloc(&h.nl_xch, need);
+    if (e != cudaSuccess) return fail(kOom, std::string("cudaMalloc (projector exchange): ") + cudaGetErrorString(e));
+    h.nl_xch_bytes = need;
+  }
+  int C, rpc;
+  split_rows(h.n_pw, C, rpc);
+  const int ldz = pad_ld(h.n_ch);
+  return launch(k_block_nl<T, 4>, C, (size_t)2 * ldz * nb * sizeof(T), s, B, h.n_ch, psi, ldpsi, nb, hpsi, ldh,
+                (long)h.n_pw, rpc, ldz, static_cast<T*>(h.nl_xch), (const int*)h.ch_atom,
+                (const int*)h.atom_ch_start, (const int*)h.d_off, (const double*)h.d_vals);
+}
+
 #define PW_BLOCK(T)                                                                                                  \
+  template bool nl_fused_ok<T>(const Handle&, int);                                                                 \
+  template Status nl_fused<T>(Handle&, const T*, const T*, long, int, T*, long, cudaStream_t);                       \
   template bool block_steps_fit<T>(long, int);                                                                      \
   template Status block_w<T>(const T*, int, const T*, const int*, int, T*, long, T*, int*, cudaStream_t);            \
   template Status block_p<T>(const T*, const T*, int, const T*, const T*, int, const T*, const T*, const int*, int, \

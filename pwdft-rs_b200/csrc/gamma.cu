@@ -397,6 +397,8 @@ Status apply_h_real(Handle& h, int spin, const double* u, long ldu, int nb, doub
     // block width: on the four-cell Si64 batch this measured 1 % above
     // keeping the FP64 GEMMs for blocks narrower than 48 or 96 bands)
     if ((r = nonlocal_mixed_real(h, u, ldu, nb, hu, ldh, s)) != kOk) return r;
+  } else if (nl_fused_ok<double>(h, nb)) {
+    if ((r = nl_fused<double>(h, g.b_real, u, ldu, nb, hu, ldh, s)) != kOk) return r;
   } else if (h.n_ch > 0) {
     if ((r = nonlocal_pq_real(h, u, ldu, nb, s)) != kOk) return r;
     const double one = 1.0;

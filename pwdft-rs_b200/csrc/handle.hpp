@@ -98,6 +98,8 @@ struct Handle {
   double2* nl_p = nullptr;  // n_ch x max_nb
   double2* nl_q = nullptr;
   int nl_cap = 0;
+  void* nl_xch = nullptr;   // exchange buffer of the one-launch projector term
+  size_t nl_xch_bytes = 0;
   double2* tmp_grid = nullptr;  // N complex scratch
   cudaStream_t stream = nullptr;
   cublasHandle_t blas = nullptr;
@@ -169,6 +171,12 @@ Status local_plane(Handle& h, int spin, int ik, const double2* psi, long ldpsi, 
 // P = B^H psi into h.nl_p and Q = D P into h.nl_q (FP64), nb columns.
 Status nonlocal_pq(Handle& h, int ik, const double2* psi, long ldpsi, int nb, cudaStream_t s,
                    StageTimer* tm = nullptr);
+
+// hpsi += B D B^H psi in one launch, for products small enough for one cluster
+// (block_steps.cu); B n_pw x n_ch, T = double (packed real) or double2.
+template <typename T> bool nl_fused_ok(const Handle& h, int nb);
+template <typename T>
+Status nl_fused(Handle& h, const T* B, const T* psi, long ldpsi, int nb, T* hpsi, long ldh, cudaStream_t s);
 
 // Local part of H|psi> only (kinetic + V_eff through the FFT pipeline).
 Status apply_local_device(Handle& h, int spin, int ik, const double2* psi, long ldpsi, int nb, double2* hpsi,

@@ -1334,6 +1334,9 @@ Status apply_h_device(Handle& h, int spin, int ik, const double2* psi, long ldps
   if ((st = apply_local_device(h, spin, ik, psi, ldpsi, nb, hpsi, ldh, precision, s, tm)) != kOk) return st;
   if (h.n_ch > 0 && precision == 1 && nl_mixed_eligible(h)) {
     if ((st = nonlocal_mixed(h, ik, psi, ldpsi, nb, hpsi, ldh, s, tm)) != kOk) return st;
+  } else if (nl_fused_ok<double2>(h, nb)) {
+    if ((st = nl_fused<double2>(h, h.kp[ik].b, psi, ldpsi, nb, hpsi, ldh, s)) != kOk) return st;
+    mark(tm, 5, s);
   } else if (h.n_ch > 0) {
     if ((st = nonlocal_pq(h, ik, psi, ldpsi, nb, s, tm)) != kOk) return st;
     const cuDoubleComplex one = make_cuDoubleComplex(1.0, 0.0);

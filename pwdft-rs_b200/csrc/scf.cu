@@ -390,12 +390,13 @@ static void release_lane(Lane& L) {
   release_nl_mixed(v);
   release_gamma_scratch(v);
   auto f = [](void* p) { if (p) cudaFree(p); };
-  f(v.work_a); f(v.work_b); f(v.nl_p); f(v.nl_q); f(v.solver_work); f(v.solver_info);
+  f(v.work_a); f(v.work_b); f(v.nl_p); f(v.nl_q); f(v.nl_xch); f(v.solver_work); f(v.solver_info);
   if (v.solver) cusolverDnDestroy(v.solver);
   if (v.blas) cublasDestroy(v.blas);
   if (v.stream) cudaStreamDestroy(v.stream);
   v.work_a = v.work_b = nullptr;
   v.nl_p = v.nl_q = nullptr;
+  v.nl_xch = nullptr;
   v.solver_work = nullptr;
   v.solver_info = nullptr;
   v.solver = nullptr;
@@ -415,6 +416,8 @@ static Status create_lane(Handle& h, Lane& L, int nd, int nlanes) {
   v.work_a = v.work_b = nullptr;
   v.nl_p = v.nl_q = nullptr;
   v.nl_cap = 0;
+  v.nl_xch = nullptr;
+  v.nl_xch_bytes = 0;
   v.nlm = nullptr;
   v.nlm_real = nullptr;
   v.scf = nullptr;
