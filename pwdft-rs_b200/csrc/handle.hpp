@@ -165,6 +165,9 @@ Status ensure_nl_capacity(Handle& h, int nb);
 // maps are built, and applies the local part of H to nb bands with the
 // compact planes in `scratch` (nb * ncol * d2 entries of R).
 Status plane_setup(Handle& h);
+// rho += sum_b fw[b] |psi_b(r)|^2 on the same grids with equal x and y lengths; the partial sums take work_b.
+Status density_plane(Handle& h, const double2* psi, long ldpsi, int nb, const double* fw_dev, double* rho,
+                     cudaStream_t s);
 template <typename R>
 Status local_plane(Handle& h, int spin, int ik, const double2* psi, long ldpsi, int nb, double2* hpsi, long ldh,
                    cudaStream_t s, void* scratch, StageTimer* tm);

@@ -1254,6 +1254,9 @@ Status density_accumulate(Handle& h, const double2* psi, long ldpsi, int nb, con
                           cudaStream_t s) {
   GridMaps& g = h.g;
   const int d0 = g.d[0], d1 = g.d[1], d2 = g.d[2];
+  // square planes, and room for at least one group of partial sums
+  if (g.plane_ok && g.pair[0] == g.pair[1] && 2L * h.chunk * g.Xp >= d0)
+    return density_plane(h, psi, ldpsi, nb, fw_dev, rho, s);
   double2* A = reinterpret_cast<double2*>(h.work_a);
   double2* B = reinterpret_cast<double2*>(h.work_b);
   if ((d0 + (kThreads / g.wx) - 1) / (kThreads / g.wx) > 16) return fail(kNotImplemented, "density: x tile too tall");

@@ -118,6 +118,86 @@ template <typename R, int R0, int R1> __device__ __noinline__ void rt_y_fwd(cplx
   plane_yd<R0, R1>(Ab, P, g, threadIdx.x, blockDim.x);
 }
 
+// Density: rho partials of one z-plane for a group of bands, y-inverse and
+// x-inverse as in k_plane, the last x stage adding fw |psi(r)|^2 into the
+// thread's registers (its butterflies are the same for every band).  part:
+// [group][z][x][y]; the groups of bands fill the GPU, which one block per line
+// tile, all bands in turn, did not: 20 bands on 36^3 took 59 us in three
+// kernels (z, y, x with the sum: 8 + 8 + 44), now 4 + 8 + 4 us.
+template <int X0, int X1>
+__global__ void __launch_bounds__(plane_threads(X0, X1), X0 > 9 || X1 > 9 ? 1 : 2)
+    k_plane_rho(const double2* __restrict__ A, const double* __restrict__ fw, int nb, int bpc, int d2, PlaneGeo gin,
+                const double2* __restrict__ twx, const double2* __restrict__ twy, double* __restrict__ part) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int d0 = X0 * X1, d1 = d0, ld = d1 | 1, T = plane_threads(X0, X1);
+  constexpr int kRounds = (X0 * d1 + T - 1) / T;
+  PlaneGeo g = gin;
+  g.d0 = d0; g.d1 = d1; g.ld = ld;
+  double2* P = reinterpret_cast<double2*>(smem_raw);
+  double2* TX = P + (g.d0 + (g.Xp > g.avail ? g.Xp - g.avail : 0)) * ld;
+  double2* TY = TX + d0;
+  const int z = blockIdx.x, tid = threadIdx.x;
+  const long ncol = (long)g.Xp * g.Yp;
+  for (int i = tid; i < d0; i += T) TX[i] = twx[i];
+  for (int i = tid; i < d1; i += T) TY[i] = twy[i];
+  double acc[kRounds][X1];
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r)
+#pragma unroll
+    for (int k = 0; k < X1; ++k) acc[r][k] = 0.0;
+  const int b0 = blockIdx.y * bpc, b1 = min(nb, b0 + bpc);
+  for (int b = b0; b < b1; ++b) {
+    __syncthreads();  // the tables, and the previous band's readers
+    plane_ya<X0, X1>(A + ((long)b * d2 + z) * ncol, P, g, TY, tid, T);
+    plane_yb<X0, X1>(P, g, tid, T);
+    plane_xa<X0, X1>(P, g, TX, tid, T);
+    const double f = fw[b];
+#pragma unroll
+    for (int r = 0; r < kRounds; ++r) {
+      const int t = tid + r * T;
+      if (t >= X0 * d1) break;
+      const int k1 = fast_div(t, d1, g.md1), y = t - k1 * d1;
+      const double2* base = P + X1 * k1 * ld + y;
+      double2 v[X1];
+#pragma unroll
+      for (int j = 0; j < X1; ++j) v[j] = base[j * ld];
+      dft_n<X1, +1>(v);
+#pragma unroll
+      for (int k = 0; k < X1; ++k) acc[r][k] += f * (v[k].x * v[k].x + v[k].y * v[k].y);
+    }
+  }
+  double* out = part + ((long)blockIdx.y * d2 + z) * d0 * d1;
+#pragma unroll
+  for (int r = 0; r < kRounds; ++r) {
+    const int t = tid + r * T;
+    if (t >= X0 * d1) break;
+    const int k1 = fast_div(t, d1, g.md1), y = t - k1 * d1;
+#pragma unroll
+    for (int k = 0; k < X1; ++k) out[(k1 + X0 * k) * d1 + y] = acc[r][k];
+  }
+}
+
+// rho[x][y][z] += sum over the groups, in order, of part[g][z][x][y]; 32 x 32 tiles of (y, z) turned in shared memory.
+__global__ void __launch_bounds__(256) k_rho_add(const double* __restrict__ part, int groups, int d0, int d1, int d2,
+                                                 double* __restrict__ rho) {
+  __shared__ double tile[32][33];
+  const int x = blockIdx.x, y0 = blockIdx.y * 32, z0 = blockIdx.z * 32;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const long n = (long)d0 * d1 * d2;
+  for (int r = ty; r < 32; r += 8) {
+    const int y = y0 + tx, z = z0 + r;
+    if (y >= d1 || z >= d2) continue;
+    double s = 0.0;
+    for (int g = 0; g < groups; ++g) s += part[g * n + ((long)z * d0 + x) * d1 + y];
+    tile[r][tx] = s;
+  }
+  __syncthreads();
+  for (int r = ty; r < 32; r += 8) {
+    const int y = y0 + r, z = z0 + tx;
+    if (y < d1 && z < d2) rho[((long)x * d1 + y) * d2 + z] += tile[tx][r];
+  }
+}
+
 constexpr int pair_id(int r0, int r1) { return r0 * 16 + r1; }
 
 template <typename R>
@@ -313,6 +393,7 @@ Status configure() {
 #define PW_CASE(r0, r1)                                                                        \
   set((const void*)k_plane<double, r0, r1>, kPlaneSmemMax);                                    \
   set((const void*)k_plane<float, r0, r1>, kPlaneSmemMax);                                     \
+  set((const void*)k_plane_rho<r0, r1>, kPlaneSmemMax);                                        \
   set((const void*)k_zi<double, r0, r1>, (size_t)kZCols * ((r0 * r1) | 1) * sizeof(double2));  \
   set((const void*)k_zi<float, r0, r1>, (size_t)kZCols * ((r0 * r1) | 1) * sizeof(float2));    \
   set((const void*)k_zf<double, r0, r1>, (size_t)kZCols * ((r0 * r1) | 1) * sizeof(double2));  \
@@ -351,6 +432,55 @@ Status plane_setup(Handle& h) {
 }
 
 template <typename R>
+static void launch_zi(const Handle& h, const double2* psi, long ldpsi, cplx<R>* A, int nb, cudaStream_t s) {
+  const GridMaps& g = h.g;
+  const dim3 grid((g.ncol + kZCols - 1) / kZCols, nb);
+  const size_t sm = (size_t)kZCols * (g.d[2] | 1) * sizeof(cplx<R>);
+  switch (g.pair[2]) {
+#define PW_CASE(r0, r1)                                                                                              \
+  case pair_id(r0, r1):                                                                                              \
+    k_zi<R, r0, r1><<<grid, kZCols*(r0 > r1 ? r0 : r1), sm, s>>>(psi, ldpsi, A, g.col_start, g.col_lo, g.ncol, g.m[2], \
+                                                                 Tables<R>::tw(g, 2));                               \
+    break;
+    PW_PAIRS(PW_CASE)
+#undef PW_CASE
+  }
+  count_launch();
+}
+
+// rho += sum_b fw[b] |psi_b(r)|^2; the partial sums take work_b.
+Status density_plane(Handle& h, const double2* psi, long ldpsi, int nb, const double* fw_dev, double* rho,
+                     cudaStream_t s) {
+  const GridMaps& g = h.g;
+  const int d0 = g.d[0], d1 = g.d[1], d2 = g.d[2];
+  double2* A = static_cast<double2*>(h.work_a);
+  double* part = static_cast<double*>(h.work_b);
+  const int cap = std::max(1, (int)((double)h.chunk * 2.0 * g.Xp / d0));  // groups that fit work_b
+  const PlaneGeo geo = geometry(g);
+  for (int c0 = 0; c0 < nb; c0 += h.chunk_a) {
+    const int cnt = std::min(h.chunk_a, nb - c0);
+    launch_zi<double>(h, psi + (long)c0 * ldpsi, ldpsi, A, cnt, s);
+    int groups = std::min(std::min(cap, cnt), std::max(1, (4 * 148 + d2 - 1) / d2));
+    const int bpc = (cnt + groups - 1) / groups;
+    groups = (cnt + bpc - 1) / bpc;
+    switch (g.pair[0]) {
+#define PW_CASE(r0, r1)                                                                                            \
+  case pair_id(r0, r1):                                                                                            \
+    k_plane_rho<r0, r1><<<dim3(d2, groups), plane_threads(r0, r1), plane_smem<double>(g), s>>>(                    \
+        A, fw_dev + c0, cnt, bpc, d2, geo, g.tw64[0], g.tw64[1], part);                                            \
+    break;
+      PW_PAIRS(PW_CASE)
+#undef PW_CASE
+    }
+    count_launch();
+    k_rho_add<<<dim3(d0, (d1 + 31) / 32, (d2 + 31) / 32), 256, 0, s>>>(part, groups, d0, d1, d2, rho);
+    count_launch();
+  }
+  PW_CUDA_TRY(cudaGetLastError());
+  return kOk;
+}
+
+template <typename R>
 Status local_plane(Handle& h, int spin, int ik, const double2* psi, long ldpsi, int nb, double2* hpsi, long ldh,
                    cudaStream_t s, void* scratch, StageTimer* tm) {
   using C = cplx<R>;
@@ -360,16 +490,7 @@ Status local_plane(Handle& h, int spin, int ik, const double2* psi, long ldpsi, 
   const R* vz = Tables<R>::vz(h, spin);
   const dim3 zgrid((g.ncol + kZCols - 1) / kZCols, nb);
   const size_t zsm = (size_t)kZCols * (g.d[2] | 1) * sizeof(C);
-  switch (g.pair[2]) {
-#define PW_CASE(r0, r1)                                                                                     \
-  case pair_id(r0, r1):                                                                                     \
-    k_zi<R, r0, r1><<<zgrid, kZCols*(r0 > r1 ? r0 : r1), zsm, s>>>(psi, ldpsi, A, g.col_start, g.col_lo,    \
-                                                                   g.ncol, g.m[2], tw2);                    \
-    break;
-    PW_PAIRS(PW_CASE)
-#undef PW_CASE
-  }
-  count_launch();
+  launch_zi<R>(h, psi, ldpsi, A, nb, s);
   mark(tm, 0, s);
   const PlaneGeo geo = geometry(g);
   const int d2 = g.d[2];

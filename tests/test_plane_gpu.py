@@ -120,3 +120,25 @@ def test_large_block_matches_single_bands():
             full = dev.apply_h(psi)
             for b in (0, 255, 256, 511, 529):
                 assert np.array_equal(full[:, b], dev.apply_h(psi[:, b:b + 1])[:, 0])
+
+
+@pytest.mark.parametrize("dims,nb", [((18, 18, 18), 1), ((36, 36, 27), 5), ((60, 60, 16), 40), ((96, 96, 12), 3),
+                                     ((24, 36, 20), 7), ((25, 25, 25), 70)])
+def test_density_matches_numpy(dims, nb):
+    """Square planes (band groups summed per plane) and an unequal one (the line kernels), occupations ending in zero."""
+    m = tuple((d - 1) // 4 for d in dims)
+    s, idx, _ = _system(dims, _sphere(m))
+    g = rng(nb)
+    psi = g.standard_normal((s.n_pw, nb)) + 1j * g.standard_normal((s.n_pw, nb))
+    occ = np.sort(g.uniform(0.1, 2.0, nb))[::-1].copy()
+    if nb > 2:
+        occ[-1] = 0.0
+    rho = np.zeros(dims)
+    for b in range(nb):
+        grid = np.zeros(int(np.prod(dims)), dtype=np.complex128)
+        grid[idx] = psi[:, b]
+        rho += occ[b] * np.abs(np.fft.ifftn(grid.reshape(dims), norm="forward")) ** 2
+    rho *= s.n_electrons / (rho.sum() * s.omega / rho.size)
+    with PwGpu(s, gamma_complex=True) as dev:
+        got = dev.density(occ[None, :], [psi])
+    assert np.max(np.abs(got - rho.ravel())) < 1e-13 * np.max(rho)
