@@ -117,6 +117,31 @@ __global__ void k_resid_precond(const S* __restrict__ X, const S* __restrict__ H
   if (threadIdx.x == 0) partials[(long)col * gridDim.x + blockIdx.x] = acc;
 }
 
+// The same with one block per column and the squared norm of the whole column
+// (narrow blocks: one launch instead of two).
+template <typename S>
+__global__ void __launch_bounds__(512)
+    k_resid_column(const S* __restrict__ X, const S* __restrict__ HX, S* __restrict__ T, long ld, int n,
+                   const double* __restrict__ lam, const double* __restrict__ kin, double v0,
+                   double* __restrict__ sumsq) {
+  __shared__ double sh[32];
+  const int col = blockIdx.x;
+  const double l = lam[col];
+  const S* x = X + (long)col * ld;
+  const S* hx = HX + (long)col * ld;
+  S* t = T + (long)col * ld;
+  double acc = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const S r = axpy_neg(hx[i], l, x[i]);
+    acc += abs2(r);
+    const double xx = (kin[i] + v0 - l) / kRyToEv;
+    const double den = 0.5 * (1.0 + xx + sqrt(1.0 + (xx - 1.0) * (xx - 1.0))) * kRyToEv;
+    t[i] = scl(r, 1.0 / den);
+  }
+  acc = block_sum(acc, sh);
+  if (threadIdx.x == 0) sumsq[col] = acc;
+}
+
 template <typename S>
 __global__ void k_col_sumsq(const S* __restrict__ X, long ld, int n, double* __restrict__ partials) {
   __shared__ double sh[32];
@@ -613,9 +638,13 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
     const auto t0 = std::chrono::steady_clock::now();
     pt.mark(0, s);
     if (!dev_lam) PW_CUDA_TRY(cudaMemcpyAsync(w.lam0, k.evals.data(), nd * sizeof(double), cudaMemcpyHostToDevice, s));
-    k_resid_precond<T><<<dim3(c.gx, nd), 256, 0, s>>>(X, HX, Tb, n, (int)n, w.lam0, kin, v0, w.partials);
-    count_launch();
-    k_col_final<<<blocks_for(nd), 256, 0, s>>>(w.partials, (int)c.gx, nd, w.colsq); count_launch();
+    if (steps) {
+      k_resid_column<T><<<nd, 512, 0, s>>>(X, HX, Tb, n, (int)n, w.lam0, kin, v0, w.colsq); count_launch();
+    } else {
+      k_resid_precond<T><<<dim3(c.gx, nd), 256, 0, s>>>(X, HX, Tb, n, (int)n, w.lam0, kin, v0, w.partials);
+      count_launch();
+      k_col_final<<<blocks_for(nd), 256, 0, s>>>(w.partials, (int)c.gx, nd, w.colsq); count_launch();
+    }
     if (steps) {
       // status, Ritz values and residual norms in one copy (they are adjacent)
       PW_CUDA_TRY(cudaMemcpyAsync(pack.data(), w.status, pack.size() * sizeof(double), cudaMemcpyDeviceToHost, s));

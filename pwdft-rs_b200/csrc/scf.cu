@@ -79,14 +79,25 @@ __global__ void k_final_sum(const double* __restrict__ partials, int n, double* 
   if (threadIdx.x == 0) *out = acc;
 }
 
-// Hartree energy partials: sum_{G^2 > thr} |rho(G)|^2 / G^2
-__global__ void k_hartree(const double2* __restrict__ rho_g, const double* __restrict__ g2, long n,
+// out[s] = sum of the n partials of slot s (stride kRedBlocks), one block per slot
+__global__ void k_final_sums(const double* __restrict__ partials, int n, double* __restrict__ out) {
+  __shared__ double sh[32];
+  const double* p = partials + (long)blockIdx.x * kRedBlocks;
+  double acc = 0.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) acc += p[i];
+  acc = block_sum(acc, sh);
+  if (threadIdx.x == 0) out[blockIdx.x] = acc;
+}
+
+// Hartree potential and energy partials, sum_{G^2 > thr} |rho(G)|^2 / G^2, of rho(G) = scale * ft
+__global__ void k_hartree(const double2* __restrict__ ft, const double* __restrict__ g2, double scale, long n,
                           double2* __restrict__ vh, double fpe2, double* __restrict__ partials) {
   __shared__ double sh[32];
   double acc = 0.0;
   for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const double q = g2[i];
-    const double2 r = rho_g[i];
+    const double2 f = ft[i];
+    const double2 r = make_double2(f.x * scale, f.y * scale);
     if (q > kG2Zero) {
       if (vh) vh[i] = make_double2(r.x * fpe2 / q, r.y * fpe2 / q);
       acc += (r.x * r.x + r.y * r.y) * fpe2 / q;
@@ -171,13 +182,15 @@ __global__ void k_scale_real(double* __restrict__ r, double s, long n) {
   if (i < n) r[i] *= s;
 }
 
-// V_eff(G) = V_loc(G) + V_H(G) + V_xc(G) (energy.rs:293-301)
-__global__ void k_veff_g(const double2* __restrict__ vloc, const double2* __restrict__ vh,
-                         const double2* __restrict__ vxc_g, double2* __restrict__ out, long n) {
+// V_eff(G) = V_loc(G) + V_H(G) + V_xc(G) (energy.rs:293-301), V_xc(G) = scale * vxc, in place over vxc and into copy
+__global__ void k_veff_g(const double2* __restrict__ vloc, const double2* __restrict__ vh, double2* __restrict__ vxc,
+                         double scale, double2* __restrict__ copy, long n) {
   const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) {
-    const double2 a = vloc[i], b = vh[i], c = vxc_g[i];
-    out[i] = make_double2(a.x + b.x + c.x, a.y + b.y + c.y);
+    const double2 a = vloc[i], b = vh[i], c = vxc[i];
+    const double2 v = make_double2(a.x + b.x + c.x * scale, a.y + b.y + c.y * scale);
+    vxc[i] = v;
+    copy[i] = v;
   }
 }
 
@@ -592,19 +605,17 @@ static Status reduce_host(Handle& h, const double* a, const double* b, long n, i
   return kOk;
 }
 
-static Status final_sum_host(Handle& h, int nparts, double& out, int slot = 0) {
-  ScfState* st = h.scf;
-  k_final_sum<<<1, 256, 0, h.stream>>>(st->partials + (long)slot * kRedBlocks, nparts, st->scal + slot); count_launch();
-  PW_CUDA_TRY(cudaMemcpyAsync(&out, st->scal + slot, sizeof(double), cudaMemcpyDeviceToHost, h.stream));
-  PW_CUDA_TRY(cudaStreamSynchronize(h.stream));
-  return kOk;
+// FFT(rho) into st->cg, not normalised
+static Status density_transform(Handle& h, const double* rho) {
+  const long N = h.g.N;
+  k_real_to_cplx<<<blocks_for(N), 256, 0, h.stream>>>(rho, h.scf->cg, N); count_launch();
+  return fft3d_full(h, h.scf->cg, -1, h.stream);
 }
 
 // rho(G) = FFT(rho)/N into st->cg
 static Status density_to_g(Handle& h, const double* rho) {
   const long N = h.g.N;
-  k_real_to_cplx<<<blocks_for(N), 256, 0, h.stream>>>(rho, h.scf->cg, N); count_launch();
-  Status s = fft3d_full(h, h.scf->cg, -1, h.stream);
+  Status s = density_transform(h, rho);
   if (s != kOk) return s;
   k_scale_cplx<<<blocks_for(N), 256, 0, h.stream>>>(h.scf->cg, 1.0 / (double)N, N); count_launch();
   return kOk;
@@ -614,40 +625,45 @@ struct PotEnergies {
   double e_hartree = 0, e_xc = 0, e_vxc = 0;
 };
 
-// Potentials from rho (device): V_eff(G) into st->cg2 (and V_eff(r) into the
-// handle's H|psi> arrays when set_hpsi), exc/vxc on the grid, energies.
+// E_H, E_xc and int rho v_xc from the three sums left in st->scal: the one
+// wait of a potential build, after all its kernels are launched.
+static Status read_energies(Handle& h, PotEnergies& e) {
+  PW_CUDA_TRY(cudaGetLastError());
+  double sum[3];
+  PW_CUDA_TRY(cudaMemcpyAsync(sum, h.scf->scal, sizeof(sum), cudaMemcpyDeviceToHost, h.stream));
+  PW_CUDA_TRY(cudaStreamSynchronize(h.stream));
+  const double dv = h.omega / (double)h.g.N;
+  e.e_hartree = sum[0] * 0.5 * h.omega;
+  e.e_xc = sum[1] * dv;
+  e.e_vxc = sum[2] * dv;
+  return kOk;
+}
+
+// Potentials from rho (device): exc/vxc on the grid and the energies; with
+// set_hpsi V_eff(G) into st->cg2 and V_eff(r) into the handle's H|psi> arrays.
 static Status potentials(Handle& h, const double* rho, bool set_hpsi, PotEnergies& e) {
   ScfState* st = h.scf;
   const long N = h.g.N;
   const cudaStream_t s = h.stream;
-  Status r = density_to_g(h, rho);
+  Status r = density_transform(h, rho);
   if (r != kOk) return r;
   const double fpe2 = 4.0 * kPi * kE2;
   const unsigned nbk = (unsigned)std::min<long>(kRedBlocks, blocks_for(N));
-  k_hartree<<<nbk, 256, 0, s>>>(st->cg, h.g_squared, N, st->vh, fpe2, st->partials); count_launch();
-  double sh = 0.0;
-  if ((r = final_sum_host(h, (int)nbk, sh)) != kOk) return r;
-  e.e_hartree = sh * 0.5 * h.omega;
-  k_lda<<<nbk, 256, 0, s>>>(rho, h.rho_core_r, N, st->exc, st->vxc, st->partials, st->partials + kRedBlocks); count_launch();
-  double sx = 0.0, sv = 0.0;
-  if ((r = final_sum_host(h, (int)nbk, sx, 0)) != kOk) return r;
-  if ((r = final_sum_host(h, (int)nbk, sv, 1)) != kOk) return r;
-  const double dv = h.omega / (double)N;
-  e.e_xc = sx * dv;
-  e.e_vxc = sv * dv;
-  // V_xc(G) = FFT(vxc)/N, V_eff(G) = V_loc + V_H + V_xc
-  k_real_to_cplx<<<blocks_for(N), 256, 0, s>>>(st->vxc, st->cg2, N); count_launch();
-  if ((r = fft3d_full(h, st->cg2, -1, s)) != kOk) return r;
-  k_scale_cplx<<<blocks_for(N), 256, 0, s>>>(st->cg2, 1.0 / (double)N, N); count_launch();
-  k_veff_g<<<blocks_for(N), 256, 0, s>>>(h.v_local_g, st->vh, st->cg2, st->cg2, N); count_launch();
+  const double inv = 1.0 / (double)N;
+  k_hartree<<<nbk, 256, 0, s>>>(st->cg, h.g_squared, inv, N, st->vh, fpe2, st->partials); count_launch();
+  k_lda<<<nbk, 256, 0, s>>>(rho, h.rho_core_r, N, st->exc, st->vxc, st->partials + kRedBlocks,
+                            st->partials + 2 * kRedBlocks); count_launch();
+  k_final_sums<<<3, 256, 0, s>>>(st->partials, (int)nbk, st->scal); count_launch();
   if (set_hpsi) {
-    PW_CUDA_TRY(cudaMemcpyAsync(h.tmp_grid, st->cg2, N * sizeof(double2), cudaMemcpyDeviceToDevice, s));
+    // V_xc(G) = FFT(vxc)/N, V_eff(G) = V_loc + V_H + V_xc
+    k_real_to_cplx<<<blocks_for(N), 256, 0, s>>>(st->vxc, st->cg2, N); count_launch();
+    if ((r = fft3d_full(h, st->cg2, -1, s)) != kOk) return r;
+    k_veff_g<<<blocks_for(N), 256, 0, s>>>(h.v_local_g, st->vh, st->cg2, inv, h.tmp_grid, N); count_launch();
     if ((r = fft3d_full(h, h.tmp_grid, +1, s)) != kOk) return r;
     k_real_part_both<<<blocks_for(N), 256, 0, s>>>(h.tmp_grid, h.veff_r[0], h.veff_r32[0], N); count_launch();
     if ((r = veff_zmajor(h, 0, s)) != kOk) return r;
   }
-  PW_CUDA_TRY(cudaGetLastError());
-  return kOk;
+  return read_energies(h, e);
 }
 
 // E_local = int rho V_loc dV over the given density channels, V_loc(r) the
@@ -1094,35 +1110,25 @@ static Status potentials_spin(Handle& h, const double* up, const double* dn, boo
   const long N = h.g.N;
   const cudaStream_t s = h.stream;
   k_axpy_to<<<blocks_for(N), 256, 0, s>>>(up, dn, 1.0, st->rtmp, N); count_launch();
-  Status r = density_to_g(h, st->rtmp);
+  Status r = density_transform(h, st->rtmp);
   if (r != kOk) return r;
   const double fpe2 = 4.0 * kPi * kE2;
   const unsigned nbk = (unsigned)std::min<long>(kRedBlocks, blocks_for(N));
-  k_hartree<<<nbk, 256, 0, s>>>(st->cg, h.g_squared, N, st->vh, fpe2, st->partials); count_launch();
-  double sh = 0.0;
-  if ((r = final_sum_host(h, (int)nbk, sh)) != kOk) return r;
-  e.e_hartree = sh * 0.5 * h.omega;
-  k_lsda<<<nbk, 256, 0, s>>>(up, dn, h.rho_core_r, N, st->vxc, st->vxc_dn, st->partials, st->partials + kRedBlocks);
+  const double inv = 1.0 / (double)N;
+  k_hartree<<<nbk, 256, 0, s>>>(st->cg, h.g_squared, inv, N, st->vh, fpe2, st->partials); count_launch();
+  k_lsda<<<nbk, 256, 0, s>>>(up, dn, h.rho_core_r, N, st->vxc, st->vxc_dn, st->partials + kRedBlocks,
+                             st->partials + 2 * kRedBlocks);
   count_launch();
-  double sx = 0.0, sv = 0.0;
-  if ((r = final_sum_host(h, (int)nbk, sx, 0)) != kOk) return r;
-  if ((r = final_sum_host(h, (int)nbk, sv, 1)) != kOk) return r;
-  const double dv = h.omega / (double)N;
-  e.e_xc = sx * dv;
-  e.e_vxc = sv * dv;
-  if (!set_hpsi) return kOk;
-  for (int sp = 0; sp < 2; ++sp) {
+  k_final_sums<<<3, 256, 0, s>>>(st->partials, (int)nbk, st->scal); count_launch();
+  for (int sp = 0; sp < 2 && set_hpsi; ++sp) {
     k_real_to_cplx<<<blocks_for(N), 256, 0, s>>>(sp == 0 ? st->vxc : st->vxc_dn, st->cg2, N); count_launch();
     if ((r = fft3d_full(h, st->cg2, -1, s)) != kOk) return r;
-    k_scale_cplx<<<blocks_for(N), 256, 0, s>>>(st->cg2, 1.0 / (double)N, N); count_launch();
-    k_veff_g<<<blocks_for(N), 256, 0, s>>>(h.v_local_g, st->vh, st->cg2, st->cg2, N); count_launch();
-    PW_CUDA_TRY(cudaMemcpyAsync(h.tmp_grid, st->cg2, N * sizeof(double2), cudaMemcpyDeviceToDevice, s));
+    k_veff_g<<<blocks_for(N), 256, 0, s>>>(h.v_local_g, st->vh, st->cg2, inv, h.tmp_grid, N); count_launch();
     if ((r = fft3d_full(h, h.tmp_grid, +1, s)) != kOk) return r;
     k_real_part_both<<<blocks_for(N), 256, 0, s>>>(h.tmp_grid, h.veff_r[sp], h.veff_r32[sp], N); count_launch();
     if ((r = veff_zmajor(h, sp, s)) != kOk) return r;
   }
-  PW_CUDA_TRY(cudaGetLastError());
-  return kOk;
+  return read_energies(h, e);
 }
 
 // Whole SCF loop: run_scf_unpolarized (driver.rs:353-735) for nspin = 1,
