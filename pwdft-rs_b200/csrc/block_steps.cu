@@ -78,9 +78,9 @@ __host__ __device__ constexpr int pad_ld(int rows) { return (rows + 15) / 16 * 1
 
 // Z (p x q, ld ldz in shared memory) = sum over the local rows of conj(A(i, a)) B(i, b).  Warps share the row
 // tiles of Z (8 x up to 32 entries each) and, when those are fewer than the warps, slices of the rows, added in
-// slice order.  la / lb return an entry, zero outside.
+// slice order.  la / lb return an entry, zero outside.  accumulate: added to Z.
 template <typename T, typename LA, typename LB>
-__device__ void local_gram(int rows, int p, int q, LA la, LB lb, T* Z, int ldz) {
+__device__ void local_gram(int rows, int p, int q, LA la, LB lb, T* Z, int ldz, bool accumulate = false) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kr = lane & 3, kc = lane >> 2;
   const int tp = (p + 7) >> 3, tg = (q + 31) >> 5;
@@ -116,12 +116,61 @@ __device__ void local_gram(int rows, int p, int q, LA la, LB lb, T* Z, int ldz) 
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
             const int c = q0 + 8 * t + 2 * kr + h;
-            if (r < p && c < q) Z[r + c * ldz] = s == 0 ? acc[t].get(h) : add(Z[r + c * ldz], acc[t].get(h));
+            if (r < p && c < q)
+              Z[r + c * ldz] = s == 0 && !accumulate ? acc[t].get(h) : add(Z[r + c * ldz], acc[t].get(h));
           }
       }
       __syncthreads();
     }
   }
+}
+
+// Columns c < ncols of `rows` rows, src(c) -> first row of the column, copied to S (row stride lds) with asynchronous
+// copies: whole rows of a column at a time, where the products' own operand reads would touch eight 32-byte sectors
+// an instruction, again for every tile.
+template <typename T, typename F> __device__ __forceinline__ void stage_cols(T* S, int lds, int rows, int ncols, F src) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int c = warp; c < ncols; c += kW) {
+    const T* g = src(c);
+    for (int i = lane; i < rows; i += 32) cp_async_zfill<sizeof(T)>(S + i + c * lds, g + i, true);
+  }
+  cp_async_commit();
+}
+__device__ __forceinline__ void stage_wait() {
+  cp_async_wait<0>();
+  __syncthreads();
+}
+
+// local_gram of the columns ca(a), a < p, and cb(b), b < q, staged through buf (cap entries, at least min_stage, or 0:
+// read in place) in chunks of rows.  Returns the row stride when one chunk held all rows (the columns are then still
+// in buf, A's first), else 0.
+template <typename T, typename FA, typename FB>
+__device__ int staged_gram(int rows, int p, int q, FA ca, FB cb, T* Z, int ldz, T* buf, int cap) {
+  if (cap == 0) {
+    local_gram<T>(
+        rows, p, q, [&](int i, int c) { return c < p ? ca(c)[i] : zero<T>(); },
+        [&](int i, int c) { return c < q ? cb(c)[i] : zero<T>(); }, Z, ldz);
+    return 0;
+  }
+  int chunk = max(rows, 4), lds = pad_ld(chunk);
+  while (chunk > 4 && (long)lds * (p + q) > cap) {
+    chunk = max(4, ((chunk + 1) / 2 + 3) & ~3);
+    lds = pad_ld(chunk);
+  }
+  const bool whole = chunk >= rows;
+  int r = 0;
+  do {
+    const int nr = min(chunk, rows - r);
+    stage_cols<T>(buf, lds, nr, p, [&](int c) { return ca(c) + r; });
+    stage_cols<T>(buf + (size_t)lds * p, lds, nr, q, [&](int c) { return cb(c) + r; });
+    stage_wait();
+    const T *A = buf, *B = buf + (size_t)lds * p;
+    local_gram<T>(
+        nr, p, q, [&](int i, int c) { return c < p ? A[i + c * lds] : zero<T>(); },
+        [&](int i, int c) { return c < q ? B[i + c * lds] : zero<T>(); }, Z, ldz, r > 0);
+    r += chunk;
+  } while (r < rows);
+  return whole ? lds : 0;
 }
 
 // Entry e of the sum over the CTAs' partials (C x n in xch), in rank order.
@@ -267,7 +316,7 @@ constexpr double kSkipTol = 1e-12;  // a Cholesky-QR pass is skipped when its bl
 template <typename T, int NQ>
 __global__ void __launch_bounds__(kT, 1)
     k_block_w(const T* __restrict__ X, int nd, const T* Tb, const int* __restrict__ idx, int na, T* W, long n,
-              int rpc, int ldy, int ldz, T* __restrict__ xch, long xch_len, int* __restrict__ status) {
+              int rpc, int ldy, int ldz, int staged, T* __restrict__ xch, long xch_len, int* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[kW];
   __shared__ double scol[kMaxBlock];
@@ -276,17 +325,18 @@ __global__ void __launch_bounds__(kT, 1)
   T* Y = reinterpret_cast<T*>(smem);       // rpc x na
   T* Z = Y + (size_t)ldy * na;             // max(nd, na) x na
   T* Ri = Z + (size_t)ldz * na;            // na x na
+  T* S = Ri + (size_t)ldz * na;            // rpc x nd: X, when staged
   const long r0 = (long)rank * rpc;
   const int rows = (int)max(0L, min((long)rpc, n - r0));
-  for (int e = threadIdx.x; e < rows * na; e += kT) {
-    const int i = e % rows, c = e / rows;
-    Y[i + c * ldy] = Tb[r0 + i + (long)(idx ? idx[c] : c) * n];
-  }
-  __syncthreads();
+  stage_cols<T>(Y, ldy, rows, na, [&](int c) { return Tb + r0 + (long)(idx ? idx[c] : c) * n; });
+  if (staged) stage_cols<T>(S, ldy, rows, nd, [&](int c) { return X + r0 + (long)c * n; });
+  stage_wait();
   int par = 0;
   auto ly = [&](int i, int c) { return c < na ? Y[i + c * ldy] : zero<T>(); };
   for (int pass = 0; pass < 2 && nd > 0; ++pass) {
-    auto lx = [&](int i, int c) { return c < nd ? X[r0 + i + (long)c * n] : zero<T>(); };
+    auto lx = [&](int i, int c) {
+      return c >= nd ? zero<T>() : staged ? S[i + c * ldy] : X[r0 + i + (long)c * n];
+    };
     local_gram<T>(rows, nd, na, lx, ly, Z, ldz);
     cluster_sum<T>(cl, Z, ldz, nd, na, xch + par * xch_len);
     par ^= 1;
@@ -348,10 +398,8 @@ __global__ void __launch_bounds__(kT, 1)
     local_update<NQ, 0, T>(rows, na, na, ly, Ri, ldz, ly, [&](int i, int c, T v) { Y[i + c * ldy] = v; });
     __syncthreads();
   }
-  for (int e = threadIdx.x; e < rows * na; e += kT) {
-    const int i = e % rows, c = e / rows;
-    W[r0 + i + (long)c * n] = Y[i + c * ldy];
-  }
+  for (int c = threadIdx.x >> 5; c < na; c += kW)
+    for (int i = threadIdx.x & 31; i < rows; i += 32) W[r0 + i + (long)c * n] = Y[i + c * ldy];
   if (rank == 0 && threadIdx.x == 0) status[0] = ok ? 0 : 1;
 }
 
@@ -363,7 +411,7 @@ __global__ void __launch_bounds__(kT, 1)
     k_block_p(const T* __restrict__ X, const T* __restrict__ HX, int nd, const T* __restrict__ W,
               const T* __restrict__ HW, int na, const T* __restrict__ Pn, const T* __restrict__ HPn,
               const int* __restrict__ idx, int np, T* __restrict__ P, T* __restrict__ HP, long n, int rpc, int ldy,
-              int ldz, double p_drop, T* __restrict__ xch, long xch_len, int* __restrict__ status) {
+              int ldz, int staged, double p_drop, T* __restrict__ xch, long xch_len, int* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[kW];
   __shared__ double scol[kMaxBlock], nu0[kMaxBlock];
@@ -374,13 +422,21 @@ __global__ void __launch_bounds__(kT, 1)
   T* Y = reinterpret_cast<T*>(smem);
   T* Z = Y + (size_t)ldy * np;
   T* Ri = Z + (size_t)ldz * np;
+  T* S = Ri + (size_t)ldz * np;                  // rpc x max(nd, na), staged >= 1: X, HX, W, HW in turn
+  T* HY = S + (size_t)ldy * max(nd, na);         // rpc x np, staged == 2: HP
   const long r0 = (long)rank * rpc;
   const int rows = (int)max(0L, min((long)rpc, n - r0));
-  for (int e = threadIdx.x; e < rows * np; e += kT) {
-    const int i = e % rows, c = e / rows;
-    Y[i + c * ldy] = Pn[r0 + i + (long)idx[c] * n];
-  }
-  __syncthreads();
+  stage_cols<T>(Y, ldy, rows, np, [&](int c) { return Pn + r0 + (long)idx[c] * n; });
+  if (staged > 1) stage_cols<T>(HY, ldy, rows, np, [&](int c) { return HPn + r0 + (long)idx[c] * n; });
+  auto stage = [&](const T* M, int cols) {
+    if (!staged) return;
+    __syncthreads();  // the readers of the last operand
+    stage_cols<T>(S, ldy, rows, cols, [&](int c) { return M + r0 + (long)c * n; });
+    stage_wait();
+  };
+  auto operand = [&](const T* M, int i, int c) { return staged ? S[i + c * ldy] : M[r0 + i + (long)c * n]; };
+  stage(X, nd);
+  if (!staged) stage_wait();
   // squared column norms of this CTA's rows, summed with the first projection (row nd of Z)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int c = warp; c < np; c += kW) {
@@ -393,8 +449,13 @@ __global__ void __launch_bounds__(kT, 1)
   int par = 0;
   auto ly = [&](int i, int c) { return c < np ? Y[i + c * ldy] : zero<T>(); };
   auto sy = [&](int i, int c, T v) { Y[i + c * ldy] = v; };
+  auto lhp = [&](int i, int c) { return staged > 1 ? HY[i + c * ldy] : HP[r0 + i + (long)c * n]; };
+  auto shp = [&](int i, int c, T v) {
+    if (staged > 1) HY[i + c * ldy] = v;
+    else HP[r0 + i + (long)c * n] = v;
+  };
   {
-    auto lx = [&](int i, int c) { return c < nd ? X[r0 + i + (long)c * n] : zero<T>(); };
+    auto lx = [&](int i, int c) { return c < nd ? operand(X, i, c) : zero<T>(); };
     local_gram<T>(rows, nd, np, lx, ly, Z, ldz);
     if (threadIdx.x < np) Z[nd + threadIdx.x * ldz] = mk<T>(nu0[threadIdx.x], 0.0);
     __syncthreads();
@@ -402,22 +463,22 @@ __global__ void __launch_bounds__(kT, 1)
     par ^= 1;
     if (threadIdx.x < np) nu0[threadIdx.x] = re(Z[nd + threadIdx.x * ldz]);
     local_update<NQ, -1, T>(rows, nd, np, lx, Z, ldz, ly, sy);
+    stage(HX, nd);
     local_update<NQ, -1, T>(
-        rows, nd, np, [&](int i, int c) { return HX[r0 + i + (long)c * n]; }, Z, ldz,
-        [&](int i, int c) { return HPn[r0 + i + (long)idx[c] * n]; },
-        [&](int i, int c, T v) { HP[r0 + i + (long)c * n] = v; });
+        rows, nd, np, [&](int i, int c) { return operand(HX, i, c); }, Z, ldz,
+        [&](int i, int c) { return staged > 1 ? HY[i + c * ldy] : HPn[r0 + i + (long)idx[c] * n]; }, shp);
     __syncthreads();
   }
-  auto lhp = [&](int i, int c) { return HP[r0 + i + (long)c * n]; };
-  auto shp = [&](int i, int c, T v) { HP[r0 + i + (long)c * n] = v; };
   {
-    auto lw = [&](int i, int c) { return c < na ? W[r0 + i + (long)c * n] : zero<T>(); };
+    stage(W, na);
+    auto lw = [&](int i, int c) { return c < na ? operand(W, i, c) : zero<T>(); };
     local_gram<T>(rows, na, np, lw, ly, Z, ldz);
     cluster_sum<T>(cl, Z, ldz, na, np, xch + par * xch_len);
     par ^= 1;
     local_update<NQ, -1, T>(rows, na, np, lw, Z, ldz, ly, sy);
+    stage(HW, na);
     local_update<NQ, -1, T>(
-        rows, na, np, [&](int i, int c) { return HW[r0 + i + (long)c * n]; }, Z, ldz, lhp, shp);
+        rows, na, np, [&](int i, int c) { return operand(HW, i, c); }, Z, ldz, lhp, shp);
     __syncthreads();
   }
   int nk = np;
@@ -473,13 +534,14 @@ __global__ void __launch_bounds__(kT, 1)
     local_update<NQ, 0, T>(
         rows, nk, nk, [&](int i, int c) { return Y[i + keep[c] * ldy]; }, Ri, ldz, ly, sy);
     local_update<NQ, 0, T>(
-        rows, nk, nk, [&](int i, int c) { return HP[r0 + i + (long)keep[c] * n]; }, Ri, ldz, lhp, shp);
+        rows, nk, nk, [&](int i, int c) { return lhp(i, keep[c]); }, Ri, ldz, lhp, shp);
     __syncthreads();
   }
-  for (int e = threadIdx.x; e < rows * nk; e += kT) {
-    const int i = e % rows, c = e / rows;
-    P[r0 + i + (long)c * n] = Y[i + c * ldy];
-  }
+  for (int c = warp; c < nk; c += kW)
+    for (int i = lane; i < rows; i += 32) {
+      P[r0 + i + (long)c * n] = Y[i + c * ldy];
+      if (staged > 1) HP[r0 + i + (long)c * n] = HY[i + c * ldy];
+    }
   if (rank == 0 && threadIdx.x == 0) status[1] = nk;
 }
 
@@ -489,22 +551,18 @@ template <typename T>
 __global__ void __launch_bounds__(kT, 1)
     k_block_rr(const T* __restrict__ B, const T* __restrict__ HB, int q, const T* __restrict__ HX,
                const int* __restrict__ cols, int nx, const double* __restrict__ lam, const T* __restrict__ XX, long n,
-               int rpc, int ldz, T* __restrict__ xch, T* __restrict__ Hs) {
+               int rpc, int ldz, int cap, T* __restrict__ xch, T* __restrict__ Hs) {
   extern __shared__ __align__(16) unsigned char smem[];
-  T* Z = reinterpret_cast<T*>(smem);  // q x (nx + q)
+  T* Z = reinterpret_cast<T*>(smem);  // q x (nx + q), then the staging buffer
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   const long r0 = (long)rank * rpc;
   const int rows = (int)max(0L, min((long)rpc, n - r0));
   const int m = nx + q, nz = q * m;
-  auto lb = [&](int i, int c) { return c < q ? B[r0 + i + (long)c * n] : zero<T>(); };
-  local_gram<T>(
-      rows, q, m, lb,
-      [&](int i, int c) {
-        if (c >= m) return zero<T>();
-        return c < nx ? HX[r0 + i + (long)(cols ? cols[c] : c) * n] : HB[r0 + i + (long)(c - nx) * n];
-      },
-      Z, ldz);
+  staged_gram<T>(
+      rows, q, m, [&](int c) { return B + r0 + (long)c * n; },
+      [&](int c) { return c < nx ? HX + r0 + (long)(cols ? cols[c] : c) * n : HB + r0 + (long)(c - nx) * n; }, Z, ldz,
+      Z + (size_t)ldz * m, cap);
   for (int e = threadIdx.x; e < nz; e += kT) xch[(size_t)rank * nz + e] = Z[e % q + (e / q) * ldz];
   cl.sync();
   // entry (r, c) of B^H [HX | HB], summed over the CTAs
@@ -594,7 +652,7 @@ __global__ void __launch_bounds__(kUpdThreads)
 template <typename T, int NQ>
 __global__ void __launch_bounds__(kT, 1)
     k_block_nl(const T* __restrict__ B, int n_ch, const T* __restrict__ psi, long ldpsi, int nb, T* __restrict__ hpsi,
-               long ldh, long n, int rpc, int ldz, T* __restrict__ xch, const int* __restrict__ ch_atom,
+               long ldh, long n, int rpc, int ldz, int cap, T* __restrict__ xch, const int* __restrict__ ch_atom,
                const int* __restrict__ atom_ch_start, const int* __restrict__ d_off,
                const double* __restrict__ d_vals) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -603,9 +661,11 @@ __global__ void __launch_bounds__(kT, 1)
   cg::cluster_group cl = cg::this_cluster();
   const long r0 = (long)cl.block_rank() * rpc;
   const int rows = (int)max(0L, min((long)rpc, n - r0));
-  auto lb = [&](int i, int c) { return c < n_ch ? B[r0 + i + (long)c * n] : zero<T>(); };
-  local_gram<T>(
-      rows, n_ch, nb, lb, [&](int i, int c) { return c < nb ? psi[r0 + i + (long)c * ldpsi] : zero<T>(); }, Z, ldz);
+  T* buf = Q + (size_t)ldz * nb;
+  const int lds = staged_gram<T>(
+      rows, n_ch, nb, [&](int c) { return B + r0 + (long)c * n; },
+      [&](int c) { return psi + r0 + (long)c * ldpsi; }, Z, ldz, buf, cap);
+  auto lb = [&](int i, int c) { return lds ? buf[i + c * lds] : B[r0 + i + (long)c * n]; };
   cluster_sum<T>(cl, Z, ldz, n_ch, nb, xch);
   for (int e = threadIdx.x; e < n_ch * nb; e += kT) {
     const int c = e % n_ch, b = e / n_ch, a = ch_atom[c], s = atom_ch_start[a], nc = atom_ch_start[a + 1] - s;
@@ -631,6 +691,14 @@ void split_rows(long n, int& C, int& rpc) {
 
 template <typename T> size_t step_smem(int rpc, int cols, int zrows) {
   return ((size_t)pad_ld(rpc) + 2 * (size_t)pad_ld(zrows)) * cols * sizeof(T);
+}
+
+// Bytes of a staging buffer for `cols` columns of up to rpc rows: all rows, or what is left, or 0 where that is less
+// than the four rows a chunk needs.
+template <typename T> size_t stage_bytes(int rpc, int cols, size_t left) {
+  const size_t all = (size_t)pad_ld(std::max(rpc, 4)) * cols * sizeof(T);
+  const size_t least = (size_t)pad_ld(4) * cols * sizeof(T);
+  return all <= left ? all : left >= least ? left / sizeof(T) * sizeof(T) : 0;
 }
 
 template <typename K> Status opt_in(K kern, bool cluster) {
@@ -715,10 +783,14 @@ Status block_w(const T* X, int nd, const T* Tb, const int* idx, int na, T* W, lo
   int C, rpc;
   split_rows(n, C, rpc);
   const int zr = std::max(nd, na), ldy = pad_ld(rpc), ldz = pad_ld(zr);
-  const size_t sm = step_smem<T>(rpc, na, zr);
+  size_t sm = step_smem<T>(rpc, na, zr);
+  const size_t more = (size_t)ldy * nd * sizeof(T);
+  const int staged = nd > 0 && sm + more <= kSmemMax;
+  if (staged) sm += more;
   const long xl = (long)(kMaxC + 1) * std::max(nd, na) * na;
-  if (na <= 32) return launch(k_block_w<T, 4>, C, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, xch, xl, status);
-  return launch(k_block_w<T, 8>, C, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, xch, xl, status);
+  if (na <= 32)
+    return launch(k_block_w<T, 4>, C, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, staged, xch, xl, status);
+  return launch(k_block_w<T, 8>, C, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, staged, xch, xl, status);
 }
 
 template <typename T>
@@ -727,13 +799,16 @@ Status block_p(const T* X, const T* HX, int nd, const T* W, const T* HW, int na,
   int C, rpc;
   split_rows(n, C, rpc);
   const int zr = std::max(nd + 1, std::max(na, np)), ldy = pad_ld(rpc), ldz = pad_ld(zr);
-  const size_t sm = step_smem<T>(rpc, np, zr);
+  size_t sm = step_smem<T>(rpc, np, zr);
+  const size_t op = (size_t)ldy * std::max(nd, na) * sizeof(T), hp = (size_t)ldy * np * sizeof(T);
+  const int staged = sm + op + hp <= kSmemMax ? 2 : sm + op <= kSmemMax ? 1 : 0;
+  sm += staged == 2 ? op + hp : staged == 1 ? op : 0;
   const long xl = (long)(kMaxC + 1) * (nd + 1) * np;
   if (np <= 32)
-    return launch(k_block_p<T, 4>, C, sm, s, X, HX, nd, W, HW, na, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, p_drop,
-                  xch, xl, status);
-  return launch(k_block_p<T, 8>, C, sm, s, X, HX, nd, W, HW, na, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, p_drop,
-                xch, xl, status);
+    return launch(k_block_p<T, 4>, C, sm, s, X, HX, nd, W, HW, na, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, staged,
+                  p_drop, xch, xl, status);
+  return launch(k_block_p<T, 8>, C, sm, s, X, HX, nd, W, HW, na, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, staged,
+                p_drop, xch, xl, status);
 }
 
 template <typename T>
@@ -742,7 +817,9 @@ Status block_rr(const T* B, const T* HB, int q, const T* HX, const int* cols, in
   int C, rpc;
   split_rows(n, C, rpc);
   const int ldz = pad_ld(q);
-  return launch(k_block_rr<T>, C, (size_t)ldz * (nx + q) * sizeof(T), s, B, HB, q, HX, cols, nx, lam, XX, n, rpc, ldz,
+  const size_t zb = (size_t)ldz * (nx + q) * sizeof(T);
+  const size_t buf = stage_bytes<T>(rpc, nx + 2 * q, kSmemMax - zb);
+  return launch(k_block_rr<T>, C, zb + buf, s, B, HB, q, HX, cols, nx, lam, XX, n, rpc, ldz, (int)(buf / sizeof(T)),
                 xch, Hs);
 }
 
@@ -784,8 +861,10 @@ Status nl_fused(Handle& h, const T* B, const T* psi, long ldpsi, int nb, T* hpsi
   int C, rpc;
   split_rows(h.n_pw, C, rpc);
   const int ldz = pad_ld(h.n_ch);
-  return launch(k_block_nl<T, 4>, C, (size_t)2 * ldz * nb * sizeof(T), s, B, h.n_ch, psi, ldpsi, nb, hpsi, ldh,
-                (long)h.n_pw, rpc, ldz, static_cast<T*>(h.nl_xch), (const int*)h.ch_atom,
+  const size_t zb = (size_t)2 * ldz * nb * sizeof(T);
+  const size_t buf = stage_bytes<T>(rpc, h.n_ch + nb, kSmemMax - zb);
+  return launch(k_block_nl<T, 4>, C, zb + buf, s, B, h.n_ch, psi, ldpsi, nb, hpsi, ldh, (long)h.n_pw, rpc, ldz,
+                (int)(buf / sizeof(T)), static_cast<T*>(h.nl_xch), (const int*)h.ch_atom,
                 (const int*)h.atom_ch_start, (const int*)h.d_off, (const double*)h.d_vals);
 }
 
