@@ -15,9 +15,10 @@
 //
 // Against the library-call steps, with the same subspace eigensolver (B200):
 // restart iteration of 8 Si atoms at Gamma (real, 22 columns, 2,945 rows)
-// 27.7 -> 17.2 ms, of 2 atoms over 6 k-points (complex, 10 columns, 411 rows)
-// 21.0 -> 9.5 ms, whole LSDA run of 8 C atoms (27 columns, 1,045 rows, 40
-// blocks on 8 lanes) 405 -> 264 ms.
+// 27.7 -> 14.5 ms, of 2 atoms over 6 k-points (complex, 10 columns, 411 rows)
+// 21.0 -> 8.7 ms, whole LSDA run of 8 C atoms (27 columns, 1,045 rows, 40
+// blocks on 8 lanes) 405 -> 238 ms.  One Cholesky barrier a column instead of
+// three, and one sum less for each of W and P, are 5 % of those.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -246,40 +247,44 @@ __device__ void local_update(int rows, int kdim, int q, LA la, const T* Z, int l
 }
 
 // Upper Cholesky factor of the q x q Hermitian G (upper triangle used) in place; false when a pivot is not
-// positive.  *rmin: smallest diagonal entry.  All threads; ends at a block barrier.
-template <typename T> __device__ bool block_cholesky(T* G, int ldg, int q, double* rmin) {
+// positive.  *rmin: smallest diagonal entry; rinv[c] (shared) = 1 / R_cc.  Rows stay unscaled until the end (the update
+// divides by the pivot), so a column costs one barrier.  All threads; ends at a block barrier.
+template <typename T> __device__ bool block_cholesky(T* G, int ldg, int q, double* rmin, double* rinv) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __syncthreads();
-  double mn = 1e300;
+  double dmin = 1e300;
   for (int c = 0; c < q; ++c) {
     const double d = re(G[c + c * ldg]);
     if (!(d > 0.0)) {  // the same value in every thread
       __syncthreads();
       return false;
     }
-    const double r = sqrt(d), ir = 1.0 / r;
-    mn = fmin(mn, r);
-    __syncthreads();
-    for (int j = c + threadIdx.x; j < q; j += kT) G[c + j * ldg] = j == c ? mk<T>(r, 0.0) : mul(G[c + j * ldg], ir);
-    __syncthreads();
-    const int rem = q - c - 1;
-    for (int e = threadIdx.x; e < rem * rem; e += kT) {
-      const int i = c + 1 + e % rem, j = c + 1 + e / rem;
-      if (i <= j) G[i + j * ldg] = sub(G[i + j * ldg], mul(cj(G[c + i * ldg]), G[c + j * ldg]));
+    dmin = fmin(dmin, d);
+    const double id = 1.0 / d;
+    for (int j = c + 1 + warp; j < q; j += kW) {
+      const T g = mul(G[c + j * ldg], id);
+      for (int i = c + 1 + lane; i <= j; i += 32) G[i + j * ldg] = sub(G[i + j * ldg], mul(cj(G[c + i * ldg]), g));
     }
     __syncthreads();
   }
-  *rmin = mn;
+  for (int c = warp; c < q; c += kW) {
+    const double d = re(G[c + c * ldg]), r = sqrt(d), ir = 1.0 / r;
+    __syncwarp();
+    for (int j = c + lane; j < q; j += 32) G[c + j * ldg] = j == c ? mk<T>(r, 0.0) : mul(G[c + j * ldg], ir);
+    if (lane == 0) rinv[c] = ir;
+  }
+  *rmin = sqrt(dmin);
+  __syncthreads();
   return true;
 }
 
 // Ri = R^-1 (q x q, zero below the diagonal), one warp per column: lane l keeps entries l and l + 32.
-template <typename T> __device__ void block_inverse(const T* R, int ldr, int q, T* Ri, int ldi) {
+template <typename T> __device__ void block_inverse(const T* R, int ldr, int q, const double* rinv, T* Ri, int ldi) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int c = warp; c < q; c += kW) {
     T z0 = mk<T>(lane == c ? 1.0 : 0.0, 0.0), z1 = mk<T>(lane + 32 == c ? 1.0 : 0.0, 0.0);
     for (int i = c; i >= 0; --i) {
-      const double id = 1.0 / re(R[i + i * ldr]);
-      const T zi = mul(i < 32 ? shfl(z0, i) : shfl(z1, i - 32), id);
+      const T zi = mul(i < 32 ? shfl(z0, i) : shfl(z1, i - 32), rinv[i]);
       if (lane < i) z0 = sub(z0, mul(R[lane + i * ldr], zi));
       if (lane + 32 < i) z1 = sub(z1, mul(R[lane + 32 + i * ldr], zi));
       if (lane == i) z0 = zi;
@@ -316,16 +321,16 @@ constexpr double kSkipTol = 1e-12;  // a Cholesky-QR pass is skipped when its bl
 template <typename T, int NQ>
 __global__ void __launch_bounds__(kT, 1)
     k_block_w(const T* __restrict__ X, int nd, const T* Tb, const int* __restrict__ idx, int na, T* W, long n,
-              int rpc, int ldy, int ldz, int staged, T* __restrict__ xch, long xch_len, int* __restrict__ status) {
+              int rpc, int ldy, int ldz, int ldi, int staged, T* __restrict__ xch, long xch_len, int* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[kW];
-  __shared__ double scol[kMaxBlock];
+  __shared__ double scol[kMaxBlock], rinv[kMaxBlock];
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
   T* Y = reinterpret_cast<T*>(smem);       // rpc x na
   T* Z = Y + (size_t)ldy * na;             // max(nd, na) x na
   T* Ri = Z + (size_t)ldz * na;            // na x na
-  T* S = Ri + (size_t)ldz * na;            // rpc x nd: X, when staged
+  T* S = Ri + (size_t)ldi * na;            // rpc x nd: X, when staged
   const long r0 = (long)rank * rpc;
   const int rows = (int)max(0L, min((long)rpc, n - r0));
   stage_cols<T>(Y, ldy, rows, na, [&](int c) { return Tb + r0 + (long)(idx ? idx[c] : c) * n; });
@@ -333,21 +338,40 @@ __global__ void __launch_bounds__(kT, 1)
   stage_wait();
   int par = 0;
   auto ly = [&](int i, int c) { return c < na ? Y[i + c * ldy] : zero<T>(); };
-  for (int pass = 0; pass < 2 && nd > 0; ++pass) {
-    auto lx = [&](int i, int c) {
-      return c >= nd ? zero<T>() : staged ? S[i + c * ldy] : X[r0 + i + (long)c * n];
-    };
+  auto lx = [&](int i, int c) {
+    return c >= nd ? zero<T>() : staged ? S[i + c * ldy] : X[r0 + i + (long)c * n];
+  };
+  auto sy = [&](int i, int c, T v) { Y[i + c * ldy] = v; };
+  if (nd > 0) {
     local_gram<T>(rows, nd, na, lx, ly, Z, ldz);
     cluster_sum<T>(cl, Z, ldz, nd, na, xch + par * xch_len);
     par ^= 1;
-    local_update<NQ, -1, T>(rows, nd, na, lx, Z, ldz, ly, [&](int i, int c, T v) { Y[i + c * ldy] = v; });
+    local_update<NQ, -1, T>(rows, nd, na, lx, Z, ldz, ly, sy);
+    __syncthreads();
+    // [X | Y]^H Y: the second projection and the Gram matrix in one sum.  Y - X Z has the Gram matrix G - Z^H Z,
+    // with Z at rounding level after the first projection, so nothing cancels.
+    local_gram<T>(
+        rows, nd + na, na, [&](int i, int c) { return c < nd ? lx(i, c) : ly(i, c - nd); }, ly, Z, ldz);
+    cluster_sum<T>(cl, Z, ldz, nd + na, na, xch + par * xch_len);
+    par ^= 1;
+    local_update<NQ, -1, T>(rows, nd, na, lx, Z, ldz, ly, sy);
+    for (int e = threadIdx.x; e < na * na; e += kT) {
+      const int r = e % na, c = e / na;
+      T g = Z[nd + r + c * ldz];
+      for (int k = 0; k < nd; ++k) g = sub(g, mul(cj(Z[k + r * ldz]), Z[k + c * ldz]));
+      Ri[r + c * ldi] = g;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < na * na; e += kT) Z[e % na + (e / na) * ldz] = Ri[e % na + (e / na) * ldi];
     __syncthreads();
   }
   bool ok = true;
   for (int pass = 0; pass < 2; ++pass) {
-    local_gram<T>(rows, na, na, ly, ly, Z, ldz);
-    cluster_sum<T>(cl, Z, ldz, na, na, xch + par * xch_len);
-    par ^= 1;
+    if (pass > 0 || nd == 0) {
+      local_gram<T>(rows, na, na, ly, ly, Z, ldz);
+      cluster_sum<T>(cl, Z, ldz, na, na, xch + par * xch_len);
+      par ^= 1;
+    }
     if (pass == 0) {
       // the Gram matrix of the unit columns
       if (threadIdx.x < na) {
@@ -375,27 +399,27 @@ __global__ void __launch_bounds__(kT, 1)
     }
     double rmin;
     // keep a copy in Ri's place for the shifted retry
-    for (int e = threadIdx.x; e < na * na; e += kT) Ri[e % na + (e / na) * ldz] = Z[e % na + (e / na) * ldz];
+    for (int e = threadIdx.x; e < na * na; e += kT) Ri[e % na + (e / na) * ldi] = Z[e % na + (e / na) * ldz];
     __syncthreads();
-    ok = block_cholesky<T>(Z, ldz, na, &rmin);
+    ok = block_cholesky<T>(Z, ldz, na, &rmin, rinv);
     if (!ok && pass == 0) {
       for (int e = threadIdx.x; e < na * na; e += kT) {
         const int r = e % na, c = e / na;
-        T g = Ri[r + c * ldz];
+        T g = Ri[r + c * ldi];
         if (r == c) g = add(g, mk<T>(1e-10 * na, 0.0));
         Z[r + c * ldz] = g;
       }
       __syncthreads();
-      ok = block_cholesky<T>(Z, ldz, na, &rmin);
+      ok = block_cholesky<T>(Z, ldz, na, &rmin, rinv);
     }
     if (!ok) break;
-    block_inverse<T>(Z, ldz, na, Ri, ldz);
+    block_inverse<T>(Z, ldz, na, rinv, Ri, ldi);
     for (int e = threadIdx.x; e < na * na; e += kT) {
       const int r = e % na, c = e / na;
-      Ri[r + c * ldz] = mul(Ri[r + c * ldz], scol[r]);
+      Ri[r + c * ldi] = mul(Ri[r + c * ldi], scol[r]);
     }
     __syncthreads();
-    local_update<NQ, 0, T>(rows, na, na, ly, Ri, ldz, ly, [&](int i, int c, T v) { Y[i + c * ldy] = v; });
+    local_update<NQ, 0, T>(rows, na, na, ly, Ri, ldi, ly, sy);
     __syncthreads();
   }
   for (int c = threadIdx.x >> 5; c < na; c += kW)
@@ -403,18 +427,19 @@ __global__ void __launch_bounds__(kT, 1)
   if (rank == 0 && threadIdx.x == 0) status[0] = ok ? 0 : 1;
 }
 
-// P, HP = the previous directions Pn(:, idx), HPn(:, idx) outside span(X, W), orthonormal: projections against X and W
-// (H with them), columns that keep less than p_drop of their norm dropped, two Cholesky-QR passes.  status[1] =
-// columns of P (0 when the block is nearly dependent).
+// P, HP = the previous directions Pn(:, idx), HPn(:, idx) outside span(X, W), orthonormal: projection against the
+// orthonormal columns [X | W], nx of them side by side in X and their H images in HX, columns that keep less than
+// p_drop of their norm dropped, two Cholesky-QR passes.  status[1] = columns of P (0 when the block is nearly
+// dependent).
 template <typename T, int NQ>
 __global__ void __launch_bounds__(kT, 1)
-    k_block_p(const T* __restrict__ X, const T* __restrict__ HX, int nd, const T* __restrict__ W,
-              const T* __restrict__ HW, int na, const T* __restrict__ Pn, const T* __restrict__ HPn,
-              const int* __restrict__ idx, int np, T* __restrict__ P, T* __restrict__ HP, long n, int rpc, int ldy,
-              int ldz, int staged, double p_drop, T* __restrict__ xch, long xch_len, int* __restrict__ status) {
+    k_block_p(const T* __restrict__ X, const T* __restrict__ HX, int nx, const T* __restrict__ Pn,
+              const T* __restrict__ HPn, const int* __restrict__ idx, int np, T* __restrict__ P,
+              T* __restrict__ HP, long n, int rpc, int ldy,
+              int ldz, int ldi, int staged, double p_drop, T* __restrict__ xch, long xch_len, int* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[kW];
-  __shared__ double scol[kMaxBlock], nu0[kMaxBlock];
+  __shared__ double scol[kMaxBlock], nu0[kMaxBlock], rinv[kMaxBlock];
   __shared__ int keep[kMaxBlock];
   __shared__ int nkeep_s;
   cg::cluster_group cl = cg::this_cluster();
@@ -422,22 +447,22 @@ __global__ void __launch_bounds__(kT, 1)
   T* Y = reinterpret_cast<T*>(smem);
   T* Z = Y + (size_t)ldy * np;
   T* Ri = Z + (size_t)ldz * np;
-  T* S = Ri + (size_t)ldz * np;                  // rpc x max(nd, na), staged >= 1: X, HX, W, HW in turn
-  T* HY = S + (size_t)ldy * max(nd, na);         // rpc x np, staged == 2: HP
+  T* S = Ri + (size_t)ldi * np;     // rpc x nx, staged >= 1: [X | W], then [HX | HW]
+  T* HY = S + (size_t)ldy * nx;     // rpc x np, staged == 2: HP
   const long r0 = (long)rank * rpc;
   const int rows = (int)max(0L, min((long)rpc, n - r0));
   stage_cols<T>(Y, ldy, rows, np, [&](int c) { return Pn + r0 + (long)idx[c] * n; });
   if (staged > 1) stage_cols<T>(HY, ldy, rows, np, [&](int c) { return HPn + r0 + (long)idx[c] * n; });
-  auto stage = [&](const T* M, int cols) {
+  auto stage = [&](const T* M) {
     if (!staged) return;
     __syncthreads();  // the readers of the last operand
-    stage_cols<T>(S, ldy, rows, cols, [&](int c) { return M + r0 + (long)c * n; });
+    stage_cols<T>(S, ldy, rows, nx, [&](int c) { return M + r0 + (long)c * n; });
     stage_wait();
   };
   auto operand = [&](const T* M, int i, int c) { return staged ? S[i + c * ldy] : M[r0 + i + (long)c * n]; };
-  stage(X, nd);
+  stage(X);
   if (!staged) stage_wait();
-  // squared column norms of this CTA's rows, summed with the first projection (row nd of Z)
+  // squared column norms of this CTA's rows, summed with the projection (row nx of Z)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int c = warp; c < np; c += kW) {
     double s = 0.0;
@@ -454,33 +479,19 @@ __global__ void __launch_bounds__(kT, 1)
     if (staged > 1) HY[i + c * ldy] = v;
     else HP[r0 + i + (long)c * n] = v;
   };
-  {
-    auto lx = [&](int i, int c) { return c < nd ? operand(X, i, c) : zero<T>(); };
-    local_gram<T>(rows, nd, np, lx, ly, Z, ldz);
-    if (threadIdx.x < np) Z[nd + threadIdx.x * ldz] = mk<T>(nu0[threadIdx.x], 0.0);
-    __syncthreads();
-    cluster_sum<T>(cl, Z, ldz, nd + 1, np, xch + par * xch_len);
-    par ^= 1;
-    if (threadIdx.x < np) nu0[threadIdx.x] = re(Z[nd + threadIdx.x * ldz]);
-    local_update<NQ, -1, T>(rows, nd, np, lx, Z, ldz, ly, sy);
-    stage(HX, nd);
-    local_update<NQ, -1, T>(
-        rows, nd, np, [&](int i, int c) { return operand(HX, i, c); }, Z, ldz,
-        [&](int i, int c) { return staged > 1 ? HY[i + c * ldy] : HPn[r0 + i + (long)idx[c] * n]; }, shp);
-    __syncthreads();
-  }
-  {
-    stage(W, na);
-    auto lw = [&](int i, int c) { return c < na ? operand(W, i, c) : zero<T>(); };
-    local_gram<T>(rows, na, np, lw, ly, Z, ldz);
-    cluster_sum<T>(cl, Z, ldz, na, np, xch + par * xch_len);
-    par ^= 1;
-    local_update<NQ, -1, T>(rows, na, np, lw, Z, ldz, ly, sy);
-    stage(HW, na);
-    local_update<NQ, -1, T>(
-        rows, na, np, [&](int i, int c) { return operand(HW, i, c); }, Z, ldz, lhp, shp);
-    __syncthreads();
-  }
+  // one projection against the orthonormal [X | W]
+  local_gram<T>(rows, nx, np, [&](int i, int c) { return c < nx ? operand(X, i, c) : zero<T>(); }, ly, Z, ldz);
+  if (threadIdx.x < np) Z[nx + threadIdx.x * ldz] = mk<T>(nu0[threadIdx.x], 0.0);
+  __syncthreads();
+  cluster_sum<T>(cl, Z, ldz, nx + 1, np, xch + par * xch_len);
+  par ^= 1;
+  if (threadIdx.x < np) nu0[threadIdx.x] = re(Z[nx + threadIdx.x * ldz]);
+  local_update<NQ, -1, T>(rows, nx, np, [&](int i, int c) { return operand(X, i, c); }, Z, ldz, ly, sy);
+  stage(HX);
+  local_update<NQ, -1, T>(
+      rows, nx, np, [&](int i, int c) { return operand(HX, i, c); }, Z, ldz,
+      [&](int i, int c) { return staged > 1 ? HY[i + c * ldy] : HPn[r0 + i + (long)idx[c] * n]; }, shp);
+  __syncthreads();
   int nk = np;
   bool ok = true;
   for (int pass = 0; pass < 2; ++pass) {
@@ -506,10 +517,10 @@ __global__ void __launch_bounds__(kT, 1)
       // the scaled Gram matrix of the kept columns, through Ri
       for (int e = threadIdx.x; e < nk * nk; e += kT) {
         const int r = e % nk, c = e / nk;
-        Ri[r + c * ldz] = mul(Z[keep[r] + keep[c] * ldz], scol[r] * scol[c]);
+        Ri[r + c * ldi] = mul(Z[keep[r] + keep[c] * ldz], scol[r] * scol[c]);
       }
       __syncthreads();
-      for (int e = threadIdx.x; e < nk * nk; e += kT) Z[e % nk + (e / nk) * ldz] = Ri[e % nk + (e / nk) * ldz];
+      for (int e = threadIdx.x; e < nk * nk; e += kT) Z[e % nk + (e / nk) * ldz] = Ri[e % nk + (e / nk) * ldi];
       __syncthreads();
     } else {
       if (threadIdx.x < nk) {
@@ -520,21 +531,21 @@ __global__ void __launch_bounds__(kT, 1)
       if (block_defect<T>(Z, ldz, nk, red) <= kSkipTol) break;
     }
     double rmin = 0.0;
-    ok = block_cholesky<T>(Z, ldz, nk, &rmin);
+    ok = block_cholesky<T>(Z, ldz, nk, &rmin, rinv);
     if (!ok || (pass == 0 && rmin < p_drop)) {
       nk = 0;
       break;
     }
-    block_inverse<T>(Z, ldz, nk, Ri, ldz);
+    block_inverse<T>(Z, ldz, nk, rinv, Ri, ldi);
     for (int e = threadIdx.x; e < nk * nk; e += kT) {
       const int r = e % nk, c = e / nk;
-      Ri[r + c * ldz] = mul(Ri[r + c * ldz], scol[r]);
+      Ri[r + c * ldi] = mul(Ri[r + c * ldi], scol[r]);
     }
     __syncthreads();
     local_update<NQ, 0, T>(
-        rows, nk, nk, [&](int i, int c) { return Y[i + keep[c] * ldy]; }, Ri, ldz, ly, sy);
+        rows, nk, nk, [&](int i, int c) { return Y[i + keep[c] * ldy]; }, Ri, ldi, ly, sy);
     local_update<NQ, 0, T>(
-        rows, nk, nk, [&](int i, int c) { return lhp(i, keep[c]); }, Ri, ldz, lhp, shp);
+        rows, nk, nk, [&](int i, int c) { return lhp(i, keep[c]); }, Ri, ldi, lhp, shp);
     __syncthreads();
   }
   for (int c = warp; c < nk; c += kW)
@@ -690,7 +701,7 @@ void split_rows(long n, int& C, int& rpc) {
 }
 
 template <typename T> size_t step_smem(int rpc, int cols, int zrows) {
-  return ((size_t)pad_ld(rpc) + 2 * (size_t)pad_ld(zrows)) * cols * sizeof(T);
+  return ((size_t)pad_ld(rpc) + pad_ld(zrows) + pad_ld(cols)) * cols * sizeof(T);
 }
 
 // Bytes of a staging buffer for `cols` columns of up to rpc rows: all rows, or what is left, or 0 where that is less
@@ -765,16 +776,16 @@ template <typename T> bool block_steps_fit(long n, int nd) {
   if (nd < 1 || nd > kMaxBlock) return false;
   int C, rpc;
   split_rows(n, C, rpc);
-  // P's block: nd columns, small matrices of nd + 1 rows; the subspace matrix: 2 nd rows, 3 nd columns
-  if (step_smem<T>(rpc, nd, nd + 1) > kSmemMax) return false;
+  // P's block: nd columns, small matrices of 2 nd + 1 rows; the subspace matrix: 2 nd rows, 3 nd columns
+  if (step_smem<T>(rpc, nd, 2 * nd + 1) > kSmemMax) return false;
   if ((size_t)pad_ld(2 * nd) * 3 * nd * sizeof(T) > kSmemMax) return false;
   bool fits = false;
   return configure<T>(&fits) == kOk && fits;
 }
 
 size_t block_steps_xch(int nd) {
-  // two buffers of (nd + 1) x nd, or one of 2 nd x 3 nd, per CTA
-  return (size_t)(kMaxC + 1) * std::max<size_t>(2 * (size_t)(nd + 1) * nd, (size_t)6 * nd * nd);
+  // two buffers of (2 nd + 1) x nd, or one of 2 nd x 3 nd, per CTA and for the total
+  return (size_t)(kMaxC + 1) * std::max<size_t>(2 * (size_t)(2 * nd + 1) * nd, (size_t)6 * nd * nd);
 }
 
 template <typename T>
@@ -782,32 +793,32 @@ Status block_w(const T* X, int nd, const T* Tb, const int* idx, int na, T* W, lo
                cudaStream_t s) {
   int C, rpc;
   split_rows(n, C, rpc);
-  const int zr = std::max(nd, na), ldy = pad_ld(rpc), ldz = pad_ld(zr);
+  const int zr = nd + na, ldy = pad_ld(rpc), ldz = pad_ld(zr);
   size_t sm = step_smem<T>(rpc, na, zr);
   const size_t more = (size_t)ldy * nd * sizeof(T);
   const int staged = nd > 0 && sm + more <= kSmemMax;
   if (staged) sm += more;
-  const long xl = (long)(kMaxC + 1) * std::max(nd, na) * na;
+  const long xl = (long)(kMaxC + 1) * (nd + na) * na;
   if (na <= 32)
-    return launch(k_block_w<T, 4>, C, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, staged, xch, xl, status);
-  return launch(k_block_w<T, 8>, C, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, staged, xch, xl, status);
+    return launch(k_block_w<T, 4>, C, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, pad_ld(na), staged, xch, xl, status);
+  return launch(k_block_w<T, 8>, C, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, pad_ld(na), staged, xch, xl, status);
 }
 
 template <typename T>
-Status block_p(const T* X, const T* HX, int nd, const T* W, const T* HW, int na, const T* Pn, const T* HPn,
-               const int* idx, int np, T* P, T* HP, long n, double p_drop, T* xch, int* status, cudaStream_t s) {
+Status block_p(const T* X, const T* HX, int nx, const T* Pn, const T* HPn, const int* idx, int np, T* P, T* HP,
+               long n, double p_drop, T* xch, int* status, cudaStream_t s) {
   int C, rpc;
   split_rows(n, C, rpc);
-  const int zr = std::max(nd + 1, std::max(na, np)), ldy = pad_ld(rpc), ldz = pad_ld(zr);
-  size_t sm = step_smem<T>(rpc, np, zr);
-  const size_t op = (size_t)ldy * std::max(nd, na) * sizeof(T), hp = (size_t)ldy * np * sizeof(T);
+  const int ldy = pad_ld(rpc), ldz = pad_ld(nx + 1);
+  size_t sm = step_smem<T>(rpc, np, nx + 1);
+  const size_t op = (size_t)ldy * nx * sizeof(T), hp = (size_t)ldy * np * sizeof(T);
   const int staged = sm + op + hp <= kSmemMax ? 2 : sm + op <= kSmemMax ? 1 : 0;
   sm += staged == 2 ? op + hp : staged == 1 ? op : 0;
-  const long xl = (long)(kMaxC + 1) * (nd + 1) * np;
+  const long xl = (long)(kMaxC + 1) * (nx + 1) * np;
   if (np <= 32)
-    return launch(k_block_p<T, 4>, C, sm, s, X, HX, nd, W, HW, na, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, staged,
+    return launch(k_block_p<T, 4>, C, sm, s, X, HX, nx, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, pad_ld(np), staged,
                   p_drop, xch, xl, status);
-  return launch(k_block_p<T, 8>, C, sm, s, X, HX, nd, W, HW, na, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, staged,
+  return launch(k_block_p<T, 8>, C, sm, s, X, HX, nx, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, pad_ld(np), staged,
                 p_drop, xch, xl, status);
 }
 

@@ -704,7 +704,7 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
     if (!pk.empty() && steps) {
       npc = (int)pk.size();
       PW_CUDA_TRY(cudaMemcpyAsync(w.idx, pk.data(), npc * sizeof(int), cudaMemcpyHostToDevice, s));
-      if ((r = block_p<T>(X, HX, nd, W, HW, na, Pn, HPn, w.idx, npc, P, HP, n, p_drop, xch, bst, s)) != kOk) return r;
+      if ((r = block_p<T>(X, HX, nd + na, Pn, HPn, w.idx, npc, P, HP, n, p_drop, xch, bst, s)) != kOk) return r;
       PW_CUDA_TRY(cudaMemcpyAsync(&npc, bst + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
       PW_CUDA_TRY(cudaStreamSynchronize(s));
     } else if (!pk.empty()) {

@@ -76,11 +76,11 @@ size_t block_steps_xch(int nd);  // entries of T in the exchange buffer
 template <typename T>
 Status block_w(const T* X, int nd, const T* Tb, const int* idx, int na, T* W, long n, T* xch, int* status,
                cudaStream_t s);
-// P, HP from Pn(:, idx), HPn(:, idx): projected out of X and W, near-dependent columns dropped, orthonormal;
-// status[1] = columns kept.
+// P, HP from Pn(:, idx), HPn(:, idx): projected out of the orthonormal columns [X | W] (nx of them side by side in X,
+// their H images in HX), near-dependent columns dropped, orthonormal; status[1] = columns kept.
 template <typename T>
-Status block_p(const T* X, const T* HX, int nd, const T* W, const T* HW, int na, const T* Pn, const T* HPn,
-               const int* idx, int np, T* P, T* HP, long n, double p_drop, T* xch, int* status, cudaStream_t s);
+Status block_p(const T* X, const T* HX, int nx, const T* Pn, const T* HPn, const int* idx, int np, T* P, T* HP,
+               long n, double p_drop, T* xch, int* status, cudaStream_t s);
 // Subspace matrix over [X(:, cols) | B], B = [W | P] with q columns (cols NULL: all in order).
 template <typename T>
 Status block_rr(const T* B, const T* HB, int q, const T* HX, const int* cols, int nx, const double* lam, const T* XX,
