@@ -658,21 +658,26 @@ __global__ void __launch_bounds__(kUpdThreads)
     }
 }
 
-// hpsi += B D B^H psi for nb bands: P = B^H psi summed over the cluster, Q = D P (D block-diagonal over atoms, blocks
-// row-major) and the update of the rows, in one launch.
+// hpsi += B D B^H psi: P = B^H psi summed over the cluster, Q = D P (D block-diagonal over atoms, blocks row-major) and
+// the update of the rows, in one launch; one cluster for every bw bands.
 template <typename T, int NQ>
 __global__ void __launch_bounds__(kT, 1)
-    k_block_nl(const T* __restrict__ B, int n_ch, const T* __restrict__ psi, long ldpsi, int nb, T* __restrict__ hpsi,
+    k_block_nl(const T* __restrict__ B, int n_ch, const T* __restrict__ psi, long ldpsi, int nb_all, int bw,
+               T* __restrict__ hpsi,
                long ldh, long n, int rpc, int ldz, int cap, T* __restrict__ xch, const int* __restrict__ ch_atom,
                const int* __restrict__ atom_ch_start, const int* __restrict__ d_off,
                const double* __restrict__ d_vals) {
   extern __shared__ __align__(16) unsigned char smem[];
-  T* Z = reinterpret_cast<T*>(smem);    // n_ch x nb
-  T* Q = Z + (size_t)ldz * nb;          // n_ch x nb
   cg::cluster_group cl = cg::this_cluster();
+  const int group = blockIdx.x / (int)cl.num_blocks(), first = group * bw, nb = min(bw, nb_all - first);
+  psi += first * ldpsi;
+  hpsi += first * ldh;
+  xch += (size_t)group * (kMaxC + 1) * n_ch * bw;
+  T* Z = reinterpret_cast<T*>(smem);    // n_ch x bw
+  T* Q = Z + (size_t)ldz * bw;          // n_ch x bw
   const long r0 = (long)cl.block_rank() * rpc;
   const int rows = (int)max(0L, min((long)rpc, n - r0));
-  T* buf = Q + (size_t)ldz * nb;
+  T* buf = Q + (size_t)ldz * bw;
   const int lds = staged_gram<T>(
       rows, n_ch, nb, [&](int c) { return B + r0 + (long)c * n; },
       [&](int c) { return psi + r0 + (long)c * ldpsi; }, Z, ldz, buf, cap);
@@ -752,10 +757,10 @@ template <typename T> Status configure(bool* fits) {
 }
 
 template <typename... P, typename... A>
-Status launch(void (*kern)(P...), int C, size_t smem, cudaStream_t s, A... args) {
+Status launch_clusters(void (*kern)(P...), int C, int clusters, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
-  cfg.gridDim = dim3(C, 1, 1);
+  cfg.gridDim = dim3(C * clusters, 1, 1);
   cfg.blockDim = dim3(kT, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
@@ -768,6 +773,16 @@ Status launch(void (*kern)(P...), int C, size_t smem, cudaStream_t s, A... args)
   count_launch();
   if (e != cudaSuccess) return fail(kCuda, std::string("block step launch: ") + cudaGetErrorString(e));
   return kOk;
+}
+template <typename... P, typename... A>
+Status launch(void (*kern)(P...), int C, size_t smem, cudaStream_t s, A... args) {
+  return launch_clusters(kern, C, 1, smem, s, args...);
+}
+
+// Bands per cluster of the projector term: groups of eight or more, eight clusters at most.
+int nl_group(int nb) {
+  const int groups = std::min(8, (nb + 7) / 8);
+  return ((nb + groups - 1) / groups + 7) / 8 * 8;
 }
 
 }  // namespace
@@ -847,20 +862,27 @@ Status block_update(T* X, const T* B, T* Pn, T* HX, const T* HB, T* HPn, const T
   return kOk;
 }
 
-// One launch is the faster form while the products are small enough for one
-// cluster's FP64 rate (16 of the 148 SMs); beyond that the library products'
-// spread over the whole GPU wins.
+// One launch is the faster form while the products are small: the clusters'
+// tile products reach a fraction of the library products' rate.  H|psi> in
+// one launch against library products, by n_pw x channels x bands (complex,
+// FP64): 725 x 10 x 12 26 us against 35, 1647 x 40 x 28 36 against 50,
+// 3791 x 40 x 28 (4.2e6) 51 against 60, 3423 x 32 x 70 (7.7e6) 86 against 92;
+// but 3301 x 80 x 20 (5.3e6) 64 against 55 and 4573 x 80 x 40 (1.5e7) 106
+// against 91.  A real multiply-add is a quarter of a complex one; three times
+// the limit is where the real form has been measured to gain (3791 x 40 x 22).
+constexpr double kNlFusedWork = 5e6;
 template <typename T> bool nl_fused_ok(const Handle& h, int nb) {
   const double work = (double)h.n_pw * h.n_ch * nb;
-  if (h.n_ch < 1 || work > (sizeof(T) == sizeof(double) ? 8.0e6 : 2.5e6)) return false;
-  if ((size_t)2 * pad_ld(h.n_ch) * nb * sizeof(T) > kSmemMax) return false;
+  if (h.n_ch < 1 || work > (sizeof(T) == sizeof(double) ? 3.0 : 1.0) * kNlFusedWork) return false;
+  if ((size_t)2 * pad_ld(h.n_ch) * nl_group(nb) * sizeof(T) > kSmemMax) return false;
   bool fits = false;
   return configure<T>(&fits) == kOk && fits;
 }
 
 template <typename T>
 Status nl_fused(Handle& h, const T* B, const T* psi, long ldpsi, int nb, T* hpsi, long ldh, cudaStream_t s) {
-  const size_t need = (size_t)(kMaxC + 1) * h.n_ch * nb * sizeof(T);
+  const int bw = nl_group(nb), clusters = (nb + bw - 1) / bw;
+  const size_t need = (size_t)clusters * (kMaxC + 1) * h.n_ch * bw * sizeof(T);
   if (need > h.nl_xch_bytes) {
     if (h.nl_xch) cudaFree(h.nl_xch);
     h.nl_xch = nullptr;
@@ -872,11 +894,12 @@ Status nl_fused(Handle& h, const T* B, const T* psi, long ldpsi, int nb, T* hpsi
   int C, rpc;
   split_rows(h.n_pw, C, rpc);
   const int ldz = pad_ld(h.n_ch);
-  const size_t zb = (size_t)2 * ldz * nb * sizeof(T);
-  const size_t buf = stage_bytes<T>(rpc, h.n_ch + nb, kSmemMax - zb);
-  return launch(k_block_nl<T, 4>, C, zb + buf, s, B, h.n_ch, psi, ldpsi, nb, hpsi, ldh, (long)h.n_pw, rpc, ldz,
-                (int)(buf / sizeof(T)), static_cast<T*>(h.nl_xch), (const int*)h.ch_atom,
-                (const int*)h.atom_ch_start, (const int*)h.d_off, (const double*)h.d_vals);
+  const size_t zb = (size_t)2 * ldz * bw * sizeof(T);
+  const size_t buf = stage_bytes<T>(rpc, h.n_ch + bw, kSmemMax - zb);
+  return launch_clusters(k_block_nl<T, 4>, C, clusters, zb + buf, s, B, h.n_ch, psi, ldpsi, nb, bw, hpsi, ldh,
+                         (long)h.n_pw, rpc, ldz, (int)(buf / sizeof(T)), static_cast<T*>(h.nl_xch),
+                         (const int*)h.ch_atom, (const int*)h.atom_ch_start, (const int*)h.d_off,
+                         (const double*)h.d_vals);
 }
 
 #define PW_BLOCK(T)                                                                                                  \
@@ -884,8 +907,8 @@ Status nl_fused(Handle& h, const T* B, const T* psi, long ldpsi, int nb, T* hpsi
   template Status nl_fused<T>(Handle&, const T*, const T*, long, int, T*, long, cudaStream_t);                       \
   template bool block_steps_fit<T>(long, int);                                                                      \
   template Status block_w<T>(const T*, int, const T*, const int*, int, T*, long, T*, int*, cudaStream_t);            \
-  template Status block_p<T>(const T*, const T*, int, const T*, const T*, int, const T*, const T*, const int*, int, \
-                             T*, T*, long, double, T*, int*, cudaStream_t);                                          \
+  template Status block_p<T>(const T*, const T*, int, const T*, const T*, const int*, int, T*, T*, long, double, T*, \
+                             int*, cudaStream_t);                                                                   \
   template Status block_rr<T>(const T*, const T*, int, const T*, const int*, int, const double*, const T*, long,     \
                               T*, T*, cudaStream_t);                                                                 \
   template Status block_update<T>(T*, const T*, T*, T*, const T*, T*, const T*, int, int, int, const int*,           \
