@@ -659,7 +659,8 @@ __global__ void __launch_bounds__(kUpdThreads)
 }
 
 // hpsi += B D B^H psi: P = B^H psi summed over the cluster, Q = D P (D block-diagonal over atoms, blocks row-major) and
-// the update of the rows, in one launch; one cluster for every bw bands.
+// the update of the rows, in one launch; one cluster for every bw bands.  Only the update reads what the launch before it
+// (the last pass of the local part) wrote, so the sums run beside that pass.
 template <typename T, int NQ>
 __global__ void __launch_bounds__(kT, 1)
     k_block_nl(const T* __restrict__ B, int n_ch, const T* __restrict__ psi, long ldpsi, int nb_all, int bw,
@@ -691,6 +692,7 @@ __global__ void __launch_bounds__(kT, 1)
     Q[c + b * ldz] = acc;
   }
   __syncthreads();
+  launch_wait();
   for (int b0 = 0; b0 < nb; b0 += 8 * NQ)
     local_update<NQ, 1, T>(
         rows, n_ch, min(8 * NQ, nb - b0), lb, Q + (size_t)b0 * ldz, ldz,
@@ -757,9 +759,9 @@ template <typename T> Status configure(bool* fits) {
 }
 
 template <typename... P, typename... A>
-Status launch_clusters(void (*kern)(P...), int C, int clusters, size_t smem, cudaStream_t s, A... args) {
+Status launch_clusters(void (*kern)(P...), int C, int clusters, bool early, size_t smem, cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   cfg.gridDim = dim3(C * clusters, 1, 1);
   cfg.blockDim = dim3(kT, 1, 1);
   cfg.dynamicSmemBytes = smem;
@@ -767,8 +769,10 @@ Status launch_clusters(void (*kern)(P...), int C, int clusters, size_t smem, cud
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = C;
   attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 2 : 1;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
   count_launch();
   if (e != cudaSuccess) return fail(kCuda, std::string("block step launch: ") + cudaGetErrorString(e));
@@ -776,7 +780,7 @@ Status launch_clusters(void (*kern)(P...), int C, int clusters, size_t smem, cud
 }
 template <typename... P, typename... A>
 Status launch(void (*kern)(P...), int C, size_t smem, cudaStream_t s, A... args) {
-  return launch_clusters(kern, C, 1, smem, s, args...);
+  return launch_clusters(kern, C, 1, false, smem, s, args...);
 }
 
 // Bands per cluster of the projector term: groups of eight or more, eight clusters at most.
@@ -896,7 +900,7 @@ Status nl_fused(Handle& h, const T* B, const T* psi, long ldpsi, int nb, T* hpsi
   const int ldz = pad_ld(h.n_ch);
   const size_t zb = (size_t)2 * ldz * bw * sizeof(T);
   const size_t buf = stage_bytes<T>(rpc, h.n_ch + bw, kSmemMax - zb);
-  return launch_clusters(k_block_nl<T, 4>, C, clusters, zb + buf, s, B, h.n_ch, psi, ldpsi, nb, bw, hpsi, ldh,
+  return launch_clusters(k_block_nl<T, 4>, C, clusters, true, zb + buf, s, B, h.n_ch, psi, ldpsi, nb, bw, hpsi, ldh,
                          (long)h.n_pw, rpc, ldz, (int)(buf / sizeof(T)), static_cast<T*>(h.nl_xch),
                          (const int*)h.ch_atom, (const int*)h.atom_ch_start, (const int*)h.d_off,
                          (const double*)h.d_vals);

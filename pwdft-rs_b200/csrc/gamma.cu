@@ -50,6 +50,7 @@ __global__ void k_unpack_pairs(const double* __restrict__ u, long ldu, int nb, d
   const double* ua = u + (long)a * ldu;
   const double* ub = u + (long)(hb ? b : a) * ldu;
   double2* cq = c + (long)q * ldc;
+  launch_release();
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t <= nh; t += gridDim.x * blockDim.x) {
     if (t == 0) {
       cq[zero] = make_double2(wa * ua[0], wb * ub[0]);
@@ -64,7 +65,7 @@ __global__ void k_unpack_pairs(const double* __restrict__ u, long ldu, int nb, d
 }
 
 // inverse of k_unpack_pairs for (H c): separate the two real bands and pack
-__global__ void k_pack_pairs(const double2* __restrict__ c, long ldc, int nb, double* __restrict__ u, long ldu,
+__global__ void k_pack_pairs(const double2* c, long ldc, int nb, double* __restrict__ u, long ldu,
                              const int* __restrict__ half_idx, const int* __restrict__ half_neg, int zero, int nh) {
   const int q = blockIdx.y;
   const int a = 2 * q, b = 2 * q + 1;
@@ -72,6 +73,8 @@ __global__ void k_pack_pairs(const double2* __restrict__ c, long ldc, int nb, do
   const double2* cq = c + (long)q * ldc;
   double* ua = u + (long)a * ldu;
   double* ub = hb ? u + (long)b * ldu : nullptr;
+  launch_wait();
+  launch_release();
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t <= nh; t += gridDim.x * blockDim.x) {
     if (t == 0) {
       const double2 z = cq[zero];
@@ -390,7 +393,8 @@ Status apply_h_real(Handle& h, int spin, const double* u, long ldu, int nb, doub
   k_unpack_pairs<<<grid, 256, 0, s>>>(u, ldu, nb, h.gam_c1, n, g.half_idx, g.half_neg, g.zero, g.nh, nullptr);
   count_launch();
   if ((r = apply_local_device(h, spin, 0, h.gam_c1, n, npairs, h.gam_c2, n, precision, s)) != kOk) return r;
-  k_pack_pairs<<<grid, 256, 0, s>>>(h.gam_c2, n, nb, hu, ldh, g.half_idx, g.half_neg, g.zero, g.nh);
+  PW_CUDA_TRY(launch_early(k_pack_pairs, grid, 256, 0, s, h.gam_c2, (long)n, nb, hu, ldh, g.half_idx, g.half_neg,
+                           g.zero, g.nh));
   count_launch();
   if (h.n_ch > 0 && precision == 1 && nl_mixed_eligible(h)) {
     // mixed form: both projector products as 3xBF16 tensor-core GEMMs (every

@@ -64,6 +64,8 @@ __global__ void __launch_bounds__(plane_threads(X0, X1), sizeof(R) == 4 ? 3 : (X
   const long ncol = (long)g.Xp * g.Yp;
   for (int i = tid; i < d0; i += T) TX[i] = twx[i];
   for (int i = tid; i < d1; i += T) TY[i] = twy[i];
+  launch_wait();
+  launch_release();
   __syncthreads();
   const R* vp = vz + (long)z * d0 * d1;
   const int b0 = blockIdx.y * bpc, b1 = min(nb, b0 + bpc);
@@ -216,6 +218,8 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2)
   const int z = blockIdx.x;
   for (int i = threadIdx.x; i < gin.d0; i += blockDim.x) TX[i] = twx[i];
   for (int i = threadIdx.x; i < gin.d1; i += blockDim.x) TY[i] = twy[i];
+  launch_wait();
+  launch_release();
   __syncthreads();
   const R* vp = vz + (long)z * gin.d0 * gin.d1;
   const long ncol = (long)gin.Xp * gin.Yp;
@@ -250,13 +254,15 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2)
 // points col_start[c] .. col_start[c + 1] - 1 at consecutive n2 from col_lo[c].
 template <typename R, int Z0, int Z1>
 __global__ void __launch_bounds__(kZCols * (Z0 > Z1 ? Z0 : Z1))
-    k_zi(const double2* __restrict__ psi, long ldpsi, cplx<R>* __restrict__ A, const int* __restrict__ col_start,
+    k_zi(const double2* psi, long ldpsi, cplx<R>* __restrict__ A, const int* __restrict__ col_start,
          const int* __restrict__ col_lo, int ncol, int m2, const cplx<R>* __restrict__ tw) {
   using C = cplx<R>;
   constexpr int d2 = Z0 * Z1, ld = d2 | 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
   const int c0 = blockIdx.x * kZCols, tid = threadIdx.x;
+  launch_wait();
+  launch_release();
   const double2* ps = psi + (long)blockIdx.y * ldpsi;
   if (tid < kZCols * Z1) {
     const int c = tid / Z1, j = tid - c * Z1, col = c0 + c;
@@ -300,7 +306,7 @@ __global__ void __launch_bounds__(kZCols * (Z0 > Z1 ? Z0 : Z1))
 // K5: z-forward of kZCols columns, Hpsi = value / N + T psi at the sphere points.
 template <typename R, int Z0, int Z1>
 __global__ void __launch_bounds__(kZCols * (Z0 > Z1 ? Z0 : Z1))
-    k_zf(const cplx<R>* __restrict__ A, const double2* __restrict__ psi, long ldpsi, double2* __restrict__ hpsi,
+    k_zf(const cplx<R>* A, const double2* __restrict__ psi, long ldpsi, double2* __restrict__ hpsi,
          long ldh, const double* __restrict__ kin, double scale, const int* __restrict__ col_start,
          const int* __restrict__ col_lo, int ncol, int m2, const cplx<R>* __restrict__ tw) {
   using C = cplx<R>;
@@ -308,6 +314,8 @@ __global__ void __launch_bounds__(kZCols * (Z0 > Z1 ? Z0 : Z1))
   extern __shared__ __align__(16) unsigned char smem_raw[];
   C* buf = reinterpret_cast<C*>(smem_raw);
   const int c0 = blockIdx.x * kZCols, tid = threadIdx.x;
+  launch_wait();
+  launch_release();
   if (tid < kZCols * Z0) {
     const int c = tid % kZCols, k1 = tid / kZCols, col = c0 + c;
     C v[Z1];
@@ -439,8 +447,8 @@ static void launch_zi(const Handle& h, const double2* psi, long ldpsi, cplx<R>* 
   switch (g.pair[2]) {
 #define PW_CASE(r0, r1)                                                                                              \
   case pair_id(r0, r1):                                                                                              \
-    k_zi<R, r0, r1><<<grid, kZCols*(r0 > r1 ? r0 : r1), sm, s>>>(psi, ldpsi, A, g.col_start, g.col_lo, g.ncol, g.m[2], \
-                                                                 Tables<R>::tw(g, 2));                               \
+    launch_early(k_zi<R, r0, r1>, grid, kZCols*(r0 > r1 ? r0 : r1), sm, s, psi, ldpsi, A, g.col_start, g.col_lo,     \
+                 g.ncol, g.m[2], Tables<R>::tw(g, 2));                                                               \
     break;
     PW_PAIRS(PW_CASE)
 #undef PW_CASE
@@ -500,23 +508,23 @@ Status local_plane(Handle& h, int spin, int ik, const double2* psi, long ldpsi, 
     switch (g.pair[0]) {
 #define PW_CASE(r0, r1)                                                                                       \
   case pair_id(r0, r1):                                                                                       \
-    k_plane<R, r0, r1><<<pgrid, plane_threads(r0, r1), plane_smem<R>(g), s>>>(A, vz, nb, bpc, d2, geo, tw0, tw1); \
+    launch_early(k_plane<R, r0, r1>, pgrid, plane_threads(r0, r1), plane_smem<R>(g), s, A, vz, nb, bpc, d2,   \
+                 geo, tw0, tw1);                                                                              \
     break;
       PW_PAIRS(PW_CASE)
 #undef PW_CASE
     }
   } else {
-    k_plane_rt<R><<<pgrid, 256, plane_smem<R>(g), s>>>(A, vz, nb, bpc, d2, geo, plane_rows(g), g.pair[0], g.pair[1],
-                                                       tw0, tw1);
+    launch_early(k_plane_rt<R>, pgrid, 256, plane_smem<R>(g), s, A, vz, nb, bpc, d2, geo, plane_rows(g), g.pair[0],
+                 g.pair[1], tw0, tw1);
   }
   count_launch();
   mark(tm, 2, s);
   switch (g.pair[2]) {
 #define PW_CASE(r0, r1)                                                                                      \
   case pair_id(r0, r1):                                                                                      \
-    k_zf<R, r0, r1><<<zgrid, kZCols*(r0 > r1 ? r0 : r1), zsm, s>>>(A, psi, ldpsi, hpsi, ldh,                 \
-                                                                   h.kp[ik].kinetic, 1.0 / (double)g.N,      \
-                                                                   g.col_start, g.col_lo, g.ncol, g.m[2], tw2); \
+    launch_early(k_zf<R, r0, r1>, zgrid, kZCols*(r0 > r1 ? r0 : r1), zsm, s, A, psi, ldpsi, hpsi, ldh,       \
+                 h.kp[ik].kinetic, 1.0 / (double)g.N, g.col_start, g.col_lo, g.ncol, g.m[2], tw2);           \
     break;
     PW_PAIRS(PW_CASE)
 #undef PW_CASE

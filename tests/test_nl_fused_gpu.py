@@ -60,3 +60,28 @@ def test_packed_real_matches_complex(nb, si_pp):
         dev.set_veff_g(veff)
         got = dev.apply_h_packed(u)
     assert np.max(np.abs(got - ref)) / np.max(np.abs(ref)) < 1e-12
+
+
+@pytest.mark.parametrize("nb", [3, 20, 64])
+def test_dependent_calls_without_waits(nb, si_pp):
+    """Each launch may begin while the one before it runs: a chain of calls, each reading the block the call before it
+    wrote and overwriting the one that call read, equals the same chain with a wait after every call."""
+    import torch
+
+    s = build_system(diamond_primitive("Si", 5.431), {"Si": si_pp}, 260.0, [KPoint(np.array([0.11, -0.23, 0.31]), 1.0)])
+    g = rng(nb)
+    psi = g.standard_normal((nb, s.n_pw)) + 1j * g.standard_normal((nb, s.n_pw))
+    with PwGpu(s) as dev:
+        dev.set_veff_g(_veff(s))
+        out = []
+        for wait in (True, False):
+            a, b = torch.from_numpy(psi).cuda(), torch.empty((nb, s.n_pw), dtype=torch.complex128, device="cuda")
+            torch.cuda.synchronize()
+            for _ in range(6):
+                dev.apply_h_device(a.data_ptr(), s.n_pw, nb, b.data_ptr(), s.n_pw)
+                if wait:
+                    torch.cuda.synchronize()
+                a, b = b, a
+            torch.cuda.synchronize()
+            out.append(a.cpu().numpy())
+    assert np.array_equal(out[0], out[1])
