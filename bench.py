@@ -64,10 +64,9 @@ BATCH = 4  # Si64 cells solved concurrently in one step
 # each band plus one FP32 V(r) read (the output stays in L2), so it is scaled
 # to a launch's band count as (capture - V) / 22 per band + V.
 XV_TRAFFIC_CAPTURE = (33503744 + 3072, 22)
-# the fused middle kernel (k_yxy_ct<float, 8, 9, 8, 9>) on the same grid:
-# dram__bytes_read.sum + dram__bytes_write.sum of one 20-band launch from one
-# ncu capture (the written planes stay in L2), scaled by a launch's bands
-YXY_TRAFFIC_CAPTURE = (17050880, 20)
+# the fused middle kernel (k_plane<float, 8, 9>) on the same grid has no
+# capture of its own yet: its traffic is reported as null
+PLANE_TRAFFIC_CAPTURE = (None, 20)
 
 
 def load_peaks():
@@ -610,7 +609,7 @@ def kernel_bench(local, steps, warmup, flush, hbm_peak, peak_kind):
         v_bytes = 4.0 * N
         traffic = (cap - v_bytes) / cap_bands * bands + v_bytes
     elif dom == "fft_x_mid" and fused and (d0, d1, d2) == (72, 72, 72):
-        cap, cap_bands = YXY_TRAFFIC_CAPTURE
+        cap, cap_bands = PLANE_TRAFFIC_CAPTURE
         traffic = None if cap is None else cap / cap_bands * bands
     roofline = {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                 "frac": achieved / hbm_peak,
@@ -626,7 +625,7 @@ def kernel_bench(local, steps, warmup, flush, hbm_peak, peak_kind):
         roofline["compulsory_frac"] = comp / (ms_launch * 1e-3) / 1e9 / hbm_peak
         roofline["compulsory_note"] = ("what the fused kernel must move: the compact planes read and written once "
                                        "per band and V(r) once; it is bound by shared memory, not HBM")
-    # the whole local H|psi> (the five FFT kernels) against its per-band algorithmic bytes
+    # the whole local H|psi> (its FFT kernels) against its per-band algorithmic bytes
     # 2c n_pw + 4c N + (c/2) N, c = 8 B (FP32 complex)
     pipe_bytes = hpsi_algorithmic_bytes(n_pw, N, 8) * nb
     fft_stages = ("fft_z_inv_scatter", "fft_y_inv", "fft_x_mid", "fft_y_fwd", "fft_z_fwd_gather")
@@ -635,7 +634,7 @@ def kernel_bench(local, steps, warmup, flush, hbm_peak, peak_kind):
     roofline["local_hpsi"] = {"bound": "hbm", "achieved": pipe_gbs, "peak": hbm_peak, "unit": "GB/s",
                               "frac": pipe_gbs / hbm_peak, "alg_bytes_per_block": pipe_bytes, "ms_per_block": pipe_ms,
                               "bands": nb,
-                              "note": "five FFT kernels of one mixed H|psi> block, per-band bytes "
+                              "note": "FFT kernels of one mixed H|psi> block, per-band bytes "
                                       "2c n_pw + 4c N + (c/2) N with c = 8 B"}
     return out, roofline, {"n_pw": n_pw, "grid": [d0, d1, d2], "n_bands": nb, "n_ch": 256}
 
