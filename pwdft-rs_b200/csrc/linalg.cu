@@ -1,4 +1,4 @@
-// Dense FP64 linear algebra of the Rayleigh-Ritz step.
+// Batched small generalized eigenproblems (pwgpu_small_geneig).
 //
 // Small generalized Hermitian eigenproblems H c = lambda S c (m <= 64) are
 // solved one problem per thread block, batched over k-points:
@@ -8,8 +8,9 @@
 //   [[c, s u], [-s u*, c]], u = A_pq/|A_pq|, t = tan(theta) from
 //   zeta = (A_qq - A_pp) / (2|A_pq|)), eigenvalues sorted ascending,
 //   C = L^{-H} V.
-// Larger problems go to cuSOLVER zhegvd.  Replaces the reference's dense
-// self_adjoint_eigen (eigensolver/dense.rs:50-98) inside the subspace.
+// The subspaces of the eigensolver are standard problems and go to eigh.cu.
+// Counterpart of the reference's dense self_adjoint_eigen
+// (eigensolver/dense.rs:50-98) for small matrices.
 #include <cusolverDn.h>
 
 #include <algorithm>
