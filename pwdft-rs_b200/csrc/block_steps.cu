@@ -15,10 +15,13 @@
 //
 // Against the library-call steps, with the same subspace eigensolver (B200):
 // restart iteration of 8 Si atoms at Gamma (real, 22 columns, 2,945 rows)
-// 27.7 -> 14.5 ms, of 2 atoms over 6 k-points (complex, 10 columns, 411 rows)
-// 21.0 -> 8.7 ms, whole LSDA run of 8 C atoms (27 columns, 1,045 rows, 40
-// blocks on 8 lanes) 405 -> 238 ms.  One Cholesky barrier a column instead of
-// three, and one sum less for each of W and P, are 5 % of those.
+// 27.7 -> 13.5 ms, of 2 atoms over 6 k-points (complex, 10 columns, 411 rows)
+// 21.0 -> 7.9 ms, whole LSDA run of 8 C atoms (27 columns, 1,045 rows, 40
+// blocks on 8 lanes) 405 -> 231 ms.  One Cholesky barrier a column instead of
+// three, and one sum less for each of W and P, are 5 % of those; launches that
+// begin beside the end of the one before them, and one copy of the column lists
+// a step, another 3 to 7 %.  A cluster lets its successor begin only near its
+// own end, so that a waiting cluster does not keep SMs from other lanes.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -422,6 +425,7 @@ __global__ void __launch_bounds__(kT, 1)
     local_update<NQ, 0, T>(rows, na, na, ly, Ri, ldi, ly, sy);
     __syncthreads();
   }
+  launch_release();
   for (int c = threadIdx.x >> 5; c < na; c += kW)
     for (int i = threadIdx.x & 31; i < rows; i += 32) W[r0 + i + (long)c * n] = Y[i + c * ldy];
   if (rank == 0 && threadIdx.x == 0) status[0] = ok ? 0 : 1;
@@ -433,8 +437,8 @@ __global__ void __launch_bounds__(kT, 1)
 // dependent).
 template <typename T, int NQ>
 __global__ void __launch_bounds__(kT, 1)
-    k_block_p(const T* __restrict__ X, const T* __restrict__ HX, int nx, const T* __restrict__ Pn,
-              const T* __restrict__ HPn, const int* __restrict__ idx, int np, T* __restrict__ P,
+    k_block_p(const T* X, const T* HX, int nx, const T* __restrict__ Pn,
+              const T* __restrict__ HPn, const int* idx, int np, T* __restrict__ P,
               T* __restrict__ HP, long n, int rpc, int ldy,
               int ldz, int ldi, int staged, double p_drop, T* __restrict__ xch, long xch_len, int* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -449,6 +453,7 @@ __global__ void __launch_bounds__(kT, 1)
   T* Ri = Z + (size_t)ldz * np;
   T* S = Ri + (size_t)ldi * np;     // rpc x nx, staged >= 1: [X | W], then [HX | HW]
   T* HY = S + (size_t)ldy * nx;     // rpc x np, staged == 2: HP
+  launch_wait();
   const long r0 = (long)rank * rpc;
   const int rows = (int)max(0L, min((long)rpc, n - r0));
   stage_cols<T>(Y, ldy, rows, np, [&](int c) { return Pn + r0 + (long)idx[c] * n; });
@@ -560,7 +565,7 @@ __global__ void __launch_bounds__(kT, 1)
 // HX(:, cols), (G + G^H) / 2 with G = B^H HB.  cols NULL: the columns in order.
 template <typename T>
 __global__ void __launch_bounds__(kT, 1)
-    k_block_rr(const T* __restrict__ B, const T* __restrict__ HB, int q, const T* __restrict__ HX,
+    k_block_rr(const T* B, const T* HB, int q, const T* HX,
                const int* __restrict__ cols, int nx, const double* __restrict__ lam, const T* __restrict__ XX, long n,
                int rpc, int ldz, int cap, T* __restrict__ xch, T* __restrict__ Hs) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -576,6 +581,7 @@ __global__ void __launch_bounds__(kT, 1)
       Z + (size_t)ldz * m, cap);
   for (int e = threadIdx.x; e < nz; e += kT) xch[(size_t)rank * nz + e] = Z[e % q + (e / q) * ldz];
   cl.sync();
+  launch_release();
   // entry (r, c) of B^H [HX | HB], summed over the CTAs
   auto entry = [&](int r, int c) { return rank_sum<T>(xch, C, nz, r + (size_t)c * q); };
   for (int e = rank * kT + threadIdx.x; e < m * m; e += C * kT) {
@@ -605,7 +611,7 @@ constexpr int kUpdThreads = 128;
 template <typename T, int NQ>
 __global__ void __launch_bounds__(kUpdThreads)
     k_block_update(T* __restrict__ X, const T* __restrict__ B, T* __restrict__ Pn, T* __restrict__ HX,
-                   const T* __restrict__ HB, T* __restrict__ HPn, const T* __restrict__ Cm, int m, int nx, int q,
+                   const T* __restrict__ HB, T* __restrict__ HPn, const T* Cm, int m, int nx, int q,
                    const int* __restrict__ cols, const int* __restrict__ pcols, int np, long n) {
   T* x = blockIdx.y ? HX : X;
   const T* b = blockIdx.y ? HB : B;
@@ -619,6 +625,8 @@ __global__ void __launch_bounds__(kUpdThreads)
   __syncthreads();
   for (int t = threadIdx.x; t < np; t += kUpdThreads) pos[pcols ? pcols[t] : t] = t;
   __syncthreads();
+  launch_wait();
+  launch_release();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kr = lane & 3, kc = lane >> 2;
   const long i = ((long)blockIdx.x * (kUpdThreads / 32) + warp) * 8 + kc;
@@ -693,6 +701,7 @@ __global__ void __launch_bounds__(kT, 1)
   }
   __syncthreads();
   launch_wait();
+  launch_release();
   for (int b0 = 0; b0 < nb; b0 += 8 * NQ)
     local_update<NQ, 1, T>(
         rows, n_ch, min(8 * NQ, nb - b0), lb, Q + (size_t)b0 * ldz, ldz,
@@ -779,8 +788,8 @@ Status launch_clusters(void (*kern)(P...), int C, int clusters, bool early, size
   return kOk;
 }
 template <typename... P, typename... A>
-Status launch(void (*kern)(P...), int C, size_t smem, cudaStream_t s, A... args) {
-  return launch_clusters(kern, C, 1, false, smem, s, args...);
+Status launch(void (*kern)(P...), int C, bool early, size_t smem, cudaStream_t s, A... args) {
+  return launch_clusters(kern, C, 1, early, smem, s, args...);
 }
 
 // Bands per cluster of the projector term: groups of eight or more, eight clusters at most.
@@ -819,8 +828,8 @@ Status block_w(const T* X, int nd, const T* Tb, const int* idx, int na, T* W, lo
   if (staged) sm += more;
   const long xl = (long)(kMaxC + 1) * (nd + na) * na;
   if (na <= 32)
-    return launch(k_block_w<T, 4>, C, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, pad_ld(na), staged, xch, xl, status);
-  return launch(k_block_w<T, 8>, C, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, pad_ld(na), staged, xch, xl, status);
+    return launch(k_block_w<T, 4>, C, false, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, pad_ld(na), staged, xch, xl, status);
+  return launch(k_block_w<T, 8>, C, false, sm, s, X, nd, Tb, idx, na, W, n, rpc, ldy, ldz, pad_ld(na), staged, xch, xl, status);
 }
 
 template <typename T>
@@ -835,9 +844,9 @@ Status block_p(const T* X, const T* HX, int nx, const T* Pn, const T* HPn, const
   sm += staged == 2 ? op + hp : staged == 1 ? op : 0;
   const long xl = (long)(kMaxC + 1) * (nx + 1) * np;
   if (np <= 32)
-    return launch(k_block_p<T, 4>, C, sm, s, X, HX, nx, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, pad_ld(np), staged,
+    return launch(k_block_p<T, 4>, C, true, sm, s, X, HX, nx, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, pad_ld(np), staged,
                   p_drop, xch, xl, status);
-  return launch(k_block_p<T, 8>, C, sm, s, X, HX, nx, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, pad_ld(np), staged,
+  return launch(k_block_p<T, 8>, C, true, sm, s, X, HX, nx, Pn, HPn, idx, np, P, HP, n, rpc, ldy, ldz, pad_ld(np), staged,
                 p_drop, xch, xl, status);
 }
 
@@ -849,7 +858,7 @@ Status block_rr(const T* B, const T* HB, int q, const T* HX, const int* cols, in
   const int ldz = pad_ld(q);
   const size_t zb = (size_t)ldz * (nx + q) * sizeof(T);
   const size_t buf = stage_bytes<T>(rpc, nx + 2 * q, kSmemMax - zb);
-  return launch(k_block_rr<T>, C, zb + buf, s, B, HB, q, HX, cols, nx, lam, XX, n, rpc, ldz, (int)(buf / sizeof(T)),
+  return launch(k_block_rr<T>, C, false, zb + buf, s, B, HB, q, HX, cols, nx, lam, XX, n, rpc, ldz, (int)(buf / sizeof(T)),
                 xch, Hs);
 }
 
@@ -858,9 +867,11 @@ Status block_update(T* X, const T* B, T* Pn, T* HX, const T* HB, T* HPn, const T
                     const int* cols, const int* pcols, int np, long n, cudaStream_t s) {
   const dim3 grid((unsigned)((n + 8 * (kUpdThreads / 32) - 1) / (8 * (kUpdThreads / 32))), 2);
   if (nx <= 32)
-    k_block_update<T, 4><<<grid, kUpdThreads, 0, s>>>(X, B, Pn, HX, HB, HPn, Cm, m, nx, q, cols, pcols, np, n);
+    PW_CUDA_TRY(launch_early(k_block_update<T, 4>, grid, kUpdThreads, 0, s, X, B, Pn, HX, HB, HPn, Cm, m, nx, q, cols,
+                             pcols, np, n));
   else
-    k_block_update<T, 8><<<grid, kUpdThreads, 0, s>>>(X, B, Pn, HX, HB, HPn, Cm, m, nx, q, cols, pcols, np, n);
+    PW_CUDA_TRY(launch_early(k_block_update<T, 8>, grid, kUpdThreads, 0, s, X, B, Pn, HX, HB, HPn, Cm, m, nx, q, cols,
+                             pcols, np, n));
   count_launch();
   PW_CUDA_TRY(cudaGetLastError());
   return kOk;

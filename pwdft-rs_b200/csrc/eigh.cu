@@ -375,7 +375,7 @@ constexpr int kOneMaxReal = 128, kOneMaxCplx = 64;  // sizes of tridiag_one
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_eigh_cluster(const T* __restrict__ A, long lda, int m, int nev, int Ct, double gtol, double* __restrict__ w_out,
+    k_eigh_cluster(const T* A, long lda, int m, int nev, int Ct, double gtol, double* __restrict__ w_out,
                    T* __restrict__ Z, long ldz, double* __restrict__ work, int* __restrict__ status) {
   extern __shared__ __align__(16) unsigned char smem[];
   cg::cluster_group cluster = cg::this_cluster();
@@ -403,6 +403,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   EIGH_MARK(0);
   if (tid == 0) bad = 0;
+  launch_wait();
+  if (rank == 0 && tid == 0) *status = 0;  // cluster barriers lie between this and a CTA that sets it
   for (int e = tid; e < nown * m; e += kThreads) {
     const int sl = e / m, i = e - sl * m;
     a_loc[e] = A[(long)(rank + sl * Ct) * lda + i];
@@ -886,6 +888,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     T* sv = a_loc;
     const int waves = (nev + nw - 1) / nw;
     const int nchunk = (m - 1 + R - 1) / R;
+    launch_release();
     auto stage = [&](int c) {
       const int k0 = m - 2 - R * c;  // reflectors k0, k0 - 1, ..., k0 - R + 1
       const int lo = max(0, k0 - R + 2) & ~127;
@@ -1074,10 +1077,12 @@ Status launch_eigh(const T* A, long lda, int m, int nev, double* w, T* Z, long l
   Status r = set_attributes<T>();
   if (r != kOk) return r;
   auto kern = k_eigh_cluster<T>;
-  PW_CUDA_TRY(cudaMemsetAsync(status, 0, sizeof(int), s));
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   const int Ct = tridiag_ctas(m, C, (int)sizeof(T));
   cudaLaunchConfig_t cfg = launch_config<T>(m, C, Ct, attr, s);
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   // Eigenvalues closer than gtol ||T|| are orthonormalised as one group: inverse iteration leaves the others
   // orthogonal to eps / gtol.  Up to m = 64 the groups are few and short, and the wide tolerance keeps the vectors
   // within 1e-12 of orthonormal; above it the serial Gram-Schmidt of a wide group would dominate.

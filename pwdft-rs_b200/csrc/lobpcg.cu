@@ -121,11 +121,11 @@ __global__ void k_resid_precond(const S* __restrict__ X, const S* __restrict__ H
 // (narrow blocks: one launch instead of two).
 template <typename S>
 __global__ void __launch_bounds__(512)
-    k_resid_column(const S* __restrict__ X, const S* __restrict__ HX, S* __restrict__ T, long ld, int n,
-                   const double* __restrict__ lam, const double* __restrict__ kin, double v0,
-                   double* __restrict__ sumsq) {
+    k_resid_column(const S* X, const S* HX, S* __restrict__ T, long ld, int n, const double* lam,
+                   const double* __restrict__ kin, double v0, double* __restrict__ sumsq) {
   __shared__ double sh[32];
   const int col = blockIdx.x;
+  launch_wait();
   const double l = lam[col];
   const S* x = X + (long)col * ld;
   const S* hx = HX + (long)col * ld;
@@ -476,8 +476,8 @@ template <typename T> Status orthonormalize(Ctx& c, T* Y, int q) {
 
 // Lowest nev eigenpairs of the Hermitian subspace matrix Hs (m x m): values
 // into w.lam, vectors into *C (ld m).
-// defer: the caller reads w.status itself (only where the cluster solver runs).
-template <typename T> Status subspace_eig(Ctx& c, int m, int nev, T** C, bool defer = false) {
+// defer: the caller reads w.status itself, and the values go to lam (only where the cluster solver runs).
+template <typename T> Status subspace_eig(Ctx& c, int m, int nev, T** C, bool defer = false, double* lam = nullptr) {
   Status r;
   T* Hs = as<T>(c.w.Hs);
   if (eigh_cluster_supported(m, !std::is_same<T, double>::value)) {
@@ -491,7 +491,7 @@ template <typename T> Status subspace_eig(Ctx& c, int m, int nev, T** C, bool de
       c.w.eigh_work_len = need;
     }
     T* Cv = as<T>(c.w.Cs);
-    if ((r = eigh_cluster(Hs, m, m, nev, c.w.lam, Cv, m, c.w.eigh_work, c.w.status, c.s)) != kOk) return r;
+    if ((r = eigh_cluster(Hs, m, m, nev, lam ? lam : c.w.lam, Cv, m, c.w.eigh_work, c.w.status, c.s)) != kOk) return r;
     *C = Cv;
     if (defer) return kOk;
     int st = 0;
@@ -630,7 +630,7 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
   std::vector<double> rn(nd), nu0, nu1;
   std::vector<double> pack(steps ? 2 + 4 * (size_t)nd : 0);  // w.status, w.lam0 (3 nd), w.colsq
   bool dev_lam = false;  // the Ritz values of the last step are in w.lam0 only
-  std::vector<int> act, pband, keep, pk;
+  std::vector<int> act, pband, keep, pk, sel;
   int np = 0;  // columns of Pn / HPn (bands pband)
   out.iters = 0;
   PhaseTimer pt(h.trace);
@@ -639,7 +639,8 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
     pt.mark(0, s);
     if (!dev_lam) PW_CUDA_TRY(cudaMemcpyAsync(w.lam0, k.evals.data(), nd * sizeof(double), cudaMemcpyHostToDevice, s));
     if (steps) {
-      k_resid_column<T><<<nd, 512, 0, s>>>(X, HX, Tb, n, (int)n, w.lam0, kin, v0, w.colsq); count_launch();
+      PW_CUDA_TRY(launch_early(k_resid_column<T>, dim3(nd), 512, 0, s, X, HX, Tb, n, (int)n, w.lam0, kin, v0, w.colsq));
+      count_launch();
     } else {
       k_resid_precond<T><<<dim3(c.gx, nd), 256, 0, s>>>(X, HX, Tb, n, (int)n, w.lam0, kin, v0, w.partials);
       count_launch();
@@ -677,11 +678,23 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
     }
     T* W = X + n * nd;
     T* HW = HX + n * nd;
+    // P: previous directions of the bands still active
+    int npc = 0;
+    pk.clear();
+    for (int j = 0, a = 0; j < np; ++j) {
+      while (a < na && act[a] < pband[j]) ++a;
+      if (a < na && act[a] == pband[j]) pk.push_back(j);
+    }
+    if ((long)pk.size() > n - nd - na) pk.resize((size_t)std::max<long>(0, n - nd - na));
     pt.mark(1, s);
-    PW_CUDA_TRY(cudaMemcpyAsync(w.idx, act.data(), na * sizeof(int), cudaMemcpyHostToDevice, s));
     if (steps) {
+      // both column lists in one copy: the active bands, then the columns of P
+      sel.assign(act.begin(), act.end());
+      sel.insert(sel.end(), pk.begin(), pk.end());
+      PW_CUDA_TRY(cudaMemcpyAsync(w.idx, sel.data(), sel.size() * sizeof(int), cudaMemcpyHostToDevice, s));
       if ((r = block_w<T>(X, nd, Tb, w.idx, na, W, n, xch, bst, s)) != kOk) return r;
     } else {
+      PW_CUDA_TRY(cudaMemcpyAsync(w.idx, act.data(), na * sizeof(int), cudaMemcpyHostToDevice, s));
       k_gather_cols<T><<<dim3(c.gx, na), 256, 0, s>>>(Tb, n, w.idx, W, n, (int)n); count_launch();
       if ((r = project_out(c, (const T*)X, (const T*)nullptr, nd, W, (T*)nullptr, na)) != kOk) return r;
       if ((r = project_out(c, (const T*)X, (const T*)nullptr, nd, W, (T*)nullptr, na)) != kOk) return r;
@@ -691,20 +704,11 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
     if ((r = apply_op(h, spin, ik, W, n, na, HW, precision, s)) != kOk) return r;
     out.happ += na;
     pt.mark(3, s);
-    // P: previous directions of the bands still active
-    int npc = 0;
-    pk.clear();
-    for (int j = 0, a = 0; j < np; ++j) {
-      while (a < na && act[a] < pband[j]) ++a;
-      if (a < na && act[a] == pband[j]) pk.push_back(j);
-    }
-    if ((long)pk.size() > n - nd - na) pk.resize((size_t)std::max<long>(0, n - nd - na));
     T* P = W + n * na;
     T* HP = HW + n * na;
     if (!pk.empty() && steps) {
       npc = (int)pk.size();
-      PW_CUDA_TRY(cudaMemcpyAsync(w.idx, pk.data(), npc * sizeof(int), cudaMemcpyHostToDevice, s));
-      if ((r = block_p<T>(X, HX, nd + na, Pn, HPn, w.idx, npc, P, HP, n, p_drop, xch, bst, s)) != kOk) return r;
+      if ((r = block_p<T>(X, HX, nd + na, Pn, HPn, w.idx + na, npc, P, HP, n, p_drop, xch, bst, s)) != kOk) return r;
       PW_CUDA_TRY(cudaMemcpyAsync(&npc, bst + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
       PW_CUDA_TRY(cudaStreamSynchronize(s));
     } else if (!pk.empty()) {
@@ -757,7 +761,7 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
       const int ms = na + q;
       std::vector<double> lam_a(na);
       for (int j = 0; j < na; ++j) lam_a[j] = k.evals[act[j]];
-      PW_CUDA_TRY(cudaMemcpyAsync(w.idx, act.data(), na * sizeof(int), cudaMemcpyHostToDevice, s));
+      if (!steps) PW_CUDA_TRY(cudaMemcpyAsync(w.idx, act.data(), na * sizeof(int), cudaMemcpyHostToDevice, s));
       PW_CUDA_TRY(cudaMemcpyAsync(w.lam0, lam_a.data(), na * sizeof(double), cudaMemcpyHostToDevice, s));
       T* C = nullptr;
       if (steps) {
@@ -844,12 +848,10 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
         return r;
       first = false;
       pt.mark(5, s);
-      if ((r = subspace_eig<T>(c, m, nd, &C, true)) != kOk) return r;
+      if ((r = subspace_eig<T>(c, m, nd, &C, true, w.lam0)) != kOk) return r;
       pt.mark(6, s);
-      PW_CUDA_TRY(cudaMemcpyAsync(w.idx, act.data(), na * sizeof(int), cudaMemcpyHostToDevice, s));
       if ((r = block_update<T>(X, W, Pn, HX, HW, HPn, C, m, nd, q, nullptr, w.idx, na, n, s)) != kOk) return r;
       // values and status are read with the next residual norms
-      PW_CUDA_TRY(cudaMemcpyAsync(w.lam0, w.lam, nd * sizeof(double), cudaMemcpyDeviceToDevice, s));
       pt.mark(7, s);
       dev_lam = true;
       np = na;
