@@ -438,9 +438,8 @@ __global__ void __launch_bounds__(kT, 1)
 template <typename T, int NQ>
 __global__ void __launch_bounds__(kT, 1)
     k_block_p(const T* X, const T* HX, int nx, const T* __restrict__ Pn,
-              const T* __restrict__ HPn, const int* idx, int np, T* __restrict__ P,
-              T* __restrict__ HP, long n, int rpc, int ldy,
-              int ldz, int ldi, int staged, double p_drop, T* __restrict__ xch, long xch_len, int* __restrict__ status) {
+              const T* __restrict__ HPn, const int* idx, int np, T* P, T* HP, long n, int rpc, int ldy,
+              int ldz, int ldi, int staged, double p_drop, T* xch, long xch_len, int* status) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[kW];
   __shared__ double scol[kMaxBlock], nu0[kMaxBlock], rinv[kMaxBlock];
@@ -610,8 +609,7 @@ __global__ void __launch_bounds__(kT, 1)
 constexpr int kUpdThreads = 128;
 template <typename T, int NQ>
 __global__ void __launch_bounds__(kUpdThreads)
-    k_block_update(T* __restrict__ X, const T* __restrict__ B, T* __restrict__ Pn, T* __restrict__ HX,
-                   const T* __restrict__ HB, T* __restrict__ HPn, const T* Cm, int m, int nx, int q,
+    k_block_update(T* X, const T* __restrict__ B, T* Pn, T* HX, const T* __restrict__ HB, T* HPn, const T* Cm, int m, int nx, int q,
                    const int* __restrict__ cols, const int* __restrict__ pcols, int np, long n) {
   T* x = blockIdx.y ? HX : X;
   const T* b = blockIdx.y ? HB : B;
@@ -672,8 +670,7 @@ __global__ void __launch_bounds__(kUpdThreads)
 template <typename T, int NQ>
 __global__ void __launch_bounds__(kT, 1)
     k_block_nl(const T* __restrict__ B, int n_ch, const T* __restrict__ psi, long ldpsi, int nb_all, int bw,
-               T* __restrict__ hpsi,
-               long ldh, long n, int rpc, int ldz, int cap, T* __restrict__ xch, const int* __restrict__ ch_atom,
+               T* hpsi, long ldh, long n, int rpc, int ldz, int cap, T* xch, const int* __restrict__ ch_atom,
                const int* __restrict__ atom_ch_start, const int* __restrict__ d_off,
                const double* __restrict__ d_vals) {
   extern __shared__ __align__(16) unsigned char smem[];

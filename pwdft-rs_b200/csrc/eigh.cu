@@ -375,8 +375,8 @@ constexpr int kOneMaxReal = 128, kOneMaxCplx = 64;  // sizes of tridiag_one
 
 template <typename T>
 __global__ void __launch_bounds__(kThreads, 1)
-    k_eigh_cluster(const T* A, long lda, int m, int nev, int Ct, double gtol, double* __restrict__ w_out,
-                   T* __restrict__ Z, long ldz, double* __restrict__ work, int* __restrict__ status) {
+    k_eigh_cluster(const T* A, long lda, int m, int nev, int Ct, double gtol, double* w_out, T* Z, long ldz, double* work,
+                   int* status) {
   extern __shared__ __align__(16) unsigned char smem[];
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks();

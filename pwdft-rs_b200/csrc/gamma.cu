@@ -65,7 +65,7 @@ __global__ void k_unpack_pairs(const double* __restrict__ u, long ldu, int nb, d
 }
 
 // inverse of k_unpack_pairs for (H c): separate the two real bands and pack
-__global__ void k_pack_pairs(const double2* c, long ldc, int nb, double* __restrict__ u, long ldu,
+__global__ void k_pack_pairs(const double2* c, long ldc, int nb, double* u, long ldu,
                              const int* __restrict__ half_idx, const int* __restrict__ half_neg, int zero, int nh) {
   const int q = blockIdx.y;
   const int a = 2 * q, b = 2 * q + 1;

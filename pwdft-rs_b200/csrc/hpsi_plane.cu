@@ -50,7 +50,7 @@ constexpr int plane_threads(int x0, int x1) {
 // 216 0.484 / 0.262, 324 0.484 / 0.269, 432 0.590 / 0.285, 648 0.564 / 0.354 ms.
 template <typename R, int X0, int X1>
 __global__ void __launch_bounds__(plane_threads(X0, X1), sizeof(R) == 4 ? 3 : (X0 > 9 || X1 > 9 ? 1 : 2))
-    k_plane(cplx<R>* __restrict__ A, const R* __restrict__ vz, int nb, int bpc, int d2, PlaneGeo gin,
+    k_plane(cplx<R>* A, const R* __restrict__ vz, int nb, int bpc, int d2, PlaneGeo gin,
             const cplx<R>* __restrict__ twx, const cplx<R>* __restrict__ twy) {
   using C = cplx<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -204,7 +204,7 @@ constexpr int pair_id(int r0, int r1) { return r0 * 16 + r1; }
 
 template <typename R>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2)
-    k_plane_rt(cplx<R>* __restrict__ A, const R* __restrict__ vz, int nb, int bpc, int d2, PlaneGeo gin, int rows,
+    k_plane_rt(cplx<R>* A, const R* __restrict__ vz, int nb, int bpc, int d2, PlaneGeo gin, int rows,
                int px, int py, const cplx<R>* __restrict__ twx, const cplx<R>* __restrict__ twy) {
   using C = cplx<R>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2)
 // points col_start[c] .. col_start[c + 1] - 1 at consecutive n2 from col_lo[c].
 template <typename R, int Z0, int Z1>
 __global__ void __launch_bounds__(kZCols * (Z0 > Z1 ? Z0 : Z1))
-    k_zi(const double2* psi, long ldpsi, cplx<R>* __restrict__ A, const int* __restrict__ col_start,
+    k_zi(const double2* psi, long ldpsi, cplx<R>* A, const int* __restrict__ col_start,
          const int* __restrict__ col_lo, int ncol, int m2, const cplx<R>* __restrict__ tw) {
   using C = cplx<R>;
   constexpr int d2 = Z0 * Z1, ld = d2 | 1;
@@ -306,8 +306,8 @@ __global__ void __launch_bounds__(kZCols * (Z0 > Z1 ? Z0 : Z1))
 // K5: z-forward of kZCols columns, Hpsi = value / N + T psi at the sphere points.
 template <typename R, int Z0, int Z1>
 __global__ void __launch_bounds__(kZCols * (Z0 > Z1 ? Z0 : Z1))
-    k_zf(const cplx<R>* A, const double2* __restrict__ psi, long ldpsi, double2* __restrict__ hpsi,
-         long ldh, const double* __restrict__ kin, double scale, const int* __restrict__ col_start,
+    k_zf(const cplx<R>* A, const double2* __restrict__ psi, long ldpsi, double2* hpsi, long ldh,
+         const double* __restrict__ kin, double scale, const int* __restrict__ col_start,
          const int* __restrict__ col_lo, int ncol, int m2, const cplx<R>* __restrict__ tw) {
   using C = cplx<R>;
   constexpr int d2 = Z0 * Z1, ld = d2 | 1;

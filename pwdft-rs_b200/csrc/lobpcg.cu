@@ -121,8 +121,8 @@ __global__ void k_resid_precond(const S* __restrict__ X, const S* __restrict__ H
 // (narrow blocks: one launch instead of two).
 template <typename S>
 __global__ void __launch_bounds__(512)
-    k_resid_column(const S* X, const S* HX, S* __restrict__ T, long ld, int n, const double* lam,
-                   const double* __restrict__ kin, double v0, double* __restrict__ sumsq) {
+    k_resid_column(const S* X, const S* HX, S* T, long ld, int n, const double* lam,
+                   const double* __restrict__ kin, double v0, double* sumsq) {
   __shared__ double sh[32];
   const int col = blockIdx.x;
   launch_wait();

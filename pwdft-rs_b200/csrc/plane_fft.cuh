@@ -124,7 +124,7 @@ struct PlaneGeo {
 
 // y-inverse, stage A: Xp compact lines of Ab ([p][q], q the sphere row) into the scratch rows
 template <int Y0, int Y1, typename C>
-__device__ __forceinline__ void plane_ya(const C* __restrict__ Ab, C* P, const PlaneGeo& g, const C* TY, int tid, int T) {
+__device__ __forceinline__ void plane_ya(const C* Ab, C* P, const PlaneGeo& g, const C* TY, int tid, int T) {
   for (int t = tid; t < g.Xp * Y1; t += T) {
     const int p = t / Y1, j = t - p * Y1;
     C v[Y0];
@@ -244,7 +244,7 @@ __device__ __forceinline__ void plane_yc(C* P, const PlaneGeo& g, const C* TY, i
 
 // y-forward, stage D: scratch rows -> the sphere rows of Ab
 template <int Y0, int Y1, typename C>
-__device__ __forceinline__ void plane_yd(C* __restrict__ Ab, const C* P, const PlaneGeo& g, int tid, int T) {
+__device__ __forceinline__ void plane_yd(C* Ab, const C* P, const PlaneGeo& g, int tid, int T) {
   for (int t = tid; t < g.Xp * Y1; t += T) {
     const int p = t / Y1, m = t - p * Y1;
     const C* row = P + g.srow(p) * g.ld + m;

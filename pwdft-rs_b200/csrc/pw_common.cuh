@@ -41,8 +41,10 @@ template <int S, typename C> __host__ __device__ __forceinline__ C mul_si(C a) {
 
 // Programmatic launch: a kernel started by launch_early() may begin while its predecessor in the stream still runs.
 // launch_wait(): the predecessor has completed and its writes are visible.  launch_release(): the successor may begin.
-// A kernel that releases does so after its own wait, so whatever ran before the predecessor has completed by then.  Data
-// of the predecessor is read through pointers without __restrict__, so that no load moves above the wait.
+// A kernel that releases does so after its own wait, so whatever ran before the predecessor has completed by then.
+// What the predecessor writes, and every output, goes through pointers without __restrict__: a compiler may move an
+// access through a __restrict__ argument across the wait, since nothing else is said to reach its memory.  Only inputs
+// that are complete before the predecessor begins (tables, V(r), blocks of earlier launches) keep the qualifier.
 // What it saves is the 2 to 3 us between two dependent launches: H|psi> of 2 Si atoms (10 bands, four launches) 24.6 ->
 // 14.8 us, of 8 C atoms mixed 26.6 -> 18.9, of 8 Si atoms (28 bands, 40^3) 51 -> 42, 160 bands on 72^3 1268 -> 1235 us.
 __device__ __forceinline__ void launch_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
