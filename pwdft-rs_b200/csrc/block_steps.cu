@@ -606,11 +606,13 @@ __global__ void __launch_bounds__(kT, 1)
 
 // Update of V = X (blockIdx.y 0) and of HV (1) over 8-row strips, one warp each: T = B C_b (C's rows nx .. nx + q - 1),
 // Pn(:, t) = T(:, pcols[t]), X(:, cols) <- X(:, cols) C_x + T in place (a strip is read whole before it is written).
+// Nothing is written when the eigensolve or W of this step failed (status[0], status[1]): the host reads the status a step
+// late, and a failed step leaves the bands as they were.
 constexpr int kUpdThreads = 128;
 template <typename T, int NQ>
 __global__ void __launch_bounds__(kUpdThreads)
     k_block_update(T* X, const T* __restrict__ B, T* Pn, T* HX, const T* __restrict__ HB, T* HPn, const T* Cm, int m, int nx, int q,
-                   const int* __restrict__ cols, const int* __restrict__ pcols, int np, long n) {
+                   const int* __restrict__ cols, const int* __restrict__ pcols, int np, long n, const int* status) {
   T* x = blockIdx.y ? HX : X;
   const T* b = blockIdx.y ? HB : B;
   T* pn = blockIdx.y ? HPn : Pn;
@@ -625,6 +627,7 @@ __global__ void __launch_bounds__(kUpdThreads)
   __syncthreads();
   launch_wait();
   launch_release();
+  if (status[0] != 0 || status[1] != 0) return;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kr = lane & 3, kc = lane >> 2;
   const long i = ((long)blockIdx.x * (kUpdThreads / 32) + warp) * 8 + kc;
@@ -861,14 +864,14 @@ Status block_rr(const T* B, const T* HB, int q, const T* HX, const int* cols, in
 
 template <typename T>
 Status block_update(T* X, const T* B, T* Pn, T* HX, const T* HB, T* HPn, const T* Cm, int m, int nx, int q,
-                    const int* cols, const int* pcols, int np, long n, cudaStream_t s) {
+                    const int* cols, const int* pcols, int np, long n, const int* status, cudaStream_t s) {
   const dim3 grid((unsigned)((n + 8 * (kUpdThreads / 32) - 1) / (8 * (kUpdThreads / 32))), 2);
   if (nx <= 32)
     PW_CUDA_TRY(launch_early(k_block_update<T, 4>, grid, kUpdThreads, 0, s, X, B, Pn, HX, HB, HPn, Cm, m, nx, q, cols,
-                             pcols, np, n));
+                             pcols, np, n, status));
   else
     PW_CUDA_TRY(launch_early(k_block_update<T, 8>, grid, kUpdThreads, 0, s, X, B, Pn, HX, HB, HPn, Cm, m, nx, q, cols,
-                             pcols, np, n));
+                             pcols, np, n, status));
   count_launch();
   PW_CUDA_TRY(cudaGetLastError());
   return kOk;
@@ -924,7 +927,7 @@ Status nl_fused(Handle& h, const T* B, const T* psi, long ldpsi, int nb, T* hpsi
   template Status block_rr<T>(const T*, const T*, int, const T*, const int*, int, const double*, const T*, long,     \
                               T*, T*, cudaStream_t);                                                                 \
   template Status block_update<T>(T*, const T*, T*, T*, const T*, T*, const T*, int, int, int, const int*,           \
-                                  const int*, int, long, cudaStream_t);
+                                  const int*, int, long, const int*, cudaStream_t);
 PW_BLOCK(double)
 PW_BLOCK(double2)
 #undef PW_BLOCK

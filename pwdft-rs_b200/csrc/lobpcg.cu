@@ -769,7 +769,7 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
         pt.mark(5, s);
         if ((r = subspace_eig<T>(c, ms, na, &C)) != kOk) return r;
         pt.mark(6, s);
-        if ((r = block_update<T>(X, W, Pn, HX, HW, HPn, C, ms, na, q, w.idx, nullptr, na, n, s)) != kOk) return r;
+        if ((r = block_update<T>(X, W, Pn, HX, HW, HPn, C, ms, na, q, w.idx, nullptr, na, n, w.status, s)) != kOk) return r;
       } else {
         T* Bx = Tb;                      // [X_a | W | P], n x ms
         T* Bh = as<T>(w.HXn);            // [HX_a | HW | HP]
@@ -850,7 +850,7 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
       pt.mark(5, s);
       if ((r = subspace_eig<T>(c, m, nd, &C, true, w.lam0)) != kOk) return r;
       pt.mark(6, s);
-      if ((r = block_update<T>(X, W, Pn, HX, HW, HPn, C, m, nd, q, nullptr, w.idx, na, n, s)) != kOk) return r;
+      if ((r = block_update<T>(X, W, Pn, HX, HW, HPn, C, m, nd, q, nullptr, w.idx, na, n, w.status, s)) != kOk) return r;
       // values and status are read with the next residual norms
       pt.mark(7, s);
       dev_lam = true;

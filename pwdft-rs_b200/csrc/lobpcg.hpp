@@ -85,9 +85,10 @@ Status block_p(const T* X, const T* HX, int nx, const T* Pn, const T* HPn, const
 template <typename T>
 Status block_rr(const T* B, const T* HB, int q, const T* HX, const int* cols, int nx, const double* lam, const T* XX,
                 long n, T* xch, T* Hs, cudaStream_t s);
-// X(:, cols) and Pn from the subspace eigenvectors Cm (m x nx), and the same for HX, HPn.
+// X(:, cols) and Pn from the subspace eigenvectors Cm (m x nx), and the same for HX, HPn; nothing when status[0] or
+// status[1] (EigWork::status) tells that the step failed.
 template <typename T>
 Status block_update(T* X, const T* B, T* Pn, T* HX, const T* HB, T* HPn, const T* Cm, int m, int nx, int q,
-                    const int* cols, const int* pcols, int np, long n, cudaStream_t s);
+                    const int* cols, const int* pcols, int np, long n, const int* status, cudaStream_t s);
 
 }  // namespace pwgpu

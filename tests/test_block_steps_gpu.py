@@ -13,7 +13,7 @@ from conftest import rng
 from oracle import pwdft_oracle as O
 from pwgpu.context import build_system
 from pwgpu.crystal import KPoint, diamond_primitive, diamond_supercell, gamma_only
-from pwgpu.lib import PwGpu
+from pwgpu.lib import PRECISION_MIXED, PwGpu, PwGpuError
 from pwgpu.symmetry import SymmetryInfo
 
 pytestmark = pytest.mark.gpu
@@ -59,3 +59,20 @@ def test_few_plane_waves(ecut, bands, si_pp):
     """Rows for one or two CTAs only, and blocks close to the whole space."""
     s = build_system(diamond_primitive("Si", 5.431), {"Si": si_pp}, ecut, [KPoint(np.array([0.05, 0.1, -0.2]), 1.0)])
     _check(s, bands)
+
+
+@pytest.mark.parametrize("gamma_complex", [True, False])
+def test_failed_step_keeps_the_bands(gamma_complex, si_pp):
+    """A potential beyond the range of FP32 makes H W of the mixed form non-finite: the step fails, and the bands left
+    on the device are the orthonormal ones from before it."""
+    s = build_system(diamond_primitive("Si", 5.431), {"Si": si_pp}, 190.0, gamma_only(), SymmetryInfo.identity_only())
+    veff = np.zeros(s.n_grid, dtype=np.complex128)
+    veff[0] = 1e39
+    with PwGpu(s, precision=PRECISION_MIXED, gamma_complex=gamma_complex) as dev:
+        dev.set_veff_g(veff)
+        with pytest.raises(PwGpuError, match="non-finite"):
+            dev.eigensolve(5, tol=1e-7, max_iter=4)
+        psi = dev.get_bands(5)
+        assert np.max(np.abs(psi.conj().T @ psi - np.eye(5))) < 1e-11
+        dev.set_veff_g(_veff(s))
+        assert dev.eigensolve(5, tol=1e-6, max_iter=200)[3] < 1e-6
