@@ -475,11 +475,12 @@ template <typename T> Status orthonormalize(Ctx& c, T* Y, int q) {
 }
 
 // Lowest nev eigenpairs of the Hermitian subspace matrix Hs (m x m): values
-// into w.lam, vectors into *C (ld m).
-// defer: the caller reads w.status itself, and the values go to lam (only where the cluster solver runs).
+// into lam (w.lam when NULL), vectors into *C (ld m).
+// defer: the caller reads w.status itself (the cluster solver's; the fallback has no status to defer).
 template <typename T> Status subspace_eig(Ctx& c, int m, int nev, T** C, bool defer = false, double* lam = nullptr) {
   Status r;
   T* Hs = as<T>(c.w.Hs);
+  if (!lam) lam = c.w.lam;
   if (eigh_cluster_supported(m, !std::is_same<T, double>::value)) {
     // this project's cluster eigensolver: lowest nev pairs, vectors into Cs
     const size_t need = eigh_cluster_work_doubles(m, nev);
@@ -491,7 +492,7 @@ template <typename T> Status subspace_eig(Ctx& c, int m, int nev, T** C, bool de
       c.w.eigh_work_len = need;
     }
     T* Cv = as<T>(c.w.Cs);
-    if ((r = eigh_cluster(Hs, m, m, nev, lam ? lam : c.w.lam, Cv, m, c.w.eigh_work, c.w.status, c.s)) != kOk) return r;
+    if ((r = eigh_cluster(Hs, m, m, nev, lam, Cv, m, c.w.eigh_work, c.w.status, c.s)) != kOk) return r;
     *C = Cv;
     if (defer) return kOk;
     int st = 0;
@@ -502,7 +503,7 @@ template <typename T> Status subspace_eig(Ctx& c, int m, int nev, T** C, bool de
   }
   // beyond the cluster solver's size (m > 544, or complex m beyond its shared memory)
   if ((r = ensure_solver(c)) != kOk) return r;
-  if ((r = heevd(c, Hs, m, c.w.lam)) != kOk) return r;
+  if ((r = heevd(c, Hs, m, lam)) != kOk) return r;
   int info = 0;
   PW_CUDA_TRY(cudaMemcpyAsync(&info, c.w.info, sizeof(int), cudaMemcpyDeviceToHost, c.s));
   PW_CUDA_TRY(cudaStreamSynchronize(c.s));
