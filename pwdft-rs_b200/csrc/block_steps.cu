@@ -811,6 +811,21 @@ template <typename T> bool block_steps_fit(long n, int nd) {
   return configure<T>(&fits) == kOk && fits;
 }
 
+// One cluster of 16 SMs against library products on the whole GPU: the
+// products of a step are ~n m^2 (m the columns of [X | W | P]), its serial
+// part (Cholesky, inverse) ~m^2, the library's cost mostly its launches.  One
+// step with every band active (m = 3 nd), library / fused in us, B200: real
+// 1,045 rows nd 48 1220 / 980, 60 1390 / 1400; 2,517 rows nd 45 1200 / 1120,
+// 56 1400 / 1530; 3,431 rows nd 40 940 / 830, 56 1450 / 1670; 6,187 rows nd 32
+// 825 / 700, 40 980 / 1060; 22,119 rows nd 16 727 / 623; complex 1,045 rows
+// nd 40 1210 / 1020; 2,517 rows nd 32 1040 / 910, 40 1180 / 1280; 6,187 rows nd
+// 24 1030 / 860, 28 1090 / 1110.  Narrow blocks keep their gain in large boxes:
+// 61,037 rows real nd 4 722 / 520, complex nd 3 960 / 642.
+template <typename T> bool block_step_gains(long n, int m) {
+  const double most = sizeof(T) == sizeof(double) ? 35e3 : 20e3;
+  return (double)m * m * (1.0 + n / 3000.0) <= most;
+}
+
 size_t block_steps_xch(int nd) {
   // two buffers of (2 nd + 1) x nd, or one of 2 nd x 3 nd, per CTA and for the total
   return (size_t)(kMaxC + 1) * std::max<size_t>(2 * (size_t)(2 * nd + 1) * nd, (size_t)6 * nd * nd);
@@ -921,6 +936,7 @@ Status nl_fused(Handle& h, const T* B, const T* psi, long ldpsi, int nb, T* hpsi
   template bool nl_fused_ok<T>(const Handle&, int);                                                                 \
   template Status nl_fused<T>(Handle&, const T*, const T*, long, int, T*, long, cudaStream_t);                       \
   template bool block_steps_fit<T>(long, int);                                                                      \
+  template bool block_step_gains<T>(long, int);                                                                     \
   template Status block_w<T>(const T*, int, const T*, const int*, int, T*, long, T*, int*, cudaStream_t);            \
   template Status block_p<T>(const T*, const T*, int, const T*, const T*, const int*, int, T*, T*, long, double, T*, \
                              int*, cudaStream_t);                                                                   \

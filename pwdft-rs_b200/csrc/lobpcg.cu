@@ -598,8 +598,8 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
     PW_CUDA_TRY(cudaStreamSynchronize(s));
     k.init = true;
   }
-  // narrow blocks take the fused block steps (block_steps.cu): one launch each for W, P, the subspace
-  // matrix and the update
+  // narrow blocks take the fused block steps (block_steps.cu), one launch each for W, P, the subspace
+  // matrix and the update, wherever these are faster than the library's
   const bool steps = block_steps_fit<T>(n, nd);
   T* xch = as<T>(w.xch);
   int* bst = w.status + 1;
@@ -687,8 +687,9 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
       if (a < na && act[a] == pband[j]) pk.push_back(j);
     }
     if ((long)pk.size() > n - nd - na) pk.resize((size_t)std::max<long>(0, n - nd - na));
+    const bool fused = steps && block_step_gains<T>(n, nd + na + (int)pk.size());
     pt.mark(1, s);
-    if (steps) {
+    if (fused) {
       // both column lists in one copy: the active bands, then the columns of P
       sel.assign(act.begin(), act.end());
       sel.insert(sel.end(), pk.begin(), pk.end());
@@ -707,7 +708,7 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
     pt.mark(3, s);
     T* P = W + n * na;
     T* HP = HW + n * na;
-    if (!pk.empty() && steps) {
+    if (!pk.empty() && fused) {
       npc = (int)pk.size();
       if ((r = block_p<T>(X, HX, nd + na, Pn, HPn, w.idx + na, npc, P, HP, n, p_drop, xch, bst, s)) != kOk) return r;
       PW_CUDA_TRY(cudaMemcpyAsync(&npc, bst + 1, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -762,10 +763,10 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
       const int ms = na + q;
       std::vector<double> lam_a(na);
       for (int j = 0; j < na; ++j) lam_a[j] = k.evals[act[j]];
-      if (!steps) PW_CUDA_TRY(cudaMemcpyAsync(w.idx, act.data(), na * sizeof(int), cudaMemcpyHostToDevice, s));
+      if (!fused) PW_CUDA_TRY(cudaMemcpyAsync(w.idx, act.data(), na * sizeof(int), cudaMemcpyHostToDevice, s));
       PW_CUDA_TRY(cudaMemcpyAsync(w.lam0, lam_a.data(), na * sizeof(double), cudaMemcpyHostToDevice, s));
       T* C = nullptr;
-      if (steps) {
+      if (fused) {
         if ((r = block_rr<T>(W, HW, q, HX, w.idx, na, w.lam0, nullptr, n, xch, as<T>(w.Hs), s)) != kOk) return r;
         pt.mark(5, s);
         if ((r = subspace_eig<T>(c, ms, na, &C)) != kOk) return r;
@@ -844,7 +845,7 @@ Status lobpcg_t(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, 
     pt.mark(4, s);
     const int m = nd + q;
     T* C = nullptr;
-    if (steps) {
+    if (fused) {
       if ((r = block_rr<T>(W, HW, q, HX, nullptr, nd, w.lam0, first ? XX : nullptr, n, xch, as<T>(w.Hs), s)) != kOk)
         return r;
       first = false;

@@ -70,6 +70,8 @@ Status lobpcg(Handle& h, EigWork& w, EigVecs& k, int spin, int ik, double v0, do
 // block_steps_fit: whether a block of nd columns of n rows takes them.
 constexpr int kMaxBlock = 64;
 template <typename T> bool block_steps_fit(long n, int nd);
+// block_step_gains: whether a step over a subspace of m columns is the faster one in these launches.
+template <typename T> bool block_step_gains(long n, int m);
 size_t block_steps_xch(int nd);  // entries of T in the exchange buffer
 // W (n x na) = orthonormal basis of Tb(:, idx) outside span(X) (idx NULL: columns in order; nd 0: no projection, W
 // may be Tb); status[0] = 1 when rank deficient.
