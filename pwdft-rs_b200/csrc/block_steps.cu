@@ -893,17 +893,25 @@ Status block_update(T* X, const T* B, T* Pn, T* HX, const T* HB, T* HPn, const T
 }
 
 // One launch is the faster form while the products are small: the clusters'
-// tile products reach a fraction of the library products' rate.  H|psi> in
-// one launch against library products, by n_pw x channels x bands (complex,
-// FP64): 725 x 10 x 12 26 us against 35, 1647 x 40 x 28 36 against 50,
-// 3791 x 40 x 28 (4.2e6) 51 against 60, 3423 x 32 x 70 (7.7e6) 86 against 92;
-// but 3301 x 80 x 20 (5.3e6) 64 against 55 and 4573 x 80 x 40 (1.5e7) 106
-// against 91.  A real multiply-add is a quarter of a complex one; three times
-// the limit is where the real form has been measured to gain (3791 x 40 x 22).
-constexpr double kNlFusedWork = 5e6;
+// tile products reach a fraction of the library products' rate, and each
+// cluster reads all of B (n_ch columns) and its share of psi and H psi with 16
+// SMs.  H|psi> in library / fused form, us, B200, by n_pw x channels x bands
+// (complex): 1045 x 40 x 28 39 / 22, 1743 x 80 x 8 1.44 times as fast, 6187 x
+// 24 x 16 1.16, 10059 x 8 x 16 62 / 53, 10059 x 16 x 28 88 / 84, 15419 x 4 x
+// 16 1.13; but 2517 x 80 x 16 42 / 45, 6187 x 80 x 1 43 / 66, 12533 x 16 x 1
+// 0.89, 10059 x 40 x 4 49 / 59, 22119 x 8 x 4 56 / 59, 76957 x 4 x 1 44 / 91.
+// Packed real (a real entry is half the bytes, a multiply-add a quarter):
+// 10059 x 40 x 16 72 / 60, 6187 x 80 x 16 71 / 65, 15419 x 16 x 28 74 / 72;
+// but 15419 x 40 x 1 66 / 71, 22119 x 16 x 16 73 / 82, 10059 x 4 x 57 91 / 97,
+// 6187 x 40 x 57 74 / 79.
 template <typename T> bool nl_fused_ok(const Handle& h, int nb) {
-  const double work = (double)h.n_pw * h.n_ch * nb;
-  if (h.n_ch < 1 || work > (sizeof(T) == sizeof(double) ? 3.0 : 1.0) * kNlFusedWork) return false;
+  const double n = (double)h.n_pw, nc = (double)h.n_ch;
+  if (h.n_ch < 1) return false;
+  if (sizeof(T) == sizeof(double)) {
+    if (n * nc * nb > 1.2e7 || n * (nc + 16) > 6e5 || n * nb > 4.4e5) return false;
+  } else {
+    if (n * nc * nb > 5e6 || n * (nc + 16) > 3.3e5 || n * nc > 1.95e5) return false;
+  }
   if ((size_t)2 * pad_ld(h.n_ch) * nl_group(nb) * sizeof(T) > kSmemMax) return false;
   bool fits = false;
   return configure<T>(&fits) == kOk && fits;

@@ -175,8 +175,8 @@ Status local_plane(Handle& h, int spin, int ik, const double2* psi, long ldpsi, 
 Status nonlocal_pq(Handle& h, int ik, const double2* psi, long ldpsi, int nb, cudaStream_t s,
                    StageTimer* tm = nullptr);
 
-// hpsi += B D B^H psi in one launch, for products small enough for one cluster
-// (block_steps.cu); B n_pw x n_ch, T = double (packed real) or double2.
+// hpsi += B D B^H psi in one launch of up to eight clusters, for products small
+// enough (block_steps.cu); B n_pw x n_ch, T = double (packed real) or double2.
 template <typename T> bool nl_fused_ok(const Handle& h, int nb);
 template <typename T>
 Status nl_fused(Handle& h, const T* B, const T* psi, long ldpsi, int nb, T* hpsi, long ldh, cudaStream_t s);
