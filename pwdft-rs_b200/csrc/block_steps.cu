@@ -917,18 +917,31 @@ template <typename T> bool nl_fused_ok(const Handle& h, int nb) {
   return configure<T>(&fits) == kOk && fits;
 }
 
+// Room in the exchange buffer for nb bands (more bands never need less).
+template <typename T> static Status ensure_nl_xch(Handle& h, int nb) {
+  const int bw = nl_group(nb), clusters = (nb + bw - 1) / bw;
+  const size_t need = (size_t)clusters * (kMaxC + 1) * h.n_ch * bw * sizeof(T);
+  if (need <= h.nl_xch_bytes) return kOk;
+  if (h.nl_xch) cudaFree(h.nl_xch);
+  h.nl_xch = nullptr;
+  h.nl_xch_bytes = 0;
+  cudaError_t e = cudaMalloc(&h.nl_xch, need);
+  if (e != cudaSuccess) return fail(kOom, std::string("cudaMalloc (projector exchange): ") + cudaGetErrorString(e));
+  h.nl_xch_bytes = need;
+  return kOk;
+}
+
+template <typename T> Status nl_fused_reserve(Handle& h, int nb) {
+  if (!nl_fused_ok<T>(h, 1)) return kOk;
+  while (!nl_fused_ok<T>(h, nb)) --nb;
+  return ensure_nl_xch<T>(h, nb);
+}
+
 template <typename T>
 Status nl_fused(Handle& h, const T* B, const T* psi, long ldpsi, int nb, T* hpsi, long ldh, cudaStream_t s) {
   const int bw = nl_group(nb), clusters = (nb + bw - 1) / bw;
-  const size_t need = (size_t)clusters * (kMaxC + 1) * h.n_ch * bw * sizeof(T);
-  if (need > h.nl_xch_bytes) {
-    if (h.nl_xch) cudaFree(h.nl_xch);
-    h.nl_xch = nullptr;
-    h.nl_xch_bytes = 0;
-    cudaError_t e = cudaMalloc(&h.nl_xch, need);
-    if (e != cudaSuccess) return fail(kOom, std::string("cudaMalloc (projector exchange): ") + cudaGetErrorString(e));
-    h.nl_xch_bytes = need;
-  }
+  const Status st = ensure_nl_xch<T>(h, nb);
+  if (st != kOk) return st;
   int C, rpc;
   split_rows(h.n_pw, C, rpc);
   const int ldz = pad_ld(h.n_ch);
@@ -942,6 +955,7 @@ Status nl_fused(Handle& h, const T* B, const T* psi, long ldpsi, int nb, T* hpsi
 
 #define PW_BLOCK(T)                                                                                                  \
   template bool nl_fused_ok<T>(const Handle&, int);                                                                 \
+  template Status nl_fused_reserve<T>(Handle&, int);                                                                \
   template Status nl_fused<T>(Handle&, const T*, const T*, long, int, T*, long, cudaStream_t);                       \
   template bool block_steps_fit<T>(long, int);                                                                      \
   template bool block_step_gains<T>(long, int);                                                                     \

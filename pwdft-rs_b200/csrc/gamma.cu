@@ -354,7 +354,7 @@ Status ensure_gamma_pq(Handle& h, int nb) {
   if ((r = galloc(&h.gam_p, (size_t)h.n_ch * nb)) != kOk) return r;
   if ((r = galloc(&h.gam_q, (size_t)h.n_ch * nb)) != kOk) return r;
   h.gam_pcap = nb;
-  return kOk;
+  return nl_fused_reserve<double>(h, nb);
 }
 
 Status apply_d_real(Handle& h, int nb, cudaStream_t s) {

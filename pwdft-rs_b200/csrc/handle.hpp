@@ -178,6 +178,8 @@ Status nonlocal_pq(Handle& h, int ik, const double2* psi, long ldpsi, int nb, cu
 // hpsi += B D B^H psi in one launch of up to eight clusters, for products small
 // enough (block_steps.cu); B n_pw x n_ch, T = double (packed real) or double2.
 template <typename T> bool nl_fused_ok(const Handle& h, int nb);
+// The exchange buffer of the widest block up to nb bands that takes it.
+template <typename T> Status nl_fused_reserve(Handle& h, int nb);
 template <typename T>
 Status nl_fused(Handle& h, const T* B, const T* psi, long ldpsi, int nb, T* hpsi, long ldh, cudaStream_t s);
 

@@ -1024,7 +1024,8 @@ Status ensure_nl_capacity(Handle& h, int nb) {
   if ((st = dalloc(&h.nl_p, (size_t)std::max(1, h.n_ch) * nb)) != kOk) return st;
   if ((st = dalloc(&h.nl_q, (size_t)std::max(1, h.n_ch) * nb)) != kOk) return st;
   h.nl_cap = nb;
-  return kOk;
+  // narrower blocks may take the one-launch form: only a call with the most bands so far allocates
+  return nl_fused_reserve<double2>(h, nb);
 }
 
 Status fft3d_full(Handle& h, double2* data, int sign, cudaStream_t stream) {

@@ -85,3 +85,27 @@ def test_dependent_calls_without_waits(nb, si_pp):
             torch.cuda.synchronize()
             out.append(a.cpu().numpy())
     assert np.array_equal(out[0], out[1])
+
+
+def test_capture_of_a_narrower_block(si_pp):
+    """After one call with a wide block (library products) a narrower one, which takes the one-launch term, can be
+    captured: it allocates nothing."""
+    import torch
+
+    s = build_system(diamond_primitive("Si", 5.431), {"Si": si_pp}, 260.0, [KPoint(np.array([0.11, -0.23, 0.31]), 1.0)])
+    wide, nb = 6_000_000 // (s.n_pw * s.projectors[0].n_ch) + 1, 8
+    g = rng(7)
+    psi = torch.from_numpy(g.standard_normal((wide, s.n_pw)) + 1j * g.standard_normal((wide, s.n_pw))).cuda()
+    out, ref = torch.zeros_like(psi), torch.zeros_like(psi)
+    with PwGpu(s) as dev:
+        dev.set_veff_g(_veff(s))
+        dev.apply_h_device(psi.data_ptr(), s.n_pw, wide, ref.data_ptr(), s.n_pw)
+        torch.cuda.synchronize()
+        graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=side):
+            dev.apply_h_device(psi.data_ptr(), s.n_pw, nb, out.data_ptr(), s.n_pw, stream=side.cuda_stream)
+        graph.replay()
+        torch.cuda.synchronize()
+        scale = float(ref.abs().max())
+        assert float((out[:nb] - ref[:nb]).abs().max()) < 1e-12 * scale
+        del graph
