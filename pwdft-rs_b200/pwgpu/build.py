@@ -19,13 +19,14 @@ INCLUDE = os.path.join(os.path.dirname(PKG_ROOT), "include")
 LIBDIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIBDIR, "libpwgpu.so")
 
-SOURCES = ["api.cu", "hpsi.cu", "hpsi_plane.cu", "linalg.cu", "lobpcg.cu", "block_steps.cu", "scf.cu", "noalloc.cu", "gemm_bf16.cu", "nl_mixed.cu", "server.cu", "gamma.cu", "setup.cu", "components.cu", "eigh.cu", "chol.cu", "upf.cu", "deck.cu"]
+SOURCES = ["api.cu", "hpsi.cu", "hpsi_plane.cu", "plane_rt.cu", "plane_len_a.cu", "plane_len_b.cu", "plane_len_c.cu", "plane_len_d.cu", "plane_len_e.cu", "linalg.cu", "lobpcg.cu", "block_steps.cu", "scf.cu", "noalloc.cu", "gemm_bf16.cu", "nl_mixed.cu", "server.cu", "gamma.cu", "setup.cu", "components.cu", "eigh.cu", "chol.cu", "upf.cu", "deck.cu"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
     "--expt-relaxed-constexpr", "-diag-suppress", "20012",
+    "-Xfatbin", "-compress-all",  # 16 MB of library against 38, 6 ms more until a process's first H|psi>
 ]
 
 
