@@ -91,3 +91,18 @@ def test_wide_blocks_of_many_rows(gamma, ecut, bands, si_pp):
     m = 3 * (bands + bands // 8)
     assert m * m * (1.0 + s.n_pw / 3000.0) > (35e3 if gamma else 20e3) > (m / 3 + 10) ** 2 * (1.0 + s.n_pw / 3000.0)
     _check(s, bands)
+
+
+@pytest.mark.parametrize("gamma", [True, False])
+def test_long_solves_stay_orthonormal(gamma, si_pp):
+    """X is rotated, not orthonormalised again, through a solve: some 20 steps at tolerance 1e-10 eV."""
+    if gamma:
+        cr = diamond_supercell("Si", 5.431, (1, 1, 1), 0.02, rng(5))
+        s = build_system(cr, {"Si": si_pp}, 190.0, gamma_only(), SymmetryInfo.identity_only())
+    else:
+        s = build_system(diamond_primitive("Si", 5.431), {"Si": si_pp}, 520.0, [KPoint(np.array([0.11, -0.23, 0.31]), 1.0)])
+    with PwGpu(s) as dev:
+        dev.set_veff_g(_veff(s))
+        _, psi, its, res = dev.eigensolve(3, tol=1e-10, max_iter=800)
+    assert res < 1e-10 and its >= 15
+    assert np.max(np.abs(psi.conj().T @ psi - np.eye(3))) < 1e-11

@@ -1,7 +1,8 @@
 """The subspace eigensolver at the edges of its one-CTA reduction: one, two and
 four rows a lane (m = 32, 64, 128 real; 32, 64 complex) and the first sizes
-past them, against LAPACK at the bars of the other eigensolver tests (1e-12
-||A||), on spread, repeated and graded spectra."""
+past them, against LAPACK: eigenvalues to 1e-12 ||A||, residuals to 1e-11
+||A||, vectors orthonormal to 1e-12 up to m = 64 (the wider Gram-Schmidt
+groups) and 1e-11 above, on spread, repeated and graded spectra."""
 
 import numpy as np
 import pytest
@@ -39,7 +40,7 @@ def test_edges_of_the_one_cta_reduction(cpx, m, kind):
         scale = np.linalg.norm(a, 2)
         assert np.max(np.abs(w - ref)) <= TOL * scale
         assert np.max(np.linalg.norm(a @ z - z * w, axis=0)) <= 10 * TOL * scale
-        assert np.max(np.abs(z.conj().T @ z - np.eye(nev))) <= 10 * TOL
+        assert np.max(np.abs(z.conj().T @ z - np.eye(nev))) <= (TOL if m <= 64 else 10 * TOL)
 
 
 @pytest.mark.parametrize("cpx", [False, True])

@@ -1,5 +1,6 @@
-"""The one-launch projector term against the dense operator: block widths around its column tiles and its size limit
-(wider blocks take the library products), D blocks of several channels, and the packed real form against the complex one.
+"""The one-launch projector term against the dense operator: block widths around its column tiles and groups of bands (up
+to two passes of column tiles a cluster), D blocks of several channels, rows staged at once and in several chunks with a
+remainder, and both sides of the work limit past which the library products run; packed real against complex.
 Bar: 1e-12 of max |H psi|, as the other FP64 H|psi> tests."""
 
 import numpy as np
@@ -7,8 +8,8 @@ import pytest
 
 from conftest import rng
 from oracle import pwdft_oracle as O
-from pwgpu.context import build_system
-from pwgpu.crystal import KPoint, diamond_primitive, diamond_supercell, gamma_only
+from pwgpu.context import Projectors, ScfSystem, build_system
+from pwgpu.crystal import Atom, Crystal, KPoint, Lattice, diamond_primitive, diamond_supercell, gamma_only, miller_to_idx
 from pwgpu.lib import PwGpu
 from pwgpu.symmetry import SymmetryInfo
 
@@ -21,7 +22,7 @@ def _veff(s):
     return s.v_local_g + O.hartree(rho_g, s.g_squared) + O.density_r_to_g(vxc, s.dims)
 
 
-@pytest.mark.parametrize("nb", [1, 2, 8, 9, 31, 33, 64, 65, 150, 200])
+@pytest.mark.parametrize("nb", [1, 2, 8, 9, 31, 33, 64, 65, 150, 200, 257, 300])
 def test_complex_matches_dense(nb, si_pp):
     s = build_system(diamond_primitive("Si", 5.431), {"Si": si_pp}, 260.0, [KPoint(np.array([0.11, -0.23, 0.31]), 1.0)])
     veff = _veff(s)
@@ -109,3 +110,66 @@ def test_capture_of_a_narrower_block(si_pp):
         scale = float(ref.abs().max())
         assert float((out[:nb] - ref[:nb]).abs().max()) < 1e-12 * scale
         del graph
+
+
+class _Basis:
+    def __init__(self, miller):
+        self.miller, self.g = miller, miller.astype(np.float64)
+
+    def __len__(self):
+        return len(self.miller)
+
+
+def _sphere_system(radius, n_ch, gamma):
+    """A sphere of plane waves with random projectors, B(-G) = conj B(G), and 4-channel D blocks; V_eff stays zero."""
+    ax = np.arange(-radius, radius + 1)
+    p = np.stack(np.meshgrid(ax, ax, ax, indexing="ij"), -1).reshape(-1, 3)
+    p = np.ascontiguousarray(p[np.sum((p / (radius + 0.4)) ** 2, 1) <= 1.0], dtype=np.int32)
+    dims, mi, g = (4 * radius + 2 if radius % 2 else 4 * radius + 4,) * 3, p.astype(np.int64), rng(n_ch)
+    b = g.standard_normal((len(p), n_ch)) + 1j * g.standard_normal((len(p), n_ch))
+    b = (b + b[::-1].conj()) / np.sqrt(4 * len(p))  # -G is the mirrored row of the symmetric list
+    d = [np.array([[2.0, 0.3, 0, 0], [0.3, -1.0, 0, 0], [0, 0, 1.5, 0], [0, 0, 0, -0.5]])] * (n_ch // 4)
+    proj = Projectors(b, d, np.arange(0, n_ch + 1, 4, dtype=np.int32))
+    n = int(np.prod(dims))
+    atoms = [Atom("Si", (4.0 * i / n_ch, 0.0, 0.0)) for i in range(n_ch // 4)]
+    k = np.zeros(3) if gamma else np.array([0.1, 0.2, 0.3])
+    return ScfSystem(Crystal(Lattice.from_rows(np.eye(3) * 2 * np.pi), atoms), _Basis(p), dims,
+                     miller_to_idx(dims, mi[:, 0], mi[:, 1], mi[:, 2]), [KPoint(k, 1.0)],
+                     [0.1 * np.sum(mi.astype(np.float64) ** 2, 1)], [proj], np.zeros(n, dtype=np.complex128), np.zeros(n),
+                     np.zeros(0), 4.0, (2 * np.pi) ** 3, 0.0, SymmetryInfo.identity_only(), np.zeros(0))
+
+
+def _dense(s, psi):
+    p = s.projectors[0]
+    return s.kinetic[0][:, None] * psi + p.b @ (p.d_dense() @ (p.b.conj().T @ psi))
+
+
+# radius 13: 10,059 rows, 629 a CTA; 16 complex (40 real) channels and 8 bands of a group do not fit at once: two chunks.
+# radius 8: 2,517 rows; 40 channels: the complex work limit lies between 49 and 50 bands, the real one between 119 and 120.
+@pytest.mark.parametrize("radius,n_ch,nb", [(13, 16, 1), (13, 16, 7), (13, 16, 28), (8, 40, 49), (8, 40, 50)])
+def test_complex_chunks_and_work_limit(radius, n_ch, nb):
+    s = _sphere_system(radius, n_ch, gamma=False)
+    g = rng(nb)
+    psi = g.standard_normal((s.n_pw, nb)) + 1j * g.standard_normal((s.n_pw, nb))
+    ref = _dense(s, psi)
+    with PwGpu(s) as dev:
+        dev.set_veff_g(s.v_local_g)
+        got = dev.apply_h(psi)
+    assert np.max(np.abs(got - ref)) / np.max(np.abs(ref)) < 1e-12
+
+
+@pytest.mark.parametrize("radius,n_ch,nb", [(13, 40, 1), (13, 40, 13), (13, 40, 28), (8, 40, 119), (8, 40, 120)])
+def test_real_chunks_and_work_limit(radius, n_ch, nb):
+    s = _sphere_system(radius, n_ch, gamma=True)
+    n, zero = s.n_pw, s.n_pw // 2
+    half = np.arange(zero + 1, n)  # first nonzero index positive, in basis order
+    u = rng(nb).standard_normal((n, nb))
+    c = np.sqrt(0.5) * (u[1:zero + 1] + 1j * u[zero + 1:])
+    psi = np.empty((n, nb), dtype=np.complex128)
+    psi[zero], psi[half], psi[zero - 1 - np.arange(zero)] = u[0], c, c.conj()
+    h = _dense(s, psi)
+    ref = np.concatenate([h[zero:zero + 1].real, np.sqrt(2.0) * h[half].real, np.sqrt(2.0) * h[half].imag])
+    with PwGpu(s) as dev:
+        dev.set_veff_g(s.v_local_g)
+        got = dev.apply_h_packed(u)
+    assert np.max(np.abs(got - ref)) / np.max(np.abs(ref)) < 1e-12
