@@ -27,10 +27,10 @@ struct EigWork {
   double2* Pn = nullptr;   // n x nd: P of the last step (active bands)
   double2* HPn = nullptr;  // n x nd
   double2* Hs = nullptr;   // m x m (m <= 3 nd): subspace matrix, then eigenvectors (cuSOLVER)
-  double2* Cs = nullptr;   // m x m: eigenvectors (batched small solver), gathered columns
+  double2* Cs = nullptr;   // m x m: eigenvectors of the subspace matrix
   double2* G = nullptr;    // m x m: Gram / coupling blocks
   double2* Z = nullptr;    // m x m: coupling block, projection coefficients
-  double2* Id = nullptr;   // m x m identity (small solver's overlap)
+  double2* Id = nullptr;   // m x m: identity of a shifted Cholesky, then the inverse of the factor
   double* lam = nullptr;   // m: Ritz values of the last subspace solve
   double* lam0 = nullptr;  // nd: Ritz values the residuals refer to
   double* colsq = nullptr; // 3 nd

@@ -19,10 +19,10 @@ constexpr int plane_threads(int x0, int x1) {
 }
 
 // The pass for planes with equal x and y lengths (every cubic grid): strides
-// and divisions are constants.  What bounds it: shared-memory wavefronts (41k
-// complex accesses a plane at 72 x 72) and the FP64 or FP32 pipe, about
-// equally, with the block barriers hidden by 2 (FP64) or 3 (FP32) blocks an
-// SM.  160 bands on 72^3: 0.484 ms FP64 and 0.265 ms FP32, against 0.915 and
+// and divisions are constants.  What bounds it: the shared-memory data path,
+// 7,240 (FP64) and 3,920 (FP32) wavefronts a plane at 72 x 72, 67 and 65 % of
+// its peak rate, and the block barriers, a quarter of the warps' stalls with 2
+// and 3 blocks an SM; the FP64 and FP32 pipes are busy 43 and 42 %, HBM 6 %.  160 bands on 72^3: 0.484 ms FP64 and 0.265 ms FP32, against 0.915 and
 // 0.461 ms for the form with two planes of shared memory, a V(r) plane and
 // eight stages (one and two blocks an SM).  Threads per block at 72 x 72:
 // 216 0.484 / 0.262, 324 0.484 / 0.269, 432 0.590 / 0.285, 648 0.564 / 0.354 ms.
