@@ -46,17 +46,8 @@ constexpr int kW = kT / 32;
 constexpr int kMaxC = 16;
 constexpr size_t kSmemMax = 227 * 1024 - 4096;
 
-__device__ __forceinline__ double ldcg(const double* p) { return __ldcg(p); }
-__device__ __forceinline__ double2 ldcg(const double2* p) { return __ldcg(p); }
 template <typename T> __device__ __forceinline__ T zero() { return mk<T>(0.0, 0.0); }
 
-// c += a b on one 8 x 8 tile: lane holds a(lane / 4, lane % 4), b(lane % 4, lane / 4) and
-// c(lane / 4, 2 (lane % 4) + {0, 1}).
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
 template <typename T> struct Tile;
 template <> struct Tile<double> {
   double c[2];

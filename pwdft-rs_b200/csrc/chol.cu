@@ -47,8 +47,6 @@ template <typename T> struct TileB;
 template <> struct TileB<double> { static constexpr int value = 32; };
 template <> struct TileB<double2> { static constexpr int value = 16; };
 
-__device__ __forceinline__ double ldcg(const double* p) { return __ldcg(p); }
-__device__ __forceinline__ double2 ldcg(const double2* p) { return __ldcg(p); }
 __device__ __forceinline__ double zero_of(double) { return 0.0; }
 __device__ __forceinline__ double2 zero_of(double2) { return make_double2(0.0, 0.0); }
 

@@ -1,4 +1,4 @@
-// Scalar helpers of the dense FP64 kernels (eigh.cu, chol.cu): double is
+// Helpers of the dense FP64 kernels (eigh.cu, chol.cu, block_steps.cu): double is
 // the real symmetric case, double2 the complex Hermitian one.
 #pragma once
 
@@ -42,6 +42,19 @@ __device__ __forceinline__ double2 shfl(double2 v, int l) {
 template <typename T> __device__ __forceinline__ T warp_sum(T v) {
   for (int o = 16; o > 0; o >>= 1) v = add(v, shfl_down(v, o));
   return shfl(v, 0);
+}
+
+
+// loads past L1, of what another CTA has written
+__device__ __forceinline__ double ldcg(const double* p) { return __ldcg(p); }
+__device__ __forceinline__ double2 ldcg(const double2* p) { return __ldcg(p); }
+
+// c += a b on one 8 x 8 tile: lane holds a(lane / 4, lane % 4), b(lane % 4, lane / 4) and
+// c(lane / 4, 2 (lane % 4) + {0, 1}).
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
 }
 
 }  // namespace dense

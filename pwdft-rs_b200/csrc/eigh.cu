@@ -182,9 +182,6 @@ __host__ __device__ inline size_t norm_offset(int m, int nev) {
   return xchg_offset(m, nev) + 2 * ((size_t)4 * m + 2 * kMaxCluster * kWarps);
 }
 
-__device__ __forceinline__ double ldcg(const double* p) { return __ldcg(p); }
-__device__ __forceinline__ double2 ldcg(const double2* p) { return __ldcg(p); }
-
 // Seeded start vector entry in [-1, 1).
 __device__ __forceinline__ double start_entry(int i, int j) {
   uint64_t x = 0x9E3779B97F4A7C15ull * (uint64_t)(i + 1) + 0xD1B54A32D192ED03ull * (uint64_t)(j + 7);
@@ -213,11 +210,6 @@ __device__ __forceinline__ double2 nmadd(double2 x, double2 a, double2 b) {
 // Sum over the warp in every lane, on the FP64 tensor core: the 8 x 8 x 4 product with a matrix of ones adds
 // the four lanes of a column of B, the two entries a lane gets back are added, and a second product adds the four
 // distinct values left (two products and one addition against five shuffle-and-add stages).
-__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
 __device__ __forceinline__ double warp_all(double v) {
   double c[2] = {0.0, 0.0}, d[2] = {0.0, 0.0};
   dmma(c, 1.0, v);
