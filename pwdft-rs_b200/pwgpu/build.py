@@ -11,6 +11,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 PKG_ROOT = os.path.dirname(HERE)
@@ -19,7 +20,12 @@ INCLUDE = os.path.join(os.path.dirname(PKG_ROOT), "include")
 LIBDIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIBDIR, "libpwgpu.so")
 
-SOURCES = ["api.cu", "hpsi.cu", "hpsi_plane.cu", "plane_rt.cu", "plane_len_a.cu", "plane_len_b.cu", "plane_len_c.cu", "plane_len_d.cu", "plane_len_e.cu", "linalg.cu", "lobpcg.cu", "block_steps.cu", "scf.cu", "noalloc.cu", "gemm_bf16.cu", "nl_mixed.cu", "server.cu", "gamma.cu", "setup.cu", "components.cu", "eigh.cu", "chol.cu", "upf.cu", "deck.cu"]
+# the sources that take longest first: they are compiled side by side
+SOURCES = [
+    "block_steps.cu", "hpsi.cu", "plane_rt.cu", "eigh.cu", "plane_len_e.cu", "gemm_bf16.cu", "plane_len_d.cu",
+    "plane_len_c.cu", "plane_len_b.cu", "plane_len_a.cu", "lobpcg.cu", "chol.cu", "scf.cu", "api.cu", "hpsi_plane.cu",
+    "linalg.cu", "noalloc.cu", "nl_mixed.cu", "server.cu", "gamma.cu", "setup.cu", "components.cu", "upf.cu", "deck.cu",
+]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -48,25 +54,28 @@ def nvcc_path() -> str:
     return "nvcc"
 
 
+def _compile(src: str, verbose: bool, extra_flags) -> str:
+    """Object of one source, compiled when the source or any header is newer."""
+    path = os.path.join(CSRC, src)
+    obj = os.path.join(LIBDIR, src.replace(".cu", ".o"))
+    deps = [path] + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".hpp"))]
+    deps.append(os.path.join(INCLUDE, "pwgpu.h"))
+    if not os.path.exists(obj) or os.path.getmtime(obj) < max(os.path.getmtime(d) for d in deps):
+        cut = cutlass_root()
+        cmd = [nvcc_path(), *NVCC_FLAGS, *(extra_flags or []), "-I", INCLUDE, "-I", os.path.join(cut, "include"),
+               "-I", os.path.join(cut, "tools", "util", "include"), "-c", path, "-o", obj]
+        if verbose:
+            print(" ".join(cmd))
+        subprocess.run(cmd, check=True)
+    return obj
+
+
 def build(verbose: bool = False, extra_flags=None) -> str:
     os.makedirs(LIBDIR, exist_ok=True)
-    objs = []
-    nvcc = nvcc_path()
-    for src in SOURCES:
-        path = os.path.join(CSRC, src)
-        obj = os.path.join(LIBDIR, src.replace(".cu", ".o"))
-        deps = [path] + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".hpp"))]
-        deps.append(os.path.join(INCLUDE, "pwgpu.h"))
-        if not os.path.exists(obj) or os.path.getmtime(obj) < max(os.path.getmtime(d) for d in deps):
-            cut = cutlass_root()
-            cmd = [nvcc, *NVCC_FLAGS, *(extra_flags or []), "-I", INCLUDE, "-I", os.path.join(cut, "include"),
-                   "-I", os.path.join(cut, "tools", "util", "include"), "-c", path, "-o", obj]
-            if verbose:
-                print(" ".join(cmd))
-            subprocess.run(cmd, check=True)
-        objs.append(obj)
+    with ThreadPoolExecutor(max_workers=max(1, min(8, os.cpu_count() or 1))) as pool:
+        objs = list(pool.map(lambda s: _compile(s, verbose, extra_flags), SOURCES))
     if not os.path.exists(LIB) or os.path.getmtime(LIB) < max(os.path.getmtime(o) for o in objs):
-        cmd = [nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", *objs, "-o", LIB,
+        cmd = [nvcc_path(), "-shared", "-gencode", "arch=compute_100a,code=sm_100a", *objs, "-o", LIB,
                "-lcublas", "-lcusolver", "-lcudart"]
         if verbose:
             print(" ".join(cmd))
